@@ -255,7 +255,7 @@ REF_SRC = "/root/reference"
 def build_ref(force: bool = False) -> str | None:
     """Compile the reference's graph.h when the reference tree is present
     (this container); on a machine without it the prebuilt library is used."""
-    if not os.path.isdir(REF_SRC):
+    if not os.path.isfile(os.path.join(REF_SRC, "sap", "graph.h")):
         return REF_LIB if os.path.exists(REF_LIB) else None
     srcs = [os.path.join(HERE, "ref_graph", "ref_graph_driver.cu"), os.path.join(HERE, "ref_graph", "cusp", "shim.h")]
     newest = max(os.path.getmtime(s) for s in srcs)
