@@ -268,6 +268,11 @@ __device__ __forceinline__ void cp_async8(void* smem, const void* gmem) {
   unsigned s = static_cast<unsigned>(__cvta_generic_to_shared(smem));
   asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" ::"r"(s), "l"(gmem));
 }
+// 16 bytes, both addresses 16-byte aligned, past L1
+__device__ __forceinline__ void cp_async16(void* smem, const void* gmem) {
+  unsigned s = static_cast<unsigned>(__cvta_generic_to_shared(smem));
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(s), "l"(gmem));
+}
 template <typename T>
 __device__ __forceinline__ void cp_async_val(T* smem, const T* gmem) {
   if constexpr (sizeof(T) == 8) cp_async8(smem, gmem);

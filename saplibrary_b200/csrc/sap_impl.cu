@@ -18,6 +18,7 @@
 
 #include "common.cuh"
 #include "krylov_kernels.cuh"
+#include "narrow_sweeps.cuh"
 #include "precond_kernels.cuh"
 #include "reorder.h"
 #include "reorder_pipeline.h"
@@ -721,15 +722,18 @@ class PrecondT : public PrecBase {
       for (auto& d : parts_h) maxsz = std::max(maxsz, d.size);
       scratch.alloc((size_t)2 * (P - 1) * maxsz * K);
       if (K > 1024) throw Error(SAP_ERR_UNSUPPORTED, "coupling width above 1024 is not supported by the spike kernel");
-      k_spikes_var<T><<<dim3(P - 1, 2), ((K + 31) / 32) * 32, 0, st>>>(parts_d.get(), B.get(), offd.get(), iface_d.get(),
-                                                                   V.get(), W.get(), scratch.get(), (long long)maxsz, K);
-      SAPB_LAUNCHED();
+      if (window(K) && window(parts_maxK())) {
+        spikes_lu(iface_d.get(), maxsz);
+      } else {
+        k_spikes_var<T><<<dim3(P - 1, 2), ((K + 31) / 32) * 32, 0, st>>>(
+            parts_d.get(), B.get(), offd.get(), iface_d.get(), V.get(), W.get(), scratch.get(), (long long)maxsz, K);
+        SAPB_LAUNCHED();
+      }
       SAPB_CUDA(cudaStreamSynchronize(st));
       scratch.release();
       t_assembly = ms_since(t2);
       t2 = Clock::now();
-      k_reduced_factor<T><<<P - 1, 512, 0, st>>>(V.get(), W.get(), S.get(), K, o.safeFactorization ? 1 : 0);
-      SAPB_LAUNCHED();
+      reduced_factor();
       SAPB_CUDA(cudaStreamSynchronize(st));
       t_fullLU = ms_since(t2);
     }
@@ -796,14 +800,28 @@ class PrecondT : public PrecBase {
       V.alloc((size_t)(P - 1) * K * K);
       W.alloc((size_t)(P - 1) * K * K);
       S.alloc((size_t)(P - 1) * K * K);
-      if (lu_ul) {
-        k_spikes_luul<T><<<dim3(P - 1, 2), ((K + 31) / 32) * 32, 0, st>>>(parts_d.get(), P, B.get(),
-                                                                        B2.get() ? B2.get() : B.get(), offd.get(),
+      const T* b2 = B2.get() ? B2.get() : B.get();
+      int maxsz = 0;
+      for (auto& p : parts_h) maxsz = std::max(maxsz, p.size);
+      if (lu_ul && window(K)) {
+        pack_corners(b2);
+        by_window(K, [&](auto R1) {
+          auto kern = k_win_spikes_luul<T, R1(), kSpikeCols>;
+          constexpr size_t smem = win_smem<T>(R1());
+          allow_smem(kern, smem);
+          kern<<<dim3(P - 1, 2, spike_groups(K)), 32 * spike_warps(K), smem, st>>>(
+              parts_d.get(), pkd.get(), pku.get(), piv.get(), pkd2.get(), pku2.get(), piv2.get(), offd.get(), V.get(),
+              W.get(), K, KP);
+        });
+        SAPB_LAUNCHED();
+      } else if (lu_ul) {
+        k_spikes_luul<T><<<dim3(P - 1, 2), ((K + 31) / 32) * 32, 0, st>>>(parts_d.get(), P, B.get(), b2, offd.get(),
                                                                         V.get(), W.get(), K);
         SAPB_LAUNCHED();
+      } else if (window(K)) {
+        scratch.alloc(spike_scratch(P - 1, K, maxsz, false));
+        spikes_lu(nullptr, maxsz);
       } else {
-        int maxsz = 0;
-        for (auto& p : parts_h) maxsz = std::max(maxsz, p.size);
         scratch.alloc((size_t)(P - 1) * K * maxsz);
         k_spikes_luonly<T><<<dim3(P - 1, 2), ((K + 31) / 32) * 32, 0, st>>>(parts_d.get(), B.get(), offd.get(),
                                                                           V.get(), W.get(), scratch.get(),
@@ -815,12 +833,59 @@ class PrecondT : public PrecBase {
       scratch.release();
       t_assembly = ms_since(t0);
       t0 = Clock::now();
-      k_reduced_factor<T><<<P - 1, 512, 0, st>>>(V.get(), W.get(), S.get(), K, o.safeFactorization ? 1 : 0);
-      SAPB_LAUNCHED();
+      reduced_factor();
       SAPB_CUDA(cudaStreamSynchronize(st));
       t_fullLU = ms_since(t0);
     }
     build_sweeps();
+  }
+
+  // The register-window kernels (narrow_sweeps.cuh) take half-bandwidths up
+  // to kWinMaxK; f gets their slot count as a compile-time constant.
+  static bool window(int k) { return k <= kWinMaxK<T>; }
+  template <class F>
+  static void by_window(int k, F&& f) {
+    switch (win_slots(k)) {
+      case 2: f(std::integral_constant<int, 2>{}); break;
+      case 3: f(std::integral_constant<int, 3>{}); break;
+      case 4: f(std::integral_constant<int, 4>{}); break;
+      case 5: f(std::integral_constant<int, 5>{}); break;
+      default: f(std::integral_constant<int, 6>{}); break;
+    }
+  }
+  template <class Kern>
+  static void allow_smem(Kern kern, size_t bytes) {
+    if (bytes > 48 * 1024)
+      SAPB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
+  }
+  // columns per warp of the spike sweeps, warps per CTA, CTAs per tip
+  static constexpr int kSpikeCols = 1;
+  static int spike_warps(int k) { return std::min(8, (k + kSpikeCols - 1) / kSpikeCols); }
+  static int spike_groups(int k) {
+    const int per = spike_warps(k) * kSpikeCols;
+    return (k + per - 1) / per;
+  }
+  // spike tips from LU factors of both neighbours, for all interfaces
+  void spikes_lu(const int* iface, int maxsz) {
+    const int maxK = parts_maxK();
+    by_window(maxK, [&](auto R1) {
+      auto kern = k_win_spikes_lu<T, R1(), kSpikeCols>;
+      constexpr size_t smem = win_smem<T>(R1());
+      allow_smem(kern, smem);
+      kern<<<dim3(P - 1, 2, spike_groups(K)), 32 * spike_warps(K), smem, st>>>(
+          parts_d.get(), pkd.get(), pku.get(), piv.get(), KP, offd.get(), iface, V.get(), W.get(), scratch.get(), (long long)maxsz, K);
+    });
+    SAPB_LAUNCHED();
+  }
+  void reduced_factor() {
+    const int boost = o.safeFactorization ? 1 : 0;
+    if (window(K)) {
+      allow_smem(k_win_reduced_factor<T>, reduced_smem<T>(K));
+      k_win_reduced_factor<T><<<P - 1, 512, reduced_smem<T>(K), st>>>(V.get(), W.get(), S.get(), K, boost);
+    } else {
+      k_reduced_factor<T><<<P - 1, 512, 0, st>>>(V.get(), W.get(), S.get(), K, boost);
+    }
+    SAPB_LAUNCHED();
   }
 
   // partBandedLU / partBlockedBandedUL (sap/precond.h:3882-3983, 4336-4418, 4780-4846).
@@ -901,6 +966,7 @@ class PrecondT : public PrecBase {
     SAPB_CUDA(cudaStreamSynchronize(st));
     if (hflag && !o.safeFactorization && !boost)
       throw Error(SAP_ZERO_PIVOTING, "Found a pivot equal to zero (partBandedLU).");
+    pack_factors();
   }
 
   void build_sweeps() {
@@ -952,6 +1018,10 @@ class PrecondT : public PrecBase {
     sweepThreads = std::max(32, ((maxK + 31) / 32) * 32);
     scanG = std::max(1, std::min(maxK, 512 / std::max(1, maxK)));
     const int nch = (int)chunks_h.size();
+    if (window(maxK)) {
+      build_window(maxK, nch);
+      return;
+    }
     const int tthreads = sweepThreads;
     size_t tsmem = (size_t)maxK * tthreads * sizeof(T);
     DBuf<T> gring;
@@ -976,10 +1046,116 @@ class PrecondT : public PrecBase {
     t_assembly += ms_since(t0);
   }
 
+  // The factors packed for the register-window sweeps (after factor()), and
+  // the UL corners of the LU_UL tips: those of partition p >= 1 at p * K, in
+  // B for the last partition, else in b2.
+  DBuf<T> pkd, pku, piv, pkd2, pku2, piv2;
+  int KP = 0;
+  void pack_factors() {
+    if (!window(parts_maxK())) return;
+    KP = pack_stride<T>(parts_maxK());
+    pkd.alloc((size_t)n * KP);
+    pku.alloc((size_t)n * KP);
+    piv.alloc(n);
+    const int np = (int)parts_h.size();
+    k_pack<T><<<dim3(grid_for(((long long)n / np + 1) * 32, 256, std::max(1, 148 * 32 / np)), (unsigned)np), 256, 0, st>>>(
+        parts_d.get(), B.get(), -1, KP, pkd.get(), pku.get(), piv.get());
+    SAPB_LAUNCHED();
+  }
+  void pack_corners(const T* b2) {
+    pkd2.alloc((size_t)P * K * KP);
+    pku2.alloc((size_t)P * K * KP);
+    piv2.alloc((size_t)P * K);
+    const int gx = grid_for((long long)K * 32, 256, 64);
+    if (P > 2) {
+      k_pack<T><<<dim3(gx, P - 1), 256, 0, st>>>(parts_d.get(), b2, K, KP, pkd2.get(), pku2.get(), piv2.get());
+      SAPB_LAUNCHED();
+    }
+    const size_t o = (size_t)(P - 1) * K;
+    k_pack<T><<<dim3(gx, 1), 256, 0, st>>>(parts_d.get() + (P - 1), B.get(), K, KP, pkd2.get() + o * KP,
+                                           pku2.get() + o * KP, piv2.get() + o);
+    SAPB_LAUNCHED();
+  }
+
+  // Transfer matrices of the register-window sweeps, and the carry scan's
+  // launch shape: about sqrt(K) column groups balance a group's share of the
+  // product against the sum over the groups; batches of as many chunks as fit
+  // twice in shared memory (one from K ~ 82 in FP64, ~ 116 in FP32 on).
+  int scanNT = 32, scanNB = 1;
+  size_t scanSmem = 0;
+  void build_window(int maxK, int nch) {
+    auto t0 = Clock::now();
+    constexpr int C = 4;
+    const int warps = std::min(16, (maxK + C - 1) / C);
+    SAPB_PROF("transfer", st);
+    by_window(maxK, [&](auto R1) {
+      auto kern = k_win_transfer<T, R1(), C>;
+      constexpr size_t smem = win_smem<T>(R1());
+      allow_smem(kern, smem);
+      allow_smem(k_win_pass1<T, R1()>, smem);
+      allow_smem(k_win_pass2<T, R1()>, smem);
+      allow_smem(k_win_pass3<T, R1()>, smem);
+      kern<<<dim3(nch, (maxK + C * warps - 1) / (C * warps), 2), 32 * warps, smem, st>>>(
+          parts_d.get(), chunks_d.get(), toff_d.get(), pkd.get(), pku.get(), KP, T1.get(), T2.get(), first1_d.get(), first2_d.get());
+    });
+    SAPB_LAUNCHED();
+    scanG = std::max(1, std::min((int)std::lround(std::sqrt((double)maxK)), 512 / maxK));
+    scanNT = ((maxK * scanG + 31) / 32) * 32;
+    const size_t fixed = (size_t)(maxK + std::max(scanNT, maxK)) * sizeof(T);
+    int longest = 1;
+    for (size_t c = 0, run = 0; c < chunks_h.size(); c++) {
+      run = c > 0 && chunks_h[c].part == chunks_h[c - 1].part ? run + 1 : 1;
+      longest = std::max(longest, (int)run);
+    }
+    auto bytes = [&](int nb) { return fixed + 2 * scan_batch<T>(maxK, nb) * sizeof(T); };
+    scanNB = 1;
+    while (scanNB < 64 && scanNB < longest && bytes(scanNB * 2) <= 200 * 1024) scanNB *= 2;
+    scanSmem = bytes(scanNB);
+    allow_smem(k_win_scan<T>, scanSmem);
+    SAPB_CUDA(cudaStreamSynchronize(st));
+    t_assembly += ms_since(t0);
+  }
+  void window_scan(const T* Tm, const T* tails, T* carry, int which) {
+    SAPB_PROF("scan", st);
+    k_win_scan<T><<<(int)parts_h.size(), std::max(scanNT, 256), scanSmem, st>>>(
+        parts_d.get(), pchunk0_d.get(), pnchunk_d.get(), koff_d.get(), toff_d.get(), Tm, tails, carry, which, scanG,
+        scanNT, scanNB);
+    SAPB_LAUNCHED();
+  }
+  void window_pair(const double* vin, double* zout, T* gout, int maxK, int nch) {
+    by_window(maxK, [&](auto R1) {
+      constexpr size_t smem = win_smem<T>(R1());
+      {
+        SAPB_PROF("pass1", st);
+        k_win_pass1<T, R1()><<<nch, 32, smem, st>>>(parts_d.get(), chunks_d.get(), koff_d.get(), pkd.get(), pku.get(),
+                                                    KP, vin, F.get(), tails1.get(), reordered ? gin_d.get() : nullptr,
+                                                    in_scale());
+        SAPB_LAUNCHED();
+      }
+      window_scan(T1.get(), tails1.get(), carry1.get(), 1);
+      {
+        SAPB_PROF("pass2", st);
+        k_win_pass2<T, R1()><<<nch, 32, smem, st>>>(parts_d.get(), chunks_d.get(), first1_d.get(), koff_d.get(),
+                                                    pkd.get(), pku.get(), KP, piv.get(), F.get(), carry1.get(),
+                                                    Y.get(), tails2.get());
+        SAPB_LAUNCHED();
+      }
+      window_scan(T2.get(), tails2.get(), carry2.get(), 2);
+      {
+        SAPB_PROF("pass3", st);
+        k_win_pass3<T, R1()><<<nch, 32, smem, st>>>(parts_d.get(), chunks_d.get(), first2_d.get(), koff_d.get(),
+                                                    pkd.get(), pku.get(), KP, Y.get(), carry2.get(), zout, gout,
+                                                    reordered ? sout_d.get() : nullptr, out_scale());
+        SAPB_LAUNCHED();
+      }
+    });
+  }
+
   // One partitioned sweep pair: out = D^-1 rhs, rhs = vin (FP64) or F.
   void sweep_pair(const double* vin, double* zout, T* gout) {
     const int nch = (int)chunks_h.size();
     const int maxK = parts_maxK();
+    if (window(maxK)) return window_pair(vin, zout, gout, maxK, nch);
     const size_t s1 = (size_t)(maxK + maxChunk) * sizeof(T);
     const int NT = sweepThreads;
     const int scanNT = ((maxK * scanG + 31) / 32) * 32;
@@ -1042,11 +1218,27 @@ class PrecondT : public PrecBase {
     if (spike) {
       sweep_pair(v, nullptr, Gv.get());
       {
-      SAPB_PROF("reduced_apply", st);
-      k_reduced_apply<T><<<P - 1, ((K + 31) / 32) * 32, 3 * K * sizeof(T), st>>>(parts_d.get(), V.get(), W.get(), S.get(),
-                                                                            offd.get(), Gv.get(), F.get(), K,
-                                                                            var_band ? iface_d.get() : nullptr);
-      SAPB_LAUNCHED();
+        SAPB_PROF("reduced_apply", st);
+        const int* map = var_band ? iface_d.get() : nullptr;
+        if (window(K)) {
+          const size_t smem = reduced_smem<T>(K) + 3 * K * sizeof(T);
+          auto launch = [&](auto kern) {
+            allow_smem(kern, smem);
+            kern<<<P - 1, 512, smem, st>>>(parts_d.get(), V.get(), W.get(), S.get(), offd.get(), Gv.get(), F.get(), K,
+                                           map);
+          };
+          switch ((K + 31) / 32) {
+            case 1: launch(k_win_reduced_apply<T, 1>); break;
+            case 2: launch(k_win_reduced_apply<T, 2>); break;
+            case 3: launch(k_win_reduced_apply<T, 3>); break;
+            case 4: launch(k_win_reduced_apply<T, 4>); break;
+            default: launch(k_win_reduced_apply<T, 5>); break;
+          }
+        } else {
+          k_reduced_apply<T><<<P - 1, ((K + 31) / 32) * 32, 3 * K * sizeof(T), st>>>(
+              parts_d.get(), V.get(), W.get(), S.get(), offd.get(), Gv.get(), F.get(), K, map);
+        }
+        SAPB_LAUNCHED();
       }
       sweep_pair(nullptr, z, nullptr);
     } else {
