@@ -8,6 +8,8 @@
 // global layout of the reference.
 #pragma once
 
+#include <type_traits>
+
 #include "common.cuh"
 
 namespace sapb {
@@ -202,33 +204,40 @@ k_factor_smem(const FactorJob* __restrict__ jobs, T* __restrict__ B, T* __restri
 
 // Blocked form of k_factor_smem for K <= 32 R - NB: the same elimination,
 // every element receiving the same updates in the same order (hence the same
-// factors bit for bit), with two CTA barriers per panel of NB pivots instead
+// factors bit for bit), with one CTA barrier per panel of NB pivots instead
 // of two per pivot.
 //
-// Panel p covers columns j0 = p NB .. j0 + NB - 1.  Warp 0 factors it in
-// registers: lane l holds rows j0 + l + 32 t (t < R) of the NB panel columns,
-// each pivot is broadcast by a shuffle, its column is divided by it and the
-// rest of the panel receives the rank-1 update.  After a barrier the warps
-// apply the panel to the K columns right of it, four columns per warp at once
-// (the columns' rows in registers, the U element of each pivot broadcast from
-// the lane holding that row, each L entry read once from shared memory for
-// the four), pivots in order.  While warp 0 factors, the other warps write
-// back the previous panel (post-divided by the pivots of its U rows) and
-// fetch, with cp.async into the freed slots, the NB columns that panel p + DPF
-// will first touch.  The ring holds W = K + NB (1 + DPF) column slots; slots
-// advance by additions, with no modulo.
+// What bounds it is the chain of pivots, so the chain has a warp of its own
+// (look-ahead): while the other warps apply panel p (columns j0 .. j0+NB-1) to
+// the columns from j0 + 2 NB on, warp 0 applies it to the NB columns of panel
+// p+1 and factors that panel.  Warp 0 holds a panel in registers: lane l rows
+// j0 + l + 32 t (t < R) of its NB columns; each pivot is broadcast by a
+// shuffle, its column is divided by it and the rest of the panel receives the
+// rank-1 update.  The panel's L columns also go, with zeros outside the band,
+// to Lp in the row alignment the updates use, so that these need no tests:
+// a warp takes CPW columns (their rows in registers, the U element of each
+// pivot broadcast from the lane holding that row), pivots in order.  Beside
+// their updates the other warps write back panel p-1 and fetch, with cp.async
+// into the freed slots, the NB columns that panel p + DPF will first touch.
+// The ring holds W = K + NB (1 + DPF) column slots; slots advance by
+// additions, with no modulo.
+template <typename T, int NB>
+inline size_t factor_panel_smem(int R, int K, int dpf) {
+  return ((size_t)(K + NB * (1 + dpf)) * (2 * K + 1) + 2 * NB * 32 * R) * sizeof(T);
+}
 template <typename T, int NB, int R>
 __global__ void __launch_bounds__(512)
 k_factor_panel(const FactorJob* __restrict__ jobs, T* __restrict__ B, T* __restrict__ B2,
                int do_boost, int* __restrict__ zero_flag, int DPF) {
-  constexpr int CPW = 4;  // columns a warp applies a panel to at once
+  constexpr int CPW = 4;   // columns a trailing warp applies a panel to at once
+  constexpr int LR = 32 * R;
   const FactorJob jb = jobs[blockIdx.x];
   const int K = jb.K, SW = 2 * K + 1, np = jb.e - jb.s, W = K + NB * (1 + DPF);
   extern __shared__ __align__(16) unsigned char sm_raw[];
   T* win = reinterpret_cast<T*>(sm_raw);
+  T* Lp = win + W * SW;  // two panels of NB columns of LR rows
   T* band = (jb.target ? B2 : B) + jb.boff;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nw = blockDim.x >> 5;
-  const int ct = tid - 32, nct = blockDim.x - 32;  // copy threads: warps 1..
   const bool mir = jb.mirror != 0;
   auto gidx = [&](int i, int p) -> long long {
     int col = mir ? (np - 1 - i) : i;
@@ -236,175 +245,177 @@ k_factor_panel(const FactorJob* __restrict__ jobs, T* __restrict__ B, T* __restr
     return (long long)col * SW + pos;
   };
   auto wrap = [&](int s) { return s >= W ? s - W : s; };  // for 0 <= s < 2 W
-  // column `col` from ring slot `sl` to the band, its U entries post-divided
-  // column `col` from ring slot `sl` to the band (its U entries are divided
-  // by their rows' pivots afterwards, k_factor_postdiv)
-  auto out = [&](int col, int sl, int p) { band[gidx(col, p)] = win[sl * SW + p]; };
-  if (ct >= 0) {  // columns [0, K + NB), then one panel's new columns per group; all in slots == column
+  if (warp != 0) {  // columns [0, K + NB), then one panel's new columns per group; all in slots == column
     for (int g = 0; g < DPF; g++) {
       const int c0 = g == 0 ? 0 : K + g * NB, c1 = min(np, K + (g + 1) * NB);
-      for (int e = ct; e < (c1 - c0) * SW; e += nct) {
-        const int c = c0 + e / SW, p = e - (c - c0) * SW;
-        cp_async_val<T>(&win[c * SW + p], band + gidx(c, p));
-      }
+      for (int c = c0 + warp - 1; c < c1; c += nw - 1)
+        for (int p = lane; p < SW; p += 32) cp_async_val<T>(&win[c * SW + p], band + gidx(c, p));
       cp_async_commit();
     }
   }
   bool zero_seen = false;
-  int j0 = 0, s0 = 0;  // s0 = j0 % W
-  for (; j0 < np; j0 += NB, s0 = wrap(s0 + NB)) {
-    const int nb = min(NB, np - j0);
-    if (DPF == 2) cp_async_wait<1>();
-    else cp_async_wait<0>();
-    __syncthreads();
-    if (warp != 0) {
-      // write back panel p-1 and fetch the columns of panel p+DPF into its slots
-      // (the thread that reads a slot element issues the copy into it)
-      const int nf0 = j0 + DPF * NB + K;
-      const int sp = s0 - NB < 0 ? s0 - NB + W : s0 - NB;
-      for (int e = ct; e < NB * SW; e += nct) {
-        const int c = e / SW, p = e - c * SW, sl = wrap(sp + c);
-        if (j0 > 0) out(j0 - NB + c, sl, p);
-        if (nf0 + c < np) cp_async_val<T>(&win[sl * SW + p], band + gidx(nf0 + c, p));
+  // warp 0: panel q (columns j .. j+nb-1, first slot s) factored in registers
+  auto factor = [&](int j, int s, int nb, T* lp) {
+    T a[R][NB];
+    auto load_panel = [&]() {
+#pragma unroll
+      for (int c = 0; c < NB; c++) {
+        const T* colp = win + wrap(s + c) * SW;
+#pragma unroll
+        for (int t = 0; t < R; t++) {
+          const int pos = K + lane + 32 * t - c;  // row j + lane + 32 t
+          a[t][c] = (c < nb && j + lane + 32 * t < np && pos >= 0 && pos <= 2 * K) ? colp[pos] : T(0);
+        }
       }
-      cp_async_commit();
-    } else {
-      T a[R][NB];
-      auto load_panel = [&]() {
+    };
+    load_panel();
+    // fast path: each quotient from the pivot's reciprocal with Markstein's
+    // correction (div_rcp_fast, equal to the division inside its range),
+    // without branches; `bad` records a lane whose operands left the range
+    bool bad = false;
 #pragma unroll
-        for (int c = 0; c < NB; c++) {
-          const T* colp = win + wrap(s0 + c) * SW;
+    for (int k = 0; k < NB; k++) {
+      if (k < nb) {
+        const int w = min(K, np - 1 - (j + k));
+        T p = __shfl_sync(0xffffffffu, a[0][k], k);
+        if (do_boost) p = boost_pivot(p);
+        else zero_seen |= fabs((double)p) < 1e-7;
+        const T y = T(1) / p;
+        T u[NB];
 #pragma unroll
-          for (int t = 0; t < R; t++) {
-            const int pos = K + lane + 32 * t - c;  // row j0 + lane + 32 t
-            a[t][c] = (c < nb && j0 + lane + 32 * t < np && pos >= 0 && pos <= 2 * K) ? colp[pos] : T(0);
+        for (int c = k + 1; c < NB; c++) u[c] = __shfl_sync(0xffffffffu, a[0][c], k);
+#pragma unroll
+        for (int t = 0; t < R; t++) {
+          const int rr = lane + 32 * t - k;  // row - pivot row
+          const bool in = rr >= 1 && rr <= w;
+          bool ok;
+          const T l = div_rcp_fast(a[t][k], p, y, ok);
+          bad |= in && !ok;
+          a[t][k] = rr == 0 ? p : (in ? l : a[t][k]);
+#pragma unroll
+          for (int c = k + 1; c < NB; c++) {
+            if (c - k <= w) {
+              const T nv = a[t][c] - l * u[c];
+              a[t][c] = in ? nv : a[t][c];
+            }
           }
         }
-      };
+      }
+    }
+    if (__any_sync(0xffffffffu, bad)) {
+      // some quotient left the range: the panel again with the division
       load_panel();
-      // fast path: each quotient from the pivot's reciprocal with Markstein's
-      // correction (div_rcp_fast, equal to the division inside its range),
-      // without branches; `bad` records a lane whose operands left the range
-      bool bad = false;
 #pragma unroll
       for (int k = 0; k < NB; k++) {
         if (k < nb) {
-          const int w = min(K, np - 1 - (j0 + k));
+          const int w = min(K, np - 1 - (j + k));
           T p = __shfl_sync(0xffffffffu, a[0][k], k);
           if (do_boost) p = boost_pivot(p);
-          else zero_seen |= fabs((double)p) < 1e-7;
-          const T y = T(1) / p;
           T u[NB];
 #pragma unroll
           for (int c = k + 1; c < NB; c++) u[c] = __shfl_sync(0xffffffffu, a[0][c], k);
 #pragma unroll
           for (int t = 0; t < R; t++) {
-            const int rr = lane + 32 * t - k;  // row - pivot row
-            const bool in = rr >= 1 && rr <= w;
-            bool ok;
-            const T l = div_rcp_fast(a[t][k], p, y, ok);
-            bad |= in && !ok;
-            a[t][k] = rr == 0 ? p : (in ? l : a[t][k]);
+            const int rr = lane + 32 * t - k;
+            if (rr == 0) {
+              a[t][k] = p;
+            } else if (rr >= 1 && rr <= w) {
+              const T l = a[t][k] / p;
+              a[t][k] = l;
 #pragma unroll
-            for (int c = k + 1; c < NB; c++) {
-              if (c - k <= w) {
-                const T nv = a[t][c] - l * u[c];
-                a[t][c] = in ? nv : a[t][c];
-              }
+              for (int c = k + 1; c < NB; c++)
+                if (c - k <= w) a[t][c] -= l * u[c];
             }
           }
-        }
-      }
-      if (__any_sync(0xffffffffu, bad)) {
-        // some quotient left the range: the panel again with the division
-        load_panel();
-#pragma unroll
-        for (int k = 0; k < NB; k++) {
-          if (k < nb) {
-            const int w = min(K, np - 1 - (j0 + k));
-            T p = __shfl_sync(0xffffffffu, a[0][k], k);
-            if (do_boost) p = boost_pivot(p);
-            T u[NB];
-#pragma unroll
-            for (int c = k + 1; c < NB; c++) u[c] = __shfl_sync(0xffffffffu, a[0][c], k);
-#pragma unroll
-            for (int t = 0; t < R; t++) {
-              const int rr = lane + 32 * t - k;
-              if (rr == 0) {
-                a[t][k] = p;
-              } else if (rr >= 1 && rr <= w) {
-                const T l = a[t][k] / p;
-                a[t][k] = l;
-#pragma unroll
-                for (int c = k + 1; c < NB; c++)
-                  if (c - k <= w) a[t][c] -= l * u[c];
-              }
-            }
-          }
-        }
-      }
-#pragma unroll
-      for (int c = 0; c < NB; c++) {
-        T* colp = win + wrap(s0 + c) * SW;
-#pragma unroll
-        for (int t = 0; t < R; t++) {
-          const int pos = K + lane + 32 * t - c;
-          if (c < nb && j0 + lane + 32 * t < np && pos >= 0 && pos <= 2 * K) colp[pos] = a[t][c];
         }
       }
     }
+#pragma unroll
+    for (int c = 0; c < NB; c++) {
+      T* colp = win + wrap(s + c) * SW;
+      const int w = c < nb ? min(K, np - 1 - (j + c)) : 0;
+#pragma unroll
+      for (int t = 0; t < R; t++) {
+        const int rr = lane + 32 * t - c, pos = K + rr;
+        if (c < nb && j + lane + 32 * t < np && pos >= 0 && pos <= 2 * K) colp[pos] = a[t][c];
+        lp[c * LR + lane + 32 * t] = rr >= 1 && rr <= w ? a[t][c] : T(0);
+      }
+    }
+  };
+  // the panel at j0 (L columns in lp) applied to the NC columns from q0 past
+  // its end on (column j0 + NB + q), the first nt of which exist
+  auto update = [&](auto ncol, int j0, int s0, const T* lp, int q0, int nt) {
+    constexpr int NC = decltype(ncol)::value;
+    T x[NC][R];
+#pragma unroll
+    for (int i = 0; i < NC; i++) {
+      const int q = q0 + i;
+      const T* colp = win + wrap(s0 + NB + q) * SW;
+#pragma unroll
+      for (int t = 0; t < R; t++) {
+        const int pos = K + lane + 32 * t - NB - q;
+        x[i][t] = (q < nt && j0 + lane + 32 * t < np && pos >= 0 && pos <= 2 * K) ? colp[pos] : T(0);
+      }
+    }
+#pragma unroll
+    for (int k = 0; k < NB; k++) {
+      T L[R];
+#pragma unroll
+      for (int t = 0; t < R; t++) L[t] = lp[k * LR + lane + 32 * t];
+#pragma unroll
+      for (int i = 0; i < NC; i++) {
+        const T U = __shfl_sync(0xffffffffu, x[i][0], k);
+#pragma unroll
+        for (int t = 0; t < R; t++) x[i][t] -= L[t] * U;
+      }
+    }
+#pragma unroll
+    for (int i = 0; i < NC; i++) {
+      const int q = q0 + i;
+      T* colp = win + wrap(s0 + NB + q) * SW;
+#pragma unroll
+      for (int t = 0; t < R; t++) {
+        const int pos = K + lane + 32 * t - NB - q;
+        if (q < nt && j0 + lane + 32 * t < np && pos >= 0 && pos <= 2 * K) colp[pos] = x[i][t];
+      }
+    }
+  };
+  // (K < NB: the next panel reaches past the columns the current one touches,
+  // into those of the newest group)
+  auto wait = [&] {
+    if (DPF == 2 && K >= NB) cp_async_wait<1>();
+    else cp_async_wait<0>();
     __syncthreads();
-    // the panel applied to the (up to K) columns right of it, CPW columns per warp at once,
-    // pivots in order: x(r, jc) -= L(r, j) U(j, jc)
-    const int nt = min(K, np - j0 - nb);
-    for (int q0 = warp * CPW; q0 < nt; q0 += nw * CPW) {
-      T x[CPW][R];
-      T* colp[CPW];
-      int kst[CPW];
-#pragma unroll
-      for (int i = 0; i < CPW; i++) {
-        const int q = q0 + i;  // column j0 + nb + q
-        colp[i] = win + wrap(s0 + nb + q) * SW;
-        kst[i] = q < nt ? max(0, nb + q - K) : NB;
-#pragma unroll
-        for (int t = 0; t < R; t++) {
-          const int pos = K + lane + 32 * t - nb - q;
-          x[i][t] = (q < nt && j0 + lane + 32 * t < np && pos >= 0 && pos <= 2 * K) ? colp[i][pos] : T(0);
+  };
+  wait();
+  if (warp == 0) factor(0, 0, min(NB, np), Lp);
+  int j0 = 0, s0 = 0, buf = 0;  // s0 = j0 % W
+  for (; j0 < np; j0 += NB, s0 = wrap(s0 + NB), buf ^= 1) {
+    const T* lp = Lp + buf * NB * LR;
+    const int nt = min(K, np - j0 - NB);
+    wait();
+    if (warp == 0) {
+      if (j0 + NB < np) {
+        update(std::integral_constant<int, NB>{}, j0, s0, lp, 0, min(nt, NB));
+        __syncwarp();
+        factor(j0 + NB, wrap(s0 + NB), min(NB, np - j0 - NB), Lp + (buf ^ 1) * NB * LR);
+      }
+    } else {
+      // write back panel p-1 and fetch the columns of panel p+DPF into its slots
+      // (the thread that reads a slot element issues the copy into it; the U
+      // entries are divided by their rows' pivots afterwards, k_factor_postdiv)
+      const int nf0 = j0 + DPF * NB + K;
+      const int sp = s0 - NB < 0 ? s0 - NB + W : s0 - NB;
+      for (int c = warp - 1; c < NB; c += nw - 1) {
+        T* slot = win + wrap(sp + c) * SW;
+        for (int p = lane; p < SW; p += 32) {
+          if (j0 > 0) band[gidx(j0 - NB + c, p)] = slot[p];
+          if (nf0 + c < np) cp_async_val<T>(slot + p, band + gidx(nf0 + c, p));
         }
       }
-#pragma unroll
-      for (int k = 0; k < NB; k++) {
-        if (k < nb) {
-          const int w = min(K, np - 1 - (j0 + k));
-          const T* lc = win + wrap(s0 + k) * SW + K;
-          T L[R];
-#pragma unroll
-          for (int t = 0; t < R; t++) {
-            const int rr = lane + 32 * t - k;
-            L[t] = (rr >= 1 && rr <= w) ? lc[rr] : T(0);
-          }
-#pragma unroll
-          for (int i = 0; i < CPW; i++) {
-            if (k >= kst[i]) {
-              const T U = __shfl_sync(0xffffffffu, x[i][0], k);
-#pragma unroll
-              for (int t = 0; t < R; t++) {
-                const int rr = lane + 32 * t - k;
-                if (rr >= 1 && rr <= w) x[i][t] -= L[t] * U;
-              }
-            }
-          }
-        }
-      }
-#pragma unroll
-      for (int i = 0; i < CPW; i++) {
-        const int q = q0 + i;
-#pragma unroll
-        for (int t = 0; t < R; t++) {
-          const int pos = K + lane + 32 * t - nb - q;
-          if (q < nt && j0 + lane + 32 * t < np && pos >= 0 && pos <= 2 * K) colp[i][pos] = x[i][t];
-        }
-      }
+      cp_async_commit();
+      for (int q0 = NB + (warp - 1) * CPW; q0 < nt; q0 += (nw - 1) * CPW)
+        update(std::integral_constant<int, CPW>{}, j0, s0, lp, q0, nt);
     }
   }
   if (zero_seen && tid == 0) atomicOr(zero_flag, 1);
@@ -412,10 +423,8 @@ k_factor_panel(const FactorJob* __restrict__ jobs, T* __restrict__ B, T* __restr
   __syncthreads();
   // the last panel: columns [j0 - NB, np) in slots from s0 - NB on
   const int jl = j0 - NB, sl0 = s0 - NB < 0 ? s0 - NB + W : s0 - NB;
-  for (int e = tid; e < (np - jl) * SW; e += blockDim.x) {
-    const int c = e / SW;
-    out(jl + c, wrap(sl0 + c), e - c * SW);
-  }
+  for (int c = warp; c < np - jl; c += nw)
+    for (int p = lane; p < SW; p += 32) band[gidx(jl + c, p)] = win[wrap(sl0 + c) * SW + p];
 }
 
 // Post-divide of the panel kernel's factors (bandLUUL_post_divide,

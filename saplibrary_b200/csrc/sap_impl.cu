@@ -934,11 +934,13 @@ class PrecondT : public PrecBase {
       k_factor_postdiv<T><<<dim3(grid_for((long long)maxrows * Kmax, 256, 1024), (int)jobs.size()), 256, 0, st>>>(
           jobs_d.get(), B.get(), B2.get());
     };
-    auto panel_smem = [&](int dpf) { return (size_t)(Kmax + NB * (1 + dpf)) * (2 * Kmax + 1) * sizeof(T); };
-    if (!ring_only && R <= 4 && panel_smem(1) <= 227 * 1024) {
+    auto panel_smem = [&](int dpf) { return factor_panel_smem<T, NB>(R, Kmax, dpf); };
+    // (a panel's rows in registers: K <= 32 R - NB with R <= 4, or 5 in FP32)
+    if (!ring_only && R <= (sizeof(T) == 4 ? 5 : 4) && panel_smem(1) <= 227 * 1024) {
       const int dpf = panel_smem(2) <= 227 * 1024 ? 2 : 1;
       const size_t psm = panel_smem(dpf);
-      const int nt = 32 * std::min(16, std::max(2, (Kmax + 3) / 4));  // four trailing columns per warp
+      // the chain's warp, and four trailing columns per other warp
+      const int nt = 32 * std::min(16, std::max(3, 1 + (Kmax - NB + 3) / 4));
       auto launch = [&](auto kern) {
         SAPB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)psm));
         kern<<<(int)jobs.size(), nt, psm, st>>>(jobs_d.get(), B.get(), B2.get(), boost ? 1 : 0, flag.get(), dpf);
@@ -948,7 +950,10 @@ class PrecondT : public PrecBase {
         case 1: launch(k_factor_panel<T, NB, 1>); break;
         case 2: launch(k_factor_panel<T, NB, 2>); break;
         case 3: launch(k_factor_panel<T, NB, 3>); break;
-        default: launch(k_factor_panel<T, NB, 4>); break;
+        case 4: launch(k_factor_panel<T, NB, 4>); break;
+        default:
+          if constexpr (sizeof(T) == 4) launch(k_factor_panel<T, NB, 5>);
+          break;
       }
       postdiv();
     } else if (smem <= 200 * 1024) {
