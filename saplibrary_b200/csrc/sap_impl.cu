@@ -259,6 +259,11 @@ class PrecondT : public PrecBase {
     if (wide) fr += wide->bytes_held();  // reused (or released) by the new setup
     const double need = WideBand<T>::factor_bytes(n, P, kmax, h16 && sizeof(T) == 4,
                                                   tf32 && sizeof(T) == 4 && WideBand<T>::tc_gemm_enabled());
+    if (need > 0.92 * (double)fr) {
+      DevicePool::instance().trim();
+      SAPB_CUDA(cudaMemGetInfo(&fr, &tot));
+      if (wide) fr += wide->bytes_held();
+    }
     if (need > 0.92 * (double)fr)
       throw Error(SAP_ERR_OUT_OF_MEMORY, "wide-band factors need " + std::to_string(need / 1e9) + " GB, " +
                                              std::to_string((double)fr / 1e9) + " GB free");
