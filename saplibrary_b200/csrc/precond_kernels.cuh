@@ -32,21 +32,42 @@ struct FactorJob {
 enum { DIR_DOWN = 1, DIR_UP = -1 };
 
 // ---------------------------------------------------------------------------
-// Row-major FP64 band (sap/banded_matrix.h layout) -> column-major FP32 band
-// (bandedMatrixTranspose, sap/device/data_transfer.cuh:733-770).
-template <typename T>
-__global__ void k_band_from_rowmajor(const double* __restrict__ A, T* __restrict__ B, int n, int K) {
+// Row-major FP64 band (sap/banded_matrix.h layout, element (r, c) at
+// A[r (2K+1) + K + c - r]) read by 32 x 32 tiles through shared memory: rows
+// come in along the columns and leave through put(r, c, value) along the rows,
+// both coalesced.  One CTA of 32 x 8 threads takes the rows [r0, r0 + 32) and
+// the columns of [lo, hi) within K of them; rows outside [lo, hi) read as zero.
+template <typename T, class Put>
+__device__ __forceinline__ void band_transpose(const double* __restrict__ A, int K, int r0, int lo, int hi, Put put) {
+  __shared__ T tile[32][33];
   const long long SW = 2LL * K + 1;
-  const long long total = SW * n;
-  for (long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x; e < total;
-       e += (long long)gridDim.x * blockDim.x) {
-    long long c = e / SW;
-    int pos = (int)(e - c * SW);
-    long long r = c + pos - K;
-    T v = 0.f;
-    if (r >= 0 && r < n) v = (T)A[r * SW + (2 * K - pos)];
-    B[e] = v;
+  const int tx = threadIdx.x, ty = threadIdx.y;
+  const int c_end = min(hi, r0 + 32 + K);
+  for (int c0 = lo + (max(r0 - K, lo) - lo) / 32 * 32; c0 < c_end; c0 += 32) {
+#pragma unroll
+    for (int k = 0; k < 32; k += 8) {
+      const int r = r0 + ty + k, c = c0 + tx;
+      tile[ty + k][tx] = (r >= lo && r < hi && c < hi && abs(r - c) <= K) ? (T)A[r * SW + K + c - r] : T(0);
+    }
+    __syncthreads();
+#pragma unroll
+    for (int k = 0; k < 32; k += 8) {
+      const int r = r0 + tx, c = c0 + ty + k;
+      if (c < hi && abs(r - c) <= K) put(r, c, tile[tx][ty + k]);
+    }
+    __syncthreads();
   }
+}
+// -> column-major band (bandedMatrixTranspose,
+// sap/device/data_transfer.cuh:733-770), zeros where a column reaches past the
+// matrix; grid: the row tiles of [-K, n + K).  K = 50, 200,000 rows, FP64: 78 us
+// with one thread per output element.
+template <typename T>
+__global__ void __launch_bounds__(256)
+k_band_from_rowmajor(const double* __restrict__ A, T* __restrict__ B, int n, int K) {
+  const long long SW = 2LL * K + 1;
+  band_transpose<T>(A, K, (int)blockIdx.x * 32 - (K + 31) / 32 * 32, 0, n,
+                    [&](int r, int c, T v) { B[c * SW + K + r - c] = v; });
 }
 
 // Diagonal scaling of the TF32 forms: s_r = 2^k with k = -floor(e / 2) for
@@ -73,6 +94,18 @@ __global__ void k_band_scale(T* __restrict__ B, int n, int K, const T* __restric
     const long long c = e / SW;
     const long long r = c + (e - c * SW) - K;
     if (r >= 0 && r < n) B[e] *= s[r] * s[c];
+  }
+}
+
+// The same scales from a row-major FP64 band.
+template <typename T>
+__global__ void k_diag_pow2_rm(const double* __restrict__ A, int n, int K, T* __restrict__ s) {
+  const long long SW = 2LL * K + 1;
+  for (int r = blockIdx.x * blockDim.x + threadIdx.x; r < n; r += gridDim.x * blockDim.x) {
+    const double d = fabs((double)(T)A[r * SW + K]);
+    int e = 0;
+    if (d > 0 && isfinite(d)) frexp(d, &e);
+    s[r] = (T)ldexp(1.0, -(e >> 1));
   }
 }
 
@@ -107,6 +140,23 @@ __global__ void k_extract_offdiag(const PartDev* __restrict__ parts, const T* __
     if (c <= r) { long long row = s + c, col = s - K + r; cv = B[col * SW + K + (row - col)]; }
     offd[(2 * i) * KK + e] = bv;
     offd[(2 * i + 1) * KK + e] = cv;
+  }
+}
+
+// The same from a row-major FP64 band, scaled by sc (null: not scaled).
+template <typename T>
+__global__ void k_extract_offdiag_rm(const PartDev* __restrict__ parts, const double* __restrict__ A,
+                                     const T* __restrict__ sc, T* __restrict__ offd, int K) {
+  const int i = blockIdx.y;
+  const long long s = parts[i + 1].start, SW = 2LL * K + 1, KK = (long long)K * K;
+  auto el = [&](long long row, long long col) -> T {
+    const T v = (T)A[row * SW + K + col - row];
+    return sc ? v * (sc[row] * sc[col]) : v;
+  };
+  for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < K * K; e += gridDim.x * blockDim.x) {
+    const int c = e / K, r = e % K;
+    offd[(2 * i) * KK + e] = r <= c ? el(s - K + c, s + r) : T(0);
+    offd[(2 * i + 1) * KK + e] = c <= r ? el(s + c, s - K + r) : T(0);
   }
 }
 

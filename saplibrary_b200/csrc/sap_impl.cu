@@ -291,8 +291,8 @@ class PrecondT : public PrecBase {
       pz[p] = parts_h[p].size;
     }
     if (!wide) wide = std::make_unique<WideBand<T>>();
-    wide->init(st, n, WideBand<T>::block_size(kmax, tf32 && sizeof(T) == 4 && WideBand<T>::tc_gemm_enabled()), ps, pz,
-               tf32, h16);
+    wide->init(st, n, WideBand<T>::block_size(kmax, tf32 && sizeof(T) == 4 && WideBand<T>::tc_gemm_enabled()), kmax,
+               ps, pz, tf32, h16);
     wide_active = true;
   }
 
@@ -314,13 +314,41 @@ class PrecondT : public PrecBase {
     n = n_;
     K = K_;
     clamp_partitions_banded();
+    if (K > 0 && use_wide(K) && o.precondType != SAP_PRECOND_NONE) return setup_wide_rowmajor(A_dev);
     B.alloc((size_t)(2 * K + 1) * n);
     auto t1 = Clock::now();
-    k_band_from_rowmajor<T><<<grid_for((long long)(2 * K + 1) * n, 256, 148 * 32), 256, 0, st>>>(A_dev, B.get(), n, K);
+    const long long tiles = ((long long)n + 31) / 32 + 2 * ((K + 31) / 32);  // rows -K .. n + K - 1 and what rounds them up
+    k_band_from_rowmajor<T><<<(unsigned)tiles, dim3(32, 8), 0, st>>>(A_dev, B.get(), n, K);
     SAPB_LAUNCHED();
     SAPB_CUDA(cudaStreamSynchronize(st));
     t_toBanded = ms_since(t1);
     setup_from_band();
+  }
+  // A wide band from its row-major form: scales, coupling blocks and factor
+  // blocks read from it directly.
+  void setup_wide_rowmajor(const double* A_dev) {
+    begin_from_band();
+    auto t0 = Clock::now();
+    if (tf32) {
+      dscaled = true;
+      dscale.alloc(n);
+      k_diag_pow2_rm<T><<<grid_for(n, 256), 256, 0, st>>>(A_dev, n, K, dscale.get());
+      SAPB_LAUNCHED();
+    }
+    if (spike) {
+      offd.alloc((size_t)2 * (P - 1) * K * K);
+      k_extract_offdiag_rm<T><<<dim3(grid_for((long long)K * K, 256, 64), P - 1), 256, 0, st>>>(
+          parts_d.get(), A_dev, dscaled ? dscale.get() : nullptr, offd.get(), K);
+      SAPB_LAUNCHED();
+    }
+    SAPB_CUDA(cudaStreamSynchronize(st));
+    t_offDiags = ms_since(t0);
+    t0 = Clock::now();
+    B.release();
+    wide_init(K);
+    wide->load_rowmajor(A_dev, K, dscaled ? dscale.get() : nullptr);
+    t_toBanded = ms_since(t0);
+    wide_factor_band();
   }
 
   void setup_csr_direct(const Csr& A, int K_) override {
@@ -745,14 +773,34 @@ class PrecondT : public PrecBase {
     build_sweeps();
   }
 
-  void setup_from_band() {
+  void begin_from_band() {
     wide_active = false;
     ptype = o.precondType;
     spike = (ptype == SAP_PRECOND_SPIKE && P > 1);
     lu_ul = spike && o.factMethod == SAP_LU_UL;
     dscaled = false;
+    if (ptype != SAP_PRECOND_NONE) init_parts_const();
+  }
+  // factors, tips and reduced system of a loaded constant wide band
+  void wide_factor_band() {
+    auto t0 = Clock::now();
+    wide->factor(factor_boost());
+    t_bandLU = ms_since(t0);
+    if (!spike) return;
+    std::vector<int> iface((size_t)(P - 1) * 2 * K);
+    for (int i = 0; i < P - 1; i++) {
+      const int s1 = parts_h[i + 1].start;
+      for (int k = 0; k < K; k++) {
+        iface[(size_t)i * 2 * K + k] = s1 - K + k;
+        iface[(size_t)i * 2 * K + K + k] = s1 + k;
+      }
+    }
+    wide_couple(iface);
+  }
+
+  void setup_from_band() {
+    begin_from_band();
     if (ptype == SAP_PRECOND_NONE) return;
-    init_parts_const();
     if (K == 0) return;
     if (tf32 && !reordered) {
       dscaled = true;
@@ -779,20 +827,7 @@ class PrecondT : public PrecBase {
       for (int p = 0; p < P; p++) boff[p] = parts_h[p].boff;
       wide->load_band(B.get(), boff, kp);
       B.release();
-      t0 = Clock::now();
-      wide->factor(factor_boost());
-      t_bandLU = ms_since(t0);
-      if (spike) {
-        std::vector<int> iface((size_t)(P - 1) * 2 * K);
-        for (int i = 0; i < P - 1; i++) {
-          const int s1 = parts_h[i + 1].start;
-          for (int k = 0; k < K; k++) {
-            iface[(size_t)i * 2 * K + k] = s1 - K + k;
-            iface[(size_t)i * 2 * K + K + k] = s1 + k;
-          }
-        }
-        wide_couple(iface);
-      }
+      wide_factor_band();
       return;
     }
     wide.reset();

@@ -7,19 +7,20 @@
 // These are exactly the L and U factors of the band LU (the LU without
 // pivoting is unique), computed as dense block operations: the diagonal block
 // LU is recursive and also returns L_ii^-1 and U_ii^-1, so every step except
-// the leaves (one CTA each, see k_leaf_lu) is a matrix product.  The apply
+// the leaves (one CTA each, see k_leaf) is a matrix product.  The apply
 // then reduces to batched matrix-vector products per block row:
 //     y_i = L_ii^-1 (f_i - L_{i,i-1} y_{i-1}),  x_i = U_ii^-1 (y_i - U_{i,i+1} x_{i+1}).
 // Blocks are column-major (element (r, c) at c*bs + r); vectors are padded to
 // nb*bs rows per partition, padding rows carry an identity diagonal.
 #pragma once
 
+#include <cooperative_groups.h>
 #include <cuda_fp16.h>
 
 #include <cstdlib>
 #include <type_traits>
 
-#include "common.cuh"
+#include "precond_kernels.cuh"
 
 namespace sapb {
 
@@ -83,6 +84,29 @@ __global__ void k_wb_from_band(const T* __restrict__ B, const long long* __restr
   }
 }
 
+// Row-major FP64 band straight into the blocks (all of half-bandwidth K),
+// scaled by sc_r sc_c (null: not scaled); grid (row tile of the partition,
+// partition), 32 x 8 threads.  Saves the column-major band in between: 2M
+// rows, K = 200 took 9.2 ms through it.
+template <typename T>
+__global__ void __launch_bounds__(256)
+k_wb_from_rowmajor(const double* __restrict__ A, int K, const T* __restrict__ sc, const int* __restrict__ pstart,
+                   const int* __restrict__ psize, int bs, int nb, T* __restrict__ Dm, T* __restrict__ Em,
+                   T* __restrict__ Fm) {
+  const int p = blockIdx.y, s = pstart[p], sz = psize[p], r0 = blockIdx.x * 32;
+  if (r0 >= sz) return;
+  const long long BB = (long long)bs * bs;
+  band_transpose<T>(A, K, s + r0, s, s + sz, [&](int r, int c, T v) {
+    if (r >= s + sz) return;
+    if (sc) v *= sc[r] * sc[c];
+    const int a = r - s, b = c - s, bi = a / bs, bj = b / bs;
+    const long long off = (long long)(b - bj * bs) * bs + (a - bi * bs);
+    if (bi == bj) Dm[((long long)p * nb + bi) * BB + off] = v;
+    else if (bj > bi) Em[((long long)p * (nb - 1) + bi) * BB + off] = v;
+    else Fm[((long long)p * (nb - 1) + bj) * BB + off] = v;
+  });
+}
+
 // Batched copy of an m x n sub-matrix (column-major, leading dimensions lds/ldd).
 template <typename T>
 __global__ void k_sub_copy(const T* __restrict__ src, int lds, long long ss, T* __restrict__ dst, int ldd,
@@ -103,151 +127,265 @@ __global__ void k_sub_fill(T* __restrict__ dst, int ldd, long long sd, int m, in
 }
 
 // Leaf of the recursive block LU: one CTA per batch element factors an n x n
-// block (n <= NL) without pivoting (pivots boosted as in the band LU when
-// `boost`, else a pivot below 1e-7 raises zero_flag) and writes L^-1 (unit
-// lower) to Li and U^-1 (upper) to Ui; M is only read.  Both inverses come
-// out of the elimination loop itself (Gauss-Jordan):
-//   * eliminating below the pivot in [A | I] turns I into L^-1, stored in
-//     place of the multipliers (step j sets G[r][j] = -l_r and updates the
-//     columns c < j like the trailing ones);
-//   * eliminating below the diagonal of [U^T | I] (row j of U is final at
-//     step j) turns I into E with U^-T = diag(U)^-1 E, so U^-1 = E^T diag(U)^-1.
-// The working matrix G and E live in registers: thread (ty, tx) of the RY x
-// 32 CTA owns rows ty + RY*i and columns tx + 32*k.  Each step the owners of
-// pivot row j and pivot column j publish them to shared memory (two buffers,
-// so one barrier per step); rows r <= j are skipped per warp.
-template <typename T, int NL, int RY>
-__global__ void __launch_bounds__(RY * 32) k_leaf_lu(const T* __restrict__ M, int ldm, long long sm,
-                                                     T* __restrict__ Li, T* __restrict__ Ui, int ld, long long stride,
-                                                     int n, int boost, int* __restrict__ zero_flag) {
-  constexpr int TM = NL / RY, TN = NL / 32, NT = RY * 32, SP = NL + 1;
-  static_assert(NL % RY == 0 && NL % 32 == 0, "leaf tiling");
-  extern __shared__ __align__(16) unsigned char leaf_smem[];
-  T* S = reinterpret_cast<T*>(leaf_smem);  // NL x SP staging (row-major)
-  T* colj = S + NL * SP;                   // [2][NL] pivot column
-  T* rowj = colj + 2 * NL;                 // [2][NL] pivot row of G
-  T* erow = rowj + 2 * NL;                 // [2][NL] pivot row of E
-  T* piv = erow + 2 * NL;                  // [NL] pivots as used
-  const int t = threadIdx.x, tx = t & 31, ty = t >> 5;
+// block (n <= leaf_max<T>) without pivoting (pivots boosted as in the band LU
+// when `boost`, else a pivot below 1e-7 raises zero_flag) and writes L^-1
+// (unit lower) to Li and U^-1 (upper) to Ui; M is only read.
+//
+// The whole block stays in shared memory (row-major, ld = n16 + 4), as 16 x 16
+// tiles, one warp per tile and product:
+//   * 16 pivots at a time: warp 0 factors the diagonal tile in registers and
+//     inverts its triangles (tile_lu), which take the tile's place in G; the
+//     panels U12 = L^-1 A12 and L21 = A21 U^-1 follow, then A22 -= L21 U12,
+//     where warp 0 takes the next diagonal tile and factors it at once while
+//     the other warps update the rest;
+//   * the inverses of the two triangular factors grow by doubling, 16 -> 32 ->
+//     64 -> 128: (L^-1)21 = -L22^-1 (L21 L11^-1), (U^-1)12 = -U11^-1 (U12
+//     U22^-1), all pairs and both triangles at once, in place of L21 and U12.
+// What bounds it is this chain of phases in one CTA per partition; larger
+// leaves replace whole levels of the recursion, whose products cost a launch
+// each (about 5 us, six on the chain of every level).
+//
+// tc: products between tiles of different 32-blocks run on the tensor cores
+// in TF32 (mma.sync, FP32 accumulation), like the products of the recursion
+// they stand for; within a 32-block, and without tc everywhere, they are FMAs
+// in T.
+template <typename T>
+constexpr int leaf_max = sizeof(T) == 4 ? 128 : 96;  // two n x (n + 4) arrays of shared memory
+constexpr int kLeafThreads = 512;
+template <typename T>
+inline size_t leaf_smem(int n) {
+  const int n16 = (n + 15) / 16 * 16;
+  return (size_t)2 * n16 * (n16 + 4) * sizeof(T);
+}
+enum { TILE_FULL = 0, TILE_UNIT_LOWER = 1, TILE_UPPER = 2 };
+// element (r, c) of a 16 x 16 tile of G read as full, unit lower or upper
+template <typename T>
+__device__ __forceinline__ T tile_el(const T* A, int ld, int r, int c, int tri) {
+  const T v = A[r * ld + c];
+  if (tri == TILE_UNIT_LOWER) return r > c ? v : (r == c ? T(1) : T(0));
+  if (tri == TILE_UPPER) return r <= c ? v : T(0);
+  return v;
+}
+__device__ __forceinline__ unsigned to_tf32(float v) {
+  unsigned r;
+  asm("cvt.rna.tf32.f32 %0, %1;" : "=r"(r) : "f"(v));
+  return r;
+}
+// acc += A B for 16 x 16 tiles, one warp.  Lane (g, t) = (lane / 4, lane % 4)
+// holds rows g, g + 8 and columns 2t, 2t+1, 8+2t, 9+2t (the accumulator layout
+// of mma.m16n8k8): acc[4 h + 2 i + j] = (g + 8 i, 8 h + 2 t + j).
+template <typename T>
+__device__ __forceinline__ void tile_mac(const T* A, int triA, const T* B, int triB, int ld, bool tc, T acc[8]) {
+  const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+  if constexpr (sizeof(T) == 4) {
+    if (tc) {
+#pragma unroll
+      for (int k = 0; k < 16; k += 8) {
+        const unsigned a0 = to_tf32(tile_el(A, ld, g, k + t, triA)), a1 = to_tf32(tile_el(A, ld, g + 8, k + t, triA)),
+                       a2 = to_tf32(tile_el(A, ld, g, k + t + 4, triA)),
+                       a3 = to_tf32(tile_el(A, ld, g + 8, k + t + 4, triA));
+#pragma unroll
+        for (int h = 0; h < 2; h++) {
+          const unsigned b0 = to_tf32(tile_el(B, ld, k + t, 8 * h + g, triB)),
+                         b1 = to_tf32(tile_el(B, ld, k + t + 4, 8 * h + g, triB));
+          asm("mma.sync.aligned.m16n8k8.row.col.f32.tf32.tf32.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, "
+              "{%0,%1,%2,%3};"
+              : "+f"(acc[4 * h]), "+f"(acc[4 * h + 1]), "+f"(acc[4 * h + 2]), "+f"(acc[4 * h + 3])
+              : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+        }
+      }
+      return;
+    }
+  }
+#pragma unroll
+  for (int k = 0; k < 16; k++) {
+    const T a0 = tile_el(A, ld, g, k, triA), a1 = tile_el(A, ld, g + 8, k, triA);
+#pragma unroll
+    for (int h = 0; h < 2; h++)
+#pragma unroll
+      for (int j = 0; j < 2; j++) {
+        const T bv = tile_el(B, ld, k, 8 * h + 2 * t + j, triB);
+        acc[4 * h + j] = fma(a0, bv, acc[4 * h + j]);
+        acc[4 * h + 2 + j] = fma(a1, bv, acc[4 * h + 2 + j]);
+      }
+  }
+}
+template <typename T>
+__device__ __forceinline__ void tile_store(T* C, int ld, const T acc[8], T alpha) {
+  const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+#pragma unroll
+  for (int h = 0; h < 2; h++)
+#pragma unroll
+    for (int i = 0; i < 2; i++)
+#pragma unroll
+      for (int j = 0; j < 2; j++) C[(g + 8 * i) * ld + 8 * h + 2 * t + j] = alpha * acc[4 * h + 2 * i + j];
+}
+template <typename T>
+__device__ __forceinline__ void tile_sub(T* C, int ld, const T acc[8]) {
+  const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+#pragma unroll
+  for (int h = 0; h < 2; h++)
+#pragma unroll
+    for (int i = 0; i < 2; i++)
+#pragma unroll
+      for (int j = 0; j < 2; j++) C[(g + 8 * i) * ld + 8 * h + 2 * t + j] -= acc[4 * h + 2 * i + j];
+}
+// One warp: LU of the 16 x 16 tile A (the first n pivots count for the zero
+// check), then A's strict lower part <- L^-1, its upper part <- U^-1.  Lane l
+// holds row l % 16; lanes 0..15 then solve for a column of L^-1, lanes 16..31
+// for a column of U^-1.
+template <typename T>
+__device__ __forceinline__ void tile_lu(T* A, int ld, int n, int boost, int* zero_flag) {
+  const unsigned full = 0xffffffffu;
+  const int lane = threadIdx.x & 31, r = lane & 15;
+  T a[16];
+#pragma unroll
+  for (int c = 0; c < 16; c++) a[c] = A[r * ld + c];
+  bool zero = false;
+#pragma unroll
+  for (int k = 0; k < 16; k++) {
+    T p = __shfl_sync(full, a[k], k);
+    if (boost) p = boost_pivot(p);
+    else zero |= k < n && fabs((double)p) < 1e-7;
+    const T inv = T(1) / p;
+    const T l = r > k ? a[k] * inv : T(0);
+#pragma unroll
+    for (int c = k + 1; c < 16; c++) a[c] = fma(-l, __shfl_sync(full, a[c], k), a[c]);
+    a[k] = r > k ? l : (r == k ? p : a[k]);
+  }
+  if (zero && lane == 0) atomicOr(zero_flag, 1);
+  // both solves run in every lane (the shuffles need the whole warp)
+  T xl[16], xu[16];
+#pragma unroll
+  for (int i = 0; i < 16; i++) {
+    T v = i == r ? T(1) : T(0);
+#pragma unroll
+    for (int k = 0; k < i; k++) v = fma(-__shfl_sync(full, a[k], i), xl[k], v);
+    xl[i] = v;
+  }
+#pragma unroll
+  for (int i = 15; i >= 0; i--) {
+    T v = i == r ? T(1) : T(0);
+#pragma unroll
+    for (int k = i + 1; k < 16; k++) v = fma(-__shfl_sync(full, a[k], i), xu[k], v);
+    xu[i] = v / __shfl_sync(full, a[i], i);
+  }
+#pragma unroll
+  for (int i = 0; i < 16; i++) {
+    if (lane < 16 && i > r) A[i * ld + r] = xl[i];
+    if (lane >= 16 && i <= r) A[i * ld + r] = xu[i];
+  }
+}
+template <typename T>
+__global__ void __launch_bounds__(kLeafThreads)
+k_leaf(const T* __restrict__ M, int ldm, long long sm, T* __restrict__ Li, T* __restrict__ Ui, int ldo,
+       long long stride, int n, int boost, int* __restrict__ zero_flag, int tc) {
+  extern __shared__ __align__(16) unsigned char leaf_raw[];
+  const int nt = (n + 15) / 16, n16 = nt * 16, ld = n16 + 4;
+  T* G = reinterpret_cast<T*>(leaf_raw);
+  T* X = G + n16 * ld;
+  const int t = threadIdx.x, lane = t & 31, warp = t >> 5, nw = blockDim.x >> 5;
   const T* Mb = M + blockIdx.x * sm;
   T* Lb = Li + blockIdx.x * stride;
   T* Ub = Ui + blockIdx.x * stride;
-  for (int idx = t; idx < n * n; idx += NT) {
-    const int c = idx / n, r = idx - c * n;
-    S[r * SP + c] = Mb[(long long)c * ldm + r];
-  }
+  for (int c = warp; c < n16; c += nw)
+    for (int r = lane; r < n16; r += 32)
+      G[r * ld + c] = (r < n && c < n) ? Mb[(long long)c * ldm + r] : (r == c ? T(1) : T(0));
   __syncthreads();
-  T g[TM][TN], e[TM][TN];
-#pragma unroll
-  for (int i = 0; i < TM; i++)
-#pragma unroll
-    for (int k = 0; k < TN; k++) {
-      const int r = ty + RY * i, c = tx + 32 * k;
-      g[i][k] = (r < n && c < n) ? S[r * SP + c] : (r == c ? T(1) : T(0));
-      e[i][k] = r == c ? T(1) : T(0);
-    }
-  for (int j = 0; j < n; j++) {
-    const int b = (j & 1) * NL;
-    if (tx == (j & 31)) {  // owners of column j
-      const int kj = j >> 5;
-#pragma unroll
-      for (int i = 0; i < TM; i++) {
-        T v = g[i][0];
-#pragma unroll
-        for (int k = 1; k < TN; k++)
-          if (kj == k) v = g[i][k];
-        colj[b + ty + RY * i] = v;
+  auto tile = [&](T* Z, int i, int j) { return Z + (16 * i) * ld + 16 * j; };
+  auto apart = [&](int i, int j) { return tc && (i >> 1) != (j >> 1); };
+  if (warp == 0) tile_lu(tile(G, 0, 0), ld, n, boost, zero_flag);
+  __syncthreads();
+  for (int k = 0; k < nt; k++) {
+    const int m = nt - 1 - k;
+    for (int q = warp; q < 2 * m; q += nw) {  // panels, in place
+      const int j = k + 1 + (q >> 1);
+      T acc[8] = {};
+      T* P;
+      if (q & 1) {
+        P = tile(G, j, k);
+        tile_mac(P, TILE_FULL, tile(G, k, k), TILE_UPPER, ld, apart(j, k), acc);
+      } else {
+        P = tile(G, k, j);
+        tile_mac(tile(G, k, k), TILE_UNIT_LOWER, P, TILE_FULL, ld, apart(j, k), acc);
       }
-    }
-    if (ty == j % RY) {  // owners of row j
-      const int ij = j / RY;
-#pragma unroll
-      for (int k = 0; k < TN; k++) {
-        T v = g[0][k], w = e[0][k];
-#pragma unroll
-        for (int i = 1; i < TM; i++)
-          if (ij == i) {
-            v = g[i][k];
-            w = e[i][k];
-          }
-        rowj[b + tx + 32 * k] = v;
-        erow[b + tx + 32 * k] = w;
-      }
+      __syncwarp();
+      tile_store(P, ld, acc, T(1));
     }
     __syncthreads();
-    T p = rowj[b + j];
-    if (boost) p = boost_pivot(p);
-    if (t == 0) {
-      piv[j] = p;
-      if (!boost && fabs((double)p) < 1e-7) atomicOr(zero_flag, 1);
+    auto trail = [&](int i, int j) {
+      T acc[8] = {};
+      // (a pivot tile of another 32-block is a product of the recursion)
+      tile_mac(tile(G, i, k), TILE_FULL, tile(G, k, j), TILE_FULL, ld, tc && (apart(i, k) || apart(j, k)), acc);
+      tile_sub(tile(G, i, j), ld, acc);
+    };
+    if (m > 0) {
+      if (warp == 0) {
+        trail(k + 1, k + 1);
+        __syncwarp();
+        tile_lu(tile(G, k + 1, k + 1), ld, n - 16 * (k + 1), boost, zero_flag);
+      } else {
+        for (int q = warp; q < m * m; q += nw - 1) trail(k + 1 + q / m, k + 1 + q % m);
+      }
+      __syncthreads();
     }
-    const T inv = T(1) / p;
-    T xr[TN], xe[TN];
-#pragma unroll
-    for (int k = 0; k < TN; k++) {
-      xr[k] = rowj[b + tx + 32 * k];
-      xe[k] = erow[b + tx + 32 * k];
-    }
-#pragma unroll
-    for (int i = 0; i < TM; i++) {
-      const int r = ty + RY * i;
-      if (r > j) {  // uniform across the warp
-        const T l = colj[b + r] * inv, m = rowj[b + r] * inv;
-#pragma unroll
-        for (int k = 0; k < TN; k++) {
-          const int c = tx + 32 * k;
-          g[i][k] = (c == j) ? -l : g[i][k] - l * xr[k];
-          if (c <= j) e[i][k] -= m * xe[k];
+  }
+  // inverses by doubling: blocks of s tiles, pairs (2s tiles); the second of a
+  // pair may be cut off by n
+  for (int s = 1; s < nt; s *= 2) {
+    const int pairs = (nt + 2 * s - 1) / (2 * s), per = s * s;
+    for (int phase = 0; phase < 2; phase++) {
+      for (int q = warp; q < pairs * per * 2; q += nw) {
+        const bool up = q & 1;
+        const int e = q >> 1, pr = e / per, i = (e % per) / s, j = (e % per) % s, o = pr * 2 * s, o2 = o + s;
+        const int s2 = min(s, nt - o2);  // tiles of the second block
+        if (s2 <= 0) continue;
+        T acc[8] = {};
+        if (!up) {  // (i, j): rows o2 + i (i < s2), columns o + j
+          if (i >= s2) continue;
+          if (phase == 0) {  // T = L21 L11^-1
+            for (int k = j; k < s; k++)
+              tile_mac(tile(G, o2 + i, o + k), TILE_FULL, tile(G, o + k, o + j), k == j ? TILE_UNIT_LOWER : TILE_FULL,
+                       ld, tc && s > 1, acc);
+            tile_store(tile(X, o2 + i, o + j), ld, acc, T(1));
+          } else {  // (L^-1)21 = -L22^-1 T
+            for (int k = 0; k <= i; k++)
+              tile_mac(tile(G, o2 + i, o2 + k), k == i ? TILE_UNIT_LOWER : TILE_FULL, tile(X, o2 + k, o + j),
+                       TILE_FULL, ld, tc && s > 1, acc);
+            tile_store(tile(G, o2 + i, o + j), ld, acc, T(-1));
+          }
+        } else {  // (i, j): rows o + i, columns o2 + j (j < s2)
+          if (j >= s2) continue;
+          if (phase == 0) {  // T = U12 U22^-1
+            for (int k = 0; k <= j; k++)
+              tile_mac(tile(G, o + i, o2 + k), TILE_FULL, tile(G, o2 + k, o2 + j), k == j ? TILE_UPPER : TILE_FULL, ld,
+                       tc && s > 1, acc);
+            tile_store(tile(X, o + i, o2 + j), ld, acc, T(1));
+          } else {  // (U^-1)12 = -U11^-1 T
+            for (int k = i; k < s; k++)
+              tile_mac(tile(G, o + i, o + k), k == i ? TILE_UPPER : TILE_FULL, tile(X, o + k, o2 + j), TILE_FULL, ld,
+                       tc && s > 1, acc);
+            tile_store(tile(G, o + i, o2 + j), ld, acc, T(-1));
+          }
         }
       }
+      __syncthreads();
     }
   }
-  __syncthreads();
-  // L^-1: unit diagonal, strict lower part of G
-#pragma unroll
-  for (int i = 0; i < TM; i++)
-#pragma unroll
-    for (int k = 0; k < TN; k++) {
-      const int r = ty + RY * i, c = tx + 32 * k;
-      S[r * SP + c] = r > c ? g[i][k] : (r == c ? T(1) : T(0));
+  for (int c = warp; c < n; c += nw)
+    for (int r = lane; r < n; r += 32) {
+      const T v = G[r * ld + c];
+      Lb[(long long)c * ldo + r] = r > c ? v : (r == c ? T(1) : T(0));
+      Ub[(long long)c * ldo + r] = r <= c ? v : T(0);
     }
-  __syncthreads();
-  for (int idx = t; idx < n * n; idx += NT) {
-    const int c = idx / n, r = idx - c * n;
-    Lb[(long long)c * ld + r] = S[r * SP + c];
-  }
-  __syncthreads();
-  // U^-1 (row c, column r) = E[r][c] / u_rr for c <= r
-#pragma unroll
-  for (int i = 0; i < TM; i++)
-#pragma unroll
-    for (int k = 0; k < TN; k++) {
-      const int r = ty + RY * i, c = tx + 32 * k;
-      S[c * SP + r] = (c <= r && r < n) ? e[i][k] / piv[r] : T(0);
-    }
-  __syncthreads();
-  for (int idx = t; idx < n * n; idx += NT) {
-    const int c = idx / n, r = idx - c * n;
-    Ub[(long long)c * ld + r] = S[r * SP + c];
-  }
 }
 
-// CTA rows (warps) and shared memory of k_leaf_lu for a leaf of NL
-// (register budget: 2 * TM * TN values per thread).
-template <typename T, int NL>
-struct LeafShape {
-  static constexpr int RY = NL >= 64 ? 16 : 8;
-  static constexpr size_t smem = (size_t)(NL * (NL + 1) + 7 * NL) * sizeof(T);
-};
-// Largest leaf: 32 (measured on the 1M-row workload's 3168 / 3040 blocks:
-// TF32 block LU 190 ms with 32, 192 with 64, 215 with 128; FP64 1029 / 1040
-// with 32 / 64); SAPB_LEAF = 64 / 128 (128 for FP32 only) overrides.
+// Largest leaf of the recursion (SAPB_LEAF: a smaller one).
 template <typename T>
 inline int leaf_size() {
   const char* e = std::getenv("SAPB_LEAF");
   const int v = e ? std::atoi(e) : 0;
-  if (v == 32 || v == 64 || (v == 128 && sizeof(T) == 4)) return v;
-  return 32;
+  return v >= 32 && v <= leaf_max<T> ? v / 32 * 32 : leaf_max<T>;
 }
 
 // Batched dense matrix-vector product with an n x n column-major block:
@@ -595,6 +733,175 @@ __global__ void __launch_bounds__(kGemvWarps * 32, 3) k_sweep(const MT* __restri
       tgemv_item<T, VEC, MT, true>(it / S, p, S, it % S, A, bs, xv, cv, yv, bs, mode, tri, ws, ctr, cs, part,
                                    last_cta);
     if (!group_barrier(bar + 2 * p, bar + 2 * p + 1, (unsigned)(G + stall), err)) return;
+  }
+}
+
+// One whole block sweep for small blocks: a cluster of C CTAs per partition,
+// the vectors exchanged through distributed shared memory.
+//
+// With blocks of a few hundred rows a step of the sweep moves some 100 KB per
+// CTA, so what bounds the schedules above is the latency of a step: the first
+// loads after each barrier, the partial sums and the barrier in global memory
+// (10.4 us per step at 448-row blocks, 32 partitions).  Here every CTA keeps
+// its share of the next step's factor block on the way into registers while
+// the current step's sums are exchanged: the loads do not depend on the chain.
+// Columns go round the 16 C warps of the cluster (column c to warp c mod 16 C),
+// which balances the triangles; a lane holds V rows of a 32 V-row tile, one
+// 16-byte load per column and tile.  Each CTA adds its warps' partial rows and
+// sends them to every CTA of the cluster; one cluster barrier later all add the
+// C shares in the same order, so all hold the same vector.
+//
+// kc: the off-diagonal factor blocks are zero outside their kc x kc corner
+// (L_{i+1,i}: rows < kc, columns >= bs - kc; U_{i,i+1}: the transpose), which
+// is all that is read.  bs <= 16 C JM columns and 32 V NT rows.
+template <typename T, int V, typename MT, int C, int JM, int NT>
+struct SweepRegs {
+  using Vec = typename VecOf<MT, V>::type;
+  static constexpr int W = kGemvWarps * C;  // columns per group
+  static constexpr int TR = 32 * V;
+  // (j, tile) is read by some column of group j: lower triangles from the
+  // tile of column W j on, upper triangles up to the tile of column W j + W-1
+  static constexpr bool need(bool lower, int j, int tile) {
+    return lower ? tile >= W * j / TR : tile <= (W * j + W - 1) / TR;
+  }
+};
+template <typename T, int V, typename MT, int C, int JM, int NT>
+__global__ void __launch_bounds__(kGemvWarps * 32, 1)
+k_sweep_cluster(const MT* __restrict__ Li, const MT* __restrict__ Ui, const MT* __restrict__ Lo,
+                const MT* __restrict__ Uo, const T* __restrict__ csL, const T* __restrict__ csU,
+                const T* __restrict__ csLo, const T* __restrict__ csUo, T* x, T* y, int nb, int bs, int kc,
+                long long BB, long long plen) {
+  using S = SweepRegs<T, V, MT, C, JM, NT>;
+  using Vec = typename S::Vec;
+  constexpr int W = S::W, TR = S::TR, ROWS = TR * NT;
+  constexpr bool scaled = !std::is_same<MT, T>::value;
+  extern __shared__ __align__(16) unsigned char sweep_raw[];
+  T* part = reinterpret_cast<T*>(sweep_raw);  // [kGemvWarps][ROWS]
+  T* xch = part + kGemvWarps * ROWS;          // [2][C][ROWS]
+  T* xs = xch + 2 * C * ROWS;                 // [ROWS]
+  const auto cluster = cooperative_groups::this_cluster();
+  const int rank = (int)cluster.block_rank(), p = blockIdx.x / C;
+  const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5, c0 = rank * kGemvWarps + w;
+  const long long bd = (long long)p * nb, bo = (long long)p * (nb - 1);
+  T* xp = x + p * plen;
+  T* yp = y + p * plen;
+  Vec a[JM][NT];
+  T sc[JM];
+  // the warp's columns of a block: rows [r0, r1), columns [k0, k1)
+  auto load = [&](auto lower, const MT* A, const T* cs, int r0, int r1, int k0, int k1) {
+    const MT* q = A + c0 * bs + V * lane;
+#pragma unroll
+    for (int j = 0; j < JM; j++, q += W * bs) {
+      const int col = W * j + c0;
+      const bool in = col >= k0 && col < k1;
+      if constexpr (scaled) sc[j] = in ? __ldg(cs + col) : T(0);
+#pragma unroll
+      for (int t = 0; t < NT; t++)
+        if (S::need(decltype(lower)::value, j, t)) {
+          const int r = TR * t + V * lane;
+          // (the triangle's empty side of a tile row is never read)
+          const bool tri = decltype(lower)::value ? TR * (t + 1) > col : TR * t <= col;
+          a[j][t] = in && tri && r >= r0 && r < r1 ? __ldg(reinterpret_cast<const Vec*>(q + TR * t)) : Vec{};
+        }
+    }
+  };
+  int buf = 0;
+  // xs <- (c ? c - A xs : A xs) for the block held in a; c: this thread's value
+  auto apply = [&](auto lower, bool minus, T cv, auto prefetch) {
+    T acc[NT][V];
+#pragma unroll
+    for (int t = 0; t < NT; t++)
+#pragma unroll
+      for (int v = 0; v < V; v++) acc[t][v] = T(0);
+#pragma unroll
+    for (int j = 0; j < JM; j++) {
+      const int col = W * j + c0;
+      T xv = col < bs ? xs[col] : T(0);
+      if constexpr (scaled) xv *= sc[j];
+#pragma unroll
+      for (int t = 0; t < NT; t++)
+        if (S::need(decltype(lower)::value, j, t)) vec_fma<T>(a[j][t], xv, acc[t]);
+    }
+    prefetch();
+#pragma unroll
+    for (int t = 0; t < NT; t++)
+#pragma unroll
+      for (int v = 0; v < V; v++) part[w * ROWS + TR * t + V * lane + v] = acc[t][v];
+    __syncthreads();
+    for (int r = tid; r < bs; r += kGemvWarps * 32) {
+      T s = T(0);
+#pragma unroll
+      for (int k = 0; k < kGemvWarps; k++) s += part[k * ROWS + r];
+#pragma unroll
+      for (int q = 0; q < C; q++) cluster.map_shared_rank(xch, q)[(buf * C + rank) * ROWS + r] = s;
+    }
+    cluster.sync();
+    for (int r = tid; r < bs; r += kGemvWarps * 32) {
+      T s = T(0);
+#pragma unroll
+      for (int q = 0; q < C; q++) s += xch[(buf * C + q) * ROWS + r];
+      xs[r] = minus ? cv - s : s;
+    }
+    buf ^= 1;
+    __syncthreads();
+  };
+  const std::true_type LO{};
+  const std::false_type UP{};
+  static_assert(ROWS <= kGemvWarps * 32, "one row per thread");
+  load(LO, Li + bd * BB, scaled ? csL + bd * bs : nullptr, 0, bs, 0, bs);
+  if (tid < bs) xs[tid] = xp[tid];
+  __syncthreads();
+  for (int i = 0; i < nb; i++) {  // y_i = L_ii^-1 (x_i - L_{i,i-1} y_{i-1})
+    const bool more = i + 1 < nb;
+    T cv = T(0);
+    apply(LO, false, T(0), [&] {
+      if (more) {
+        load(UP, Lo + (bo + i) * BB, scaled ? csLo + (bo + i) * bs : nullptr, 0, kc, bs - kc, bs);
+        if (tid < bs) cv = xp[(long long)(i + 1) * bs + tid];
+      } else {
+        load(UP, Ui + (bd + i) * BB, scaled ? csU + (bd + i) * bs : nullptr, 0, bs, 0, bs);
+      }
+    });
+    if (!more) break;
+    if (rank == 0 && tid < bs) yp[(long long)i * bs + tid] = xs[tid];
+    apply(UP, true, cv, [&] {
+      load(LO, Li + (bd + i + 1) * BB, scaled ? csL + (bd + i + 1) * bs : nullptr, 0, bs, 0, bs);
+    });
+  }
+  // x_i = U_ii^-1 (y_i - U_{i,i+1} x_{i+1}); rank 0 wrote the y_i: its writes
+  // reach the other CTAs through the cluster barriers that followed
+  for (int i = nb - 1; i >= 0; i--) {
+    const bool more = i > 0;
+    T cv = T(0);
+    apply(UP, false, T(0), [&] {
+      if (more) {
+        load(LO, Uo + (bo + i - 1) * BB, scaled ? csUo + (bo + i - 1) * bs : nullptr, bs - kc, bs, 0, kc);
+        if (tid < bs) cv = __ldcg(yp + (long long)(i - 1) * bs + tid);
+      }
+    });
+    if (rank == 0 && tid < bs) xp[(long long)i * bs + tid] = xs[tid];
+    if (!more) break;
+    apply(LO, true, cv, [&] {
+      load(UP, Ui + (bd + i - 1) * BB, scaled ? csU + (bd + i - 1) * bs : nullptr, 0, bs, 0, bs);
+    });
+  }
+  cluster.sync();  // no CTA leaves while another may still write to it
+}
+
+// D <- L, L <- 0, U <- 0 for the bs x bs blocks of every batch element (L and D
+// may have different batch strides; all 16-byte aligned)
+template <typename T>
+__global__ void k_take_block(T* __restrict__ L, T* __restrict__ U, long long sl, T* __restrict__ D, long long sd,
+                             long long count) {
+  uint4* l = reinterpret_cast<uint4*>(L + blockIdx.y * sl);
+  uint4* u = reinterpret_cast<uint4*>(U + blockIdx.y * sl);
+  uint4* d = reinterpret_cast<uint4*>(D + blockIdx.y * sd);
+  const long long m = count * (long long)sizeof(T) / 16;
+  const uint4 z = make_uint4(0, 0, 0, 0);
+  for (long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x; e < m; e += (long long)gridDim.x * blockDim.x) {
+    d[e] = l[e];
+    l[e] = z;
+    u[e] = z;
   }
 }
 

@@ -212,18 +212,10 @@ class BlockLU {
     const int n1 = split(n), n2 = n - n1;
     return std::max(rec_ws(n1, leaf), (long long)n1 * n2 + (long long)pad4(n2) * n1 + rec_ws(n2, leaf));
   }
-  template <int NL>
   void leaf_launch(Mat<T> M, Mat<T> Li, Mat<T> Ui, int n) {
-    using LS = LeafShape<T, NL>;
-    static bool smem_set = false;  // first call runs outside any graph capture
-    if (!smem_set) {
-      SAPB_CUDA(cudaFuncSetAttribute(k_leaf_lu<T, NL, LS::RY>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                     (int)LS::smem));
-      smem_set = true;
-    }
     SAPB_PROF("wb_leaf", st);
-    k_leaf_lu<T, NL, LS::RY><<<batch, LS::RY * 32, LS::smem, st>>>(M.p, M.ld, M.s, Li.p, Ui.p, Li.ld, Li.s, n,
-                                                                    boost ? 1 : 0, flag);
+    k_leaf<T><<<batch, kLeafThreads, leaf_smem<T>(n), st>>>(M.p, M.ld, M.s, Li.p, Ui.p, Li.ld, Li.s, n, boost ? 1 : 0,
+                                                            flag, tc ? 1 : 0);
     SAPB_LAUNCHED();
   }
 
@@ -233,9 +225,7 @@ class BlockLU {
   void rec(Mat<T> M, Mat<T> Li, Mat<T> Ui, int n, long long wo = 0) {
     if (n <= leaf) {
       if (Li.s != Ui.s || Li.ld != Ui.ld) throw Error(SAP_ERR_INVALID_ARGUMENT, "leaf inverse layouts differ");
-      if (leaf <= 32) leaf_launch<32>(M, Li, Ui, n);
-      else if (leaf <= 64 || sizeof(T) != 4) leaf_launch<64>(M, Li, Ui, n);
-      else leaf_launch<(sizeof(T) == 4 ? 128 : 64)>(M, Li, Ui, n);
+      leaf_launch(M, Li, Ui, n);
       return;
     }
     const int n1 = split(n), n2 = n - n1;
@@ -275,6 +265,9 @@ class WideBand {
   cublasHandle_t h = nullptr;
   cudaStream_t st = nullptr;
   int n = 0, P = 0, bs = 0, nb = 0, K = 0;  // K: width of the coupling blocks
+  // the off-diagonal blocks E_i, F_i and their factors are zero outside a
+  // kc x kc corner (E: bottom left, F: top right): the half-bandwidth, rounded up
+  int kc = 0;
   int ldK = 0;                               // leading dimension of the K x K blocks (16-byte multiple)
   long long sK = 0;                          // their batch stride, ldK * K
   bool spike = false;
@@ -329,7 +322,7 @@ class WideBand {
   // (every buffer it touches is kept across setups of the layout).
   cudaGraphExec_t fgraph = nullptr;
   long long fgraph_key = -1;
-  int fgraph_cut = 0, fgraph_leaf = 0;
+  int fgraph_cut = 0, fgraph_leaf = 0, fgraph_kc = 0;
   // SAPB_FACTOR_GRAPH=0 runs the factorization's launches directly every time
   static bool graph_enabled() {
     const char* e = std::getenv("SAPB_FACTOR_GRAPH");
@@ -473,7 +466,8 @@ class WideBand {
     lu.gerr = gemm_err.get();
   }
 
-  void init(cudaStream_t s, int n_, int bs_, const std::vector<int>& pstart, const std::vector<int>& psize,
+  // kmax: the largest half-bandwidth; the blocks may be larger (block_size)
+  void init(cudaStream_t s, int n_, int bs_, int kmax, const std::vector<int>& pstart, const std::vector<int>& psize,
             bool tf32_ = false, bool h16_ = false) {
     st = s;
     tf32 = tf32_ && sizeof(T) == 4;
@@ -481,6 +475,7 @@ class WideBand {
     n = n_;
     P = (int)pstart.size();
     bs = bs_;
+    kc = std::min(bs, (kmax + kLeaf - 1) / kLeaf * kLeaf);
     pstart_h = pstart;
     psize_h = psize;
     if (!h) cublas_check(cublasCreate(&h), "cublasCreate");
@@ -509,6 +504,8 @@ class WideBand {
       gemm_err.zero(st);
     }
     if (tc_on()) umma::prepare();  // kernel attributes, before any capture
+    SAPB_CUDA(cudaFuncSetAttribute(k_leaf<T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                   (int)leaf_smem<T>(leaf_max<T>)));
     int maxsz = 0;
     for (int v : psize) maxsz = std::max(maxsz, v);
     nb = std::max(1, (maxsz + bs - 1) / bs);
@@ -556,6 +553,15 @@ class WideBand {
     pad();
     SAPB_CUDA(cudaStreamSynchronize(st));
   }
+  void load_rowmajor(const double* A, int K_, const T* sc) {
+    int maxsz = 1;
+    for (int v : psize_h) maxsz = std::max(maxsz, v);
+    k_wb_from_rowmajor<T><<<dim3((maxsz + 31) / 32, P), dim3(32, 8), 0, st>>>(
+        A, K_, sc, pstart_d.get(), psize_d.get(), bs, nb, Linv.get(), Uoff.get(), Loff.get());
+    SAPB_LAUNCHED();
+    pad();
+    SAPB_CUDA(cudaStreamSynchronize(st));
+  }
   void load_coo(const int* rows, const int* cols, const T* vals, long long nz) {
     k_wb_scatter<T><<<grid1d(nz), 256, 0, st>>>(rows, cols, vals, nz, rowpart_d.get(), pstart_d.get(), psize_d.get(),
                                                  bs, nb, Linv.get(), Uoff.get(), Loff.get());
@@ -573,7 +579,8 @@ class WideBand {
     Rw.alloc((size_t)P * std::max(1LL, BlockLU<T>::rec_ws(bs, leaf_size<T>())));
     flag.alloc(1);
     const long long key = (((long long)P * 65537 + bs) * 65537 + nb) * 4 + (boost ? 2 : 0) + (tf32 ? 1 : 0);
-    if (key != fgraph_key || factor_cut() != fgraph_cut || leaf_size<T>() != fgraph_leaf) {
+    if (key != fgraph_key || kc != fgraph_kc || factor_cut() != fgraph_cut || leaf_size<T>() != fgraph_leaf) {
+      fgraph_kc = kc;
       fgraph_cut = factor_cut();
       fgraph_leaf = leaf_size<T>();
       if (fgraph) cudaGraphExecDestroy(fgraph);
@@ -639,13 +646,14 @@ class WideBand {
       const Mat<T> Li = blk(Linv, nb, i), Ui = blk(Uinv, nb, i);
       {
         SAPB_PROF("wb_copy", st);
-        lu.copy(Li, D, bs, bs);  // D_i (loaded into the L_ii^-1 slot)
-        lu.fill(Li, bs, bs, T(0));
-        lu.fill(Ui, bs, bs, T(0));
+        // D_i, loaded into the L_ii^-1 slot, to the workspace; both inverses start from zero
+        k_take_block<T><<<dim3(grid1d(BB * (long long)sizeof(T) / 16, 256, std::max(8, 148 * 8 / P)), P), 256, 0, st>>>(
+            Li.p, Ui.p, Li.s, D.p, D.s, BB);
+        SAPB_LAUNCHED();
       }
-      if (i > 0) {  // D_i -= L_{i,i-1} U_{i-1,i}: upper times lower
+      if (i > 0) {  // D_i -= L_{i,i-1} U_{i-1,i}: upper times lower, in the corner
         SAPB_PROF("wb_schur", st);
-        lu.prod_UL_acc(bs, T(-1), blk(Loff, nb - 1, i - 1), blk(Uoff, nb - 1, i - 1), D);
+        lu.prod_UL_acc(kc, T(-1), blk(Loff, nb - 1, i - 1).at(0, bs - kc), blk(Uoff, nb - 1, i - 1).at(bs - kc, 0), D);
       }
       {
         SAPB_PROF("wb_rec", st);
@@ -657,11 +665,13 @@ class WideBand {
         // (upper times upper); D is free again as the second lane's scratch
         SAPB_PROF("wb_offdiag", st);
         lu.fork();
-        lu.prod_LL(bs, T(1), Li, blk(Uoff, nb - 1, i), Wm);
-        lu.copy(Wm, blk(Uoff, nb - 1, i), bs, bs);
+        const int c0 = bs - kc;
+        const Mat<T> E = blk(Uoff, nb - 1, i).at(c0, 0), F = blk(Loff, nb - 1, i).at(0, c0);
+        lu.prod_LL(kc, T(1), Li.at(c0, c0), E, Wm);
+        lu.copy(Wm, E, kc, kc);
         lu.lane2([&] {
-          lu.prod_UU(bs, T(1), blk(Loff, nb - 1, i), Ui, D);
-          lu.copy(D, blk(Loff, nb - 1, i), bs, bs);
+          lu.prod_UU(kc, T(1), F, Ui.at(c0, c0), D);
+          lu.copy(D, F, kc, kc);
         });
         lu.join();
       }
@@ -817,6 +827,47 @@ class WideBand {
     SAPB_CUDA(cudaStreamSynchronize(st));
     throw Error(SAP_ERR_DEVICE_TIMEOUT, "a block-sweep barrier wait ran out of its iteration limit");
   }
+  // Sweeps of small blocks (k_sweep_cluster): clusters of 8 CTAs while they
+  // all fit the chip at once, else of 4; the blocks a thread's registers hold.
+  static constexpr int kClusterMaxBs = sizeof(T) == 8 ? 320 : 448;
+  template <int V, typename MT, int C>
+  void sweep_cluster_launch(T* x, const MT* Li, const MT* Ui, const MT* Lo, const MT* Uo, const T* cL, const T* cU,
+                            const T* cLo, const T* cUo) {
+    constexpr int W = kGemvWarps * C, JM = (kClusterMaxBs + W - 1) / W, NT = (kClusterMaxBs + 32 * V - 1) / (32 * V);
+    auto kern = k_sweep_cluster<T, V, MT, C, JM, NT>;
+    const size_t smem = (size_t)(kGemvWarps + 2 * C + 1) * 32 * V * NT * sizeof(T);
+    SAPB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(P * C);
+    cfg.blockDim = dim3(kGemvWarps * 32);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = C;
+    attr[0].val.clusterDim.y = 1;
+    attr[0].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    SAPB_CUDA(cudaLaunchKernelEx(&cfg, kern, Li, Ui, Lo, Uo, cL, cU, cLo, cUo, x, yv.get(), nb, bs, kc, BB, plen));
+    SAPB_LAUNCHED();
+  }
+  void sweep_cluster(T* x) {
+    auto go = [&](auto V, auto* Li, auto* Ui, auto* Lo, auto* Uo, const T* cL, const T* cU, const T* cLo,
+                  const T* cUo) {
+      using MT = std::remove_const_t<std::remove_pointer_t<decltype(Li)>>;
+      if (P * 8 <= 148) sweep_cluster_launch<V(), MT, 8>(x, Li, Ui, Lo, Uo, cL, cU, cLo, cUo);
+      else sweep_cluster_launch<V(), MT, 4>(x, Li, Ui, Lo, Uo, cL, cU, cLo, cUo);
+    };
+    const T* no = nullptr;
+    if constexpr (sizeof(T) == 4) {
+      if (h16)
+        return go(std::integral_constant<int, 8>{}, Lh.get(), Uh.get(), Loh.get(), Uoh.get(), csL.get(), csU.get(),
+                  csLo.get(), csUo.get());
+    }
+    go(std::integral_constant<int, 16 / (int)sizeof(T)>{}, Linv.get(), Uinv.get(), Loff.get(), Uoff.get(), no, no, no,
+       no);
+  }
   // One block sweep in schedule `mode`: 0 persistent (k_sweep), 1 / 2 / 4
   // lanes of per-step launches (fewer when a lane would get fewer than two
   // partitions).  False when the persistent launch is not possible.
@@ -850,7 +901,7 @@ class WideBand {
     return true;
   }
 
-  // Sweep schedule autotuner, keyed on the layout (P, block size, blocks per
+  // Sweep schedule autotuner of larger blocks, keyed on the layout (P, block size, blocks per
   // partition, bytes per factor value): the first sweep of an unseen key
   // times the candidate schedules (persistent, 2 lanes, 4 lanes; best of
   // two runs each, CUDA events) on a copy of its right-hand side and keeps
@@ -907,6 +958,7 @@ class WideBand {
   }
   void solve_blocks(T* x) {
     int mode = fixed_mode();
+    if (mode < 0 && bs <= kClusterMaxBs) return sweep_cluster(x);
     if (mode < 0) {
       const auto key = std::make_tuple(P, bs, nb, h16 ? 2 : (int)sizeof(T));
       auto it = tuned().find(key);
@@ -1067,12 +1119,14 @@ class WideBand {
         // forward with L_{i,i-1} (upper) and L_ii^-1 (lower), backward with
         // U_{i,i+1} (lower) and U_ii^-1 (upper)
         for (int i = ib0; i < nb; i++) {
-          if (i > ib0) ops.prod_UF(bs, w, T(-1), Fk(Loff, nb - 1, i - 1), Xb(i - 1), T(1), Xb(i));
+          if (i > ib0)
+            ops.prod_UF(kc, w, T(-1), Fk(Loff, nb - 1, i - 1).at(0, bs - kc), Xb(i - 1).at(bs - kc, 0), T(1), Xb(i));
           ops.prod_LF(bs, w, T(1), Fk(Linv, nb, i), Xb(i), T(0), Wm);
           ops.copy(Wm, Xb(i), bs, w);
         }
         for (int i = nb - 1; i >= ib0; i--) {
-          if (i < nb - 1) ops.prod_LF(bs, w, T(-1), Fk(Uoff, nb - 1, i), Xb(i + 1), T(1), Xb(i));
+          if (i < nb - 1)
+            ops.prod_LF(kc, w, T(-1), Fk(Uoff, nb - 1, i).at(bs - kc, 0), Xb(i + 1), T(1), Xb(i).at(bs - kc, 0));
           ops.prod_UF(bs, w, T(1), Fk(Uinv, nb, i), Xb(i), T(0), Wm);
           ops.copy(Wm, Xb(i), bs, w);
         }
