@@ -99,7 +99,20 @@ struct Spmv {
   void apply(const double* x, double* y, cudaStream_t s) const {
     if (kind == 0) {
       SAPB_PROF("spmv_banded", s);
-      k_spmv_banded<<<grid_for((long long)band->n * 32, 256, 148 * 32), 256, 0, s>>>(band->A.get(), x, y, band->n, band->K);
+      const int SW = 2 * band->K + 1, L = band_lanes(SW), TR = 256 / L;
+      if (SW <= kBandTile / 16) {
+        const size_t smem = ((size_t)TR * SW + TR + 2 * band->K) * sizeof(double);
+        const int grid = (band->n + TR - 1) / TR;
+        auto go = [&](auto kern) { kern<<<grid, 256, smem, s>>>(band->A.get(), x, y, band->n, band->K); };
+        if (L == 1) go(k_spmv_band_tile<1>);
+        else if (L == 2) go(k_spmv_band_tile<2>);
+        else if (L == 4) go(k_spmv_band_tile<4>);
+        else if (L == 8) go(k_spmv_band_tile<8>);
+        else go(k_spmv_band_tile<16>);
+      } else {
+        k_spmv_banded<<<grid_for((long long)band->n * 32, 256, 148 * 32), 256, 0, s>>>(band->A.get(), x, y, band->n,
+                                                                                       band->K);
+      }
       SAPB_LAUNCHED();
     } else if (kind == 1) {
       SAPB_PROF("spmv_csr", s);
@@ -1411,10 +1424,9 @@ class Solver {
     for (int q = 0; q < nq; q++) { a.x[q] = xs[q]; a.y[q] = ys[q]; }
     {
       SAPB_PROF("dots", st);
-      k_dots<<<kDotBlocks, kDotThreads, 0, st>>>(n, a, dots_part.get(), dots_ctr.get(), dots_out.get());
+      k_dots<<<dot_blocks(n), kDotThreads, 0, st>>>(n, a, dots_part.get(), dots_ctr.get(), pinned);
       SAPB_LAUNCHED();
     }
-    SAPB_CUDA(cudaMemcpyAsync(pinned, dots_out.get(), nq * sizeof(double), cudaMemcpyDeviceToHost, st));
     SAPB_CUDA(cudaStreamSynchronize(st));
     for (int q = 0; q < nq; q++) out[q] = pinned[q];
   }
@@ -1430,7 +1442,7 @@ class Solver {
     a.x[0] = w;
     a.y[0] = w;
     SAPB_PROF("dots", st);
-    k_dots<<<kDotBlocks, kDotThreads, 0, st>>>(n, a, dots_part.get(), dots_ctr.get(), dots_out.get());
+    k_dots<<<dot_blocks(n), kDotThreads, 0, st>>>(n, a, dots_part.get(), dots_ctr.get(), dots_out.get());
     SAPB_LAUNCHED();
   }
   // one classical Gram-Schmidt pass against basis vectors 0..m-1 (device
@@ -1438,7 +1450,7 @@ class Solver {
   void cgs_pass(int m, const double* const* vs, double* w, double* h) {
     {
       SAPB_PROF("dots", st);
-      k_mdot<<<dim3(kMdotBlocks, m), kMdotThreads, 0, st>>>(n, vs, w, gs_part.get(), gs_ctr.get(), h);
+      k_mdot<<<dim3(mdot_blocks(n), m), kMdotThreads, 0, st>>>(n, vs, w, gs_part.get(), gs_ctr.get(), h);
       SAPB_LAUNCHED();
     }
     k_maxpy<<<grid_for(n, 256), 256, 0, st>>>(n, m, vs, h, w);
@@ -1449,10 +1461,9 @@ class Solver {
   double axpy_nrm2(const double* x, double* y, double a) {
     {
       SAPB_PROF("dots", st);
-      k_axpy_sqnorm<<<kDotBlocks, kDotThreads, 0, st>>>(n, a, x, y, dots_part.get(), dots_ctr.get(), dots_out.get());
+      k_axpy_sqnorm<<<dot_blocks(n), kDotThreads, 0, st>>>(n, a, x, y, dots_part.get(), dots_ctr.get(), pinned);
       SAPB_LAUNCHED();
     }
-    SAPB_CUDA(cudaMemcpyAsync(pinned, dots_out.get(), sizeof(double), cudaMemcpyDeviceToHost, st));
     SAPB_CUDA(cudaStreamSynchronize(st));
     return std::sqrt(pinned[0]);
   }
@@ -1513,12 +1524,8 @@ class Solver {
         cgs_pass(j + 1, gs_v.get(), Vb[j + 1], h1);
         cgs_pass(j + 1, gs_v.get(), Vb[j + 1], h2);
         sqnorm_dev(Vb[j + 1]);
-        k_scale_inv_norm<<<grid_for(n, 256), 256, 0, st>>>(n, Vb[j + 1], dots_out.get());
+        k_scale_inv_norm<<<grid_for(n, 256), 256, 0, st>>>(n, Vb[j + 1], dots_out.get(), j + 1, gs_h.get(), h2, pinned);
         SAPB_LAUNCHED();
-        SAPB_CUDA(cudaMemcpyAsync(pinned, gs_h.get(), (size_t)(j + 1) * sizeof(double), cudaMemcpyDeviceToHost, st));
-        SAPB_CUDA(cudaMemcpyAsync(pinned + kMaxBasis, h2, (size_t)(j + 1) * sizeof(double), cudaMemcpyDeviceToHost,
-                                  st));
-        SAPB_CUDA(cudaMemcpyAsync(pinned + 2 * kMaxBasis, dots_out.get(), sizeof(double), cudaMemcpyDeviceToHost, st));
         SAPB_CUDA(cudaStreamSynchronize(st));
         for (int i = 0; i <= j; i++) h(i, j) = pinned[i] + pinned[kMaxBasis + i];
         const double hn = std::sqrt(pinned[2 * kMaxBasis]);
