@@ -384,15 +384,19 @@ __device__ __forceinline__ void cp_async_wait() {
 // is the quotient.  `ok` is false outside exponent ranges that guarantee
 // this (non-finite, subnormal, very large or very small operands), where the
 // caller must use the division; with ok true the result equals a / b.
+// The ranges are tested on the magnitudes' leading bits (integers, beside the
+// chain of multiply-adds).
 template <typename T>
 struct DivRange;
 template <>
-struct DivRange<double> {
-  static constexpr double lo_a = 0x1p-960, lo = 0x1p-1000, hi = 0x1p1000;
+struct DivRange<double> {  // 2^-960, 2^-1000, 2^1000
+  static constexpr unsigned lo_a = 63u << 20, lo = 23u << 20, hi = 2023u << 20;
+  static __device__ __forceinline__ unsigned mag(double v) { return (unsigned)__double2hiint(v) & 0x7fffffffu; }
 };
 template <>
-struct DivRange<float> {
-  static constexpr float lo_a = 0x1p-96f, lo = 0x1p-120f, hi = 0x1p120f;
+struct DivRange<float> {  // 2^-96, 2^-120, 2^120
+  static constexpr unsigned lo_a = 31u << 23, lo = 7u << 23, hi = 247u << 23;
+  static __device__ __forceinline__ unsigned mag(float v) { return (unsigned)__float_as_int(v) & 0x7fffffffu; }
 };
 template <typename T>
 __device__ __forceinline__ T div_rcp_fast(T a, T b, T y, bool& ok) {
@@ -400,8 +404,8 @@ __device__ __forceinline__ T div_rcp_fast(T a, T b, T y, bool& ok) {
   const T q0 = a * y;
   const T r = fma(-q0, b, a);
   const T q = fma(r, y, q0);
-  const T aa = fabs(a), aq = fabs(q0), ay = fabs(y);
-  ok = ay >= L::lo && ay <= L::hi && (a == T(0) || (aa >= L::lo_a && aq >= L::lo && aq <= L::hi));
+  constexpr unsigned span = L::hi - L::lo;
+  ok = L::mag(y) - L::lo < span && (a == T(0) || (L::mag(a) >= L::lo_a && L::mag(q0) - L::lo < span));
   return a == T(0) ? q0 : q;
 }
 

@@ -258,34 +258,42 @@ k_factor_smem(const FactorJob* __restrict__ jobs, T* __restrict__ B, T* __restri
 // of two per pivot.
 //
 // What bounds it is the chain of pivots, so the chain has a warp of its own
-// (look-ahead): while the other warps apply panel p (columns j0 .. j0+NB-1) to
-// the columns from j0 + 2 NB on, warp 0 applies it to the NB columns of panel
-// p+1 and factors that panel.  Warp 0 holds a panel in registers: lane l rows
-// j0 + l + 32 t (t < R) of its NB columns; each pivot is broadcast by a
-// shuffle, its column is divided by it and the rest of the panel receives the
-// rank-1 update.  The panel's L columns also go, with zeros outside the band,
-// to Lp in the row alignment the updates use, so that these need no tests:
-// a warp takes CPW columns (their rows in registers, the U element of each
+// (look-ahead): the first HW warps apply panel p (columns j0 .. j0+NB-1) to the
+// NB columns of panel p+1, warp 0 then factors that panel while the other
+// warps apply panel p to the columns from j0 + 2 NB on.  Warp 0 holds a panel
+// in registers: lane l rows j0 + l + 32 t (t < R) of its NB columns; each pivot
+// is broadcast by a shuffle, its column is divided by it and the rest of the
+// panel receives the rank-1 update.  The panel's L columns also go, with zeros
+// outside the band, to Lp in the row alignment the updates use.  An updating
+// warp takes a few columns (their rows in registers, the U element of each
 // pivot broadcast from the lane holding that row), pivots in order.  Beside
-// their updates the other warps write back panel p-1 and fetch, with cp.async
-// into the freed slots, the NB columns that panel p + DPF will first touch.
-// The ring holds W = K + NB (1 + DPF) column slots; slots advance by
-// additions, with no modulo.
+// their updates the warps other than 0 write back panel p-1 and fetch, with
+// cp.async into the freed slots, the NB columns that panel p + DPF will first
+// touch.
+//
+// The instructions of warp 0 are what the chain costs (4 to 5 cycles each), so
+// the ring's W = K + NB (1 + DPF) slots are padded by NB - 1 zeros: the rows
+// j0 .. j0+NB+K-1 of every column near the panel are at constant offsets with
+// no test, those outside its band being zeros of the padding (or, past the
+// partition's end, elements that meet zeros of Lp and stay as they are).
+// 200,000 rows, K = 50, P = 10, FP64: 15.1 ms with one phase after the other,
+// 10.4 ms with look-ahead and a test per element.
 template <typename T, int NB>
 inline size_t factor_panel_smem(int R, int K, int dpf) {
-  return ((size_t)(K + NB * (1 + dpf)) * (2 * K + 1) + 2 * NB * 32 * R) * sizeof(T);
+  return (NB + (size_t)(K + NB * (1 + dpf)) * (2 * K + NB) + 2 * NB * 32 * R) * sizeof(T);
 }
 template <typename T, int NB, int R>
 __global__ void __launch_bounds__(512)
 k_factor_panel(const FactorJob* __restrict__ jobs, T* __restrict__ B, T* __restrict__ B2,
                int do_boost, int* __restrict__ zero_flag, int DPF) {
   constexpr int CPW = 4;   // columns a trailing warp applies a panel to at once
+  constexpr int HW = 4;    // warps that update the next panel
   constexpr int LR = 32 * R;
   const FactorJob jb = jobs[blockIdx.x];
-  const int K = jb.K, SW = 2 * K + 1, np = jb.e - jb.s, W = K + NB * (1 + DPF);
+  const int K = jb.K, SW = 2 * K + 1, SP = 2 * K + NB, np = jb.e - jb.s, W = K + NB * (1 + DPF);
   extern __shared__ __align__(16) unsigned char sm_raw[];
-  T* win = reinterpret_cast<T*>(sm_raw);
-  T* Lp = win + W * SW;  // two panels of NB columns of LR rows
+  T* win = reinterpret_cast<T*>(sm_raw) + NB;
+  T* Lp = win + W * SP;  // two panels of NB columns of LR rows
   T* band = (jb.target ? B2 : B) + jb.boff;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nw = blockDim.x >> 5;
   const bool mir = jb.mirror != 0;
@@ -295,30 +303,31 @@ k_factor_panel(const FactorJob* __restrict__ jobs, T* __restrict__ B, T* __restr
     return (long long)col * SW + pos;
   };
   auto wrap = [&](int s) { return s >= W ? s - W : s; };  // for 0 <= s < 2 W
+  const bool tail = lane + 32 * (R - 1) < K + NB;  // the last row slot of this lane is in use
+  for (int e = tid; e < NB; e += blockDim.x) win[e - NB] = T(0);
+  for (int e = tid; e < W * (NB - 1); e += blockDim.x) win[(e / (NB - 1)) * SP + SW + e % (NB - 1)] = T(0);
   if (warp != 0) {  // columns [0, K + NB), then one panel's new columns per group; all in slots == column
     for (int g = 0; g < DPF; g++) {
       const int c0 = g == 0 ? 0 : K + g * NB, c1 = min(np, K + (g + 1) * NB);
       for (int c = c0 + warp - 1; c < c1; c += nw - 1)
-        for (int p = lane; p < SW; p += 32) cp_async_val<T>(&win[c * SW + p], band + gidx(c, p));
+        for (int p = lane; p < SW; p += 32) cp_async_val<T>(&win[c * SP + p], band + gidx(c, p));
       cp_async_commit();
     }
   }
   bool zero_seen = false;
-  // warp 0: panel q (columns j .. j+nb-1, first slot s) factored in registers
+  // warp 0: the panel of columns j .. j+nb-1 (first slot s) factored in registers
   auto factor = [&](int j, int s, int nb, T* lp) {
     T a[R][NB];
     auto load_panel = [&]() {
 #pragma unroll
       for (int c = 0; c < NB; c++) {
-        const T* colp = win + wrap(s + c) * SW;
+        const T* colp = win + wrap(s + c) * SP + K - c + lane;  // row j + lane + 32 t
 #pragma unroll
-        for (int t = 0; t < R; t++) {
-          const int pos = K + lane + 32 * t - c;  // row j + lane + 32 t
-          a[t][c] = (c < nb && j + lane + 32 * t < np && pos >= 0 && pos <= 2 * K) ? colp[pos] : T(0);
-        }
+        for (int t = 0; t < R; t++) a[t][c] = (c < nb && (t + 1 < R || tail)) ? colp[32 * t] : T(0);
       }
     };
     load_panel();
+    const int last = np - 1 - j;  // the panel's rows are 0 .. last
     // fast path: each quotient from the pivot's reciprocal with Markstein's
     // correction (div_rcp_fast, equal to the division inside its range),
     // without branches; `bad` records a lane whose operands left the range
@@ -326,7 +335,7 @@ k_factor_panel(const FactorJob* __restrict__ jobs, T* __restrict__ B, T* __restr
 #pragma unroll
     for (int k = 0; k < NB; k++) {
       if (k < nb) {
-        const int w = min(K, np - 1 - (j + k));
+        const int end = min(K + k, last);  // last row of the pivot's column
         T p = __shfl_sync(0xffffffffu, a[0][k], k);
         if (do_boost) p = boost_pivot(p);
         else zero_seen |= fabs((double)p) < 1e-7;
@@ -336,76 +345,68 @@ k_factor_panel(const FactorJob* __restrict__ jobs, T* __restrict__ B, T* __restr
         for (int c = k + 1; c < NB; c++) u[c] = __shfl_sync(0xffffffffu, a[0][c], k);
 #pragma unroll
         for (int t = 0; t < R; t++) {
-          const int rr = lane + 32 * t - k;  // row - pivot row
-          const bool in = rr >= 1 && rr <= w;
+          const bool in = (t > 0 || lane > k) && lane + 32 * t <= end;
           bool ok;
-          const T l = div_rcp_fast(a[t][k], p, y, ok);
+          const T l = div_rcp_fast(a[t][k], p, y, ok), lm = in ? l : T(0);
           bad |= in && !ok;
-          a[t][k] = rr == 0 ? p : (in ? l : a[t][k]);
+          a[t][k] = in ? l : a[t][k];
+          if (t == 0) a[t][k] = lane == k ? p : a[t][k];
 #pragma unroll
-          for (int c = k + 1; c < NB; c++) {
-            if (c - k <= w) {
-              const T nv = a[t][c] - l * u[c];
-              a[t][c] = in ? nv : a[t][c];
-            }
-          }
+          for (int c = k + 1; c < NB; c++) a[t][c] -= lm * u[c];
+          lp[k * LR + lane + 32 * t] = lm;
         }
       }
     }
     if (__any_sync(0xffffffffu, bad)) {
       // some quotient left the range: the panel again with the division
       load_panel();
+#pragma unroll 1
+      for (int k = 0; k < nb; k++) {
+        const int end = min(K + k, last);
+        T p = T(0);
 #pragma unroll
-      for (int k = 0; k < NB; k++) {
-        if (k < nb) {
-          const int w = min(K, np - 1 - (j + k));
-          T p = __shfl_sync(0xffffffffu, a[0][k], k);
-          if (do_boost) p = boost_pivot(p);
-          T u[NB];
+        for (int c = 0; c < NB; c++)
+          if (c == k) p = __shfl_sync(0xffffffffu, a[0][c], k);
+        if (do_boost) p = boost_pivot(p);
+        T u[NB];
 #pragma unroll
-          for (int c = k + 1; c < NB; c++) u[c] = __shfl_sync(0xffffffffu, a[0][c], k);
+        for (int c = 0; c < NB; c++) u[c] = __shfl_sync(0xffffffffu, a[0][c], k);
 #pragma unroll
-          for (int t = 0; t < R; t++) {
-            const int rr = lane + 32 * t - k;
-            if (rr == 0) {
-              a[t][k] = p;
-            } else if (rr >= 1 && rr <= w) {
-              const T l = a[t][k] / p;
-              a[t][k] = l;
+        for (int t = 0; t < R; t++) {
+          const bool in = (t > 0 || lane > k) && lane + 32 * t <= end;
+          T l = T(0);
 #pragma unroll
-              for (int c = k + 1; c < NB; c++)
-                if (c - k <= w) a[t][c] -= l * u[c];
-            }
+          for (int c = 0; c < NB; c++)
+            if (c == k) l = a[t][c] / p;
+          l = in ? l : T(0);
+          lp[k * LR + lane + 32 * t] = l;
+#pragma unroll
+          for (int c = 0; c < NB; c++) {
+            if (c > k) a[t][c] -= l * u[c];
+            else if (c == k) a[t][c] = t == 0 && lane == k ? p : (in ? l : a[t][c]);
           }
         }
       }
     }
 #pragma unroll
     for (int c = 0; c < NB; c++) {
-      T* colp = win + wrap(s + c) * SW;
-      const int w = c < nb ? min(K, np - 1 - (j + c)) : 0;
+      T* colp = win + wrap(s + c) * SP + K - c + lane;
 #pragma unroll
-      for (int t = 0; t < R; t++) {
-        const int rr = lane + 32 * t - c, pos = K + rr;
-        if (c < nb && j + lane + 32 * t < np && pos >= 0 && pos <= 2 * K) colp[pos] = a[t][c];
-        lp[c * LR + lane + 32 * t] = rr >= 1 && rr <= w ? a[t][c] : T(0);
-      }
+      for (int t = 0; t < R; t++)
+        if (c < nb && (t + 1 < R || tail)) colp[32 * t] = a[t][c];
     }
   };
   // the panel at j0 (L columns in lp) applied to the NC columns from q0 past
   // its end on (column j0 + NB + q), the first nt of which exist
-  auto update = [&](auto ncol, int j0, int s0, const T* lp, int q0, int nt) {
+  auto update = [&](auto ncol, int s0, const T* lp, int q0, int nt) {
     constexpr int NC = decltype(ncol)::value;
     T x[NC][R];
+    T* colp[NC];
 #pragma unroll
     for (int i = 0; i < NC; i++) {
-      const int q = q0 + i;
-      const T* colp = win + wrap(s0 + NB + q) * SW;
+      colp[i] = win + wrap(s0 + NB + q0 + i) * SP + K - NB - q0 - i + lane;
 #pragma unroll
-      for (int t = 0; t < R; t++) {
-        const int pos = K + lane + 32 * t - NB - q;
-        x[i][t] = (q < nt && j0 + lane + 32 * t < np && pos >= 0 && pos <= 2 * K) ? colp[pos] : T(0);
-      }
+      for (int t = 0; t < R; t++) x[i][t] = (q0 + i < nt && (t + 1 < R || tail)) ? colp[i][32 * t] : T(0);
     }
 #pragma unroll
     for (int k = 0; k < NB; k++) {
@@ -420,15 +421,10 @@ k_factor_panel(const FactorJob* __restrict__ jobs, T* __restrict__ B, T* __restr
       }
     }
 #pragma unroll
-    for (int i = 0; i < NC; i++) {
-      const int q = q0 + i;
-      T* colp = win + wrap(s0 + NB + q) * SW;
+    for (int i = 0; i < NC; i++)
 #pragma unroll
-      for (int t = 0; t < R; t++) {
-        const int pos = K + lane + 32 * t - NB - q;
-        if (q < nt && j0 + lane + 32 * t < np && pos >= 0 && pos <= 2 * K) colp[pos] = x[i][t];
-      }
-    }
+      for (int t = 0; t < R; t++)
+        if (q0 + i < nt && (t + 1 < R || tail)) colp[i][32 * t] = x[i][t];
   };
   // (K < NB: the next panel reaches past the columns the current one touches,
   // into those of the newest group)
@@ -444,12 +440,14 @@ k_factor_panel(const FactorJob* __restrict__ jobs, T* __restrict__ B, T* __restr
     const T* lp = Lp + buf * NB * LR;
     const int nt = min(K, np - j0 - NB);
     wait();
+    if (warp < HW) {
+      if (warp * (NB / HW) < nt)
+        update(std::integral_constant<int, NB / HW>{}, s0, lp, warp * (NB / HW), min(nt, NB));
+      if (warp == 0) asm volatile("bar.sync 1, %0;" ::"n"(32 * HW) : "memory");
+      else asm volatile("bar.arrive 1, %0;" ::"n"(32 * HW) : "memory");
+    }
     if (warp == 0) {
-      if (j0 + NB < np) {
-        update(std::integral_constant<int, NB>{}, j0, s0, lp, 0, min(nt, NB));
-        __syncwarp();
-        factor(j0 + NB, wrap(s0 + NB), min(NB, np - j0 - NB), Lp + (buf ^ 1) * NB * LR);
-      }
+      if (j0 + NB < np) factor(j0 + NB, wrap(s0 + NB), min(NB, np - j0 - NB), Lp + (buf ^ 1) * NB * LR);
     } else {
       // write back panel p-1 and fetch the columns of panel p+DPF into its slots
       // (the thread that reads a slot element issues the copy into it; the U
@@ -457,7 +455,7 @@ k_factor_panel(const FactorJob* __restrict__ jobs, T* __restrict__ B, T* __restr
       const int nf0 = j0 + DPF * NB + K;
       const int sp = s0 - NB < 0 ? s0 - NB + W : s0 - NB;
       for (int c = warp - 1; c < NB; c += nw - 1) {
-        T* slot = win + wrap(sp + c) * SW;
+        T* slot = win + wrap(sp + c) * SP;
         for (int p = lane; p < SW; p += 32) {
           if (j0 > 0) band[gidx(j0 - NB + c, p)] = slot[p];
           if (nf0 + c < np) cp_async_val<T>(slot + p, band + gidx(nf0 + c, p));
@@ -465,7 +463,7 @@ k_factor_panel(const FactorJob* __restrict__ jobs, T* __restrict__ B, T* __restr
       }
       cp_async_commit();
       for (int q0 = NB + (warp - 1) * CPW; q0 < nt; q0 += (nw - 1) * CPW)
-        update(std::integral_constant<int, CPW>{}, j0, s0, lp, q0, nt);
+        update(std::integral_constant<int, CPW>{}, s0, lp, q0, nt);
     }
   }
   if (zero_seen && tid == 0) atomicOr(zero_flag, 1);
@@ -474,7 +472,7 @@ k_factor_panel(const FactorJob* __restrict__ jobs, T* __restrict__ B, T* __restr
   // the last panel: columns [j0 - NB, np) in slots from s0 - NB on
   const int jl = j0 - NB, sl0 = s0 - NB < 0 ? s0 - NB + W : s0 - NB;
   for (int c = warp; c < np - jl; c += nw)
-    for (int p = lane; p < SW; p += 32) band[gidx(jl + c, p)] = win[wrap(sl0 + c) * SW + p];
+    for (int p = lane; p < SW; p += 32) band[gidx(jl + c, p)] = win[wrap(sl0 + c) * SP + p];
 }
 
 // Post-divide of the panel kernel's factors (bandLUUL_post_divide,

@@ -976,10 +976,8 @@ class PrecondT : public PrecBase {
     NT = std::max(NT, 64);
     constexpr int D = 8;
     size_t smem = ((size_t)(Kmax + 1 + D) * (2 * Kmax + 1) + (Kmax + 1 + D)) * sizeof(T);
-    constexpr int NB = 8;
     const char* fk = std::getenv("SAPB_FACTOR_KERNEL");
     const bool ring_only = fk && std::string(fk) == "ring";
-    const int R = (Kmax + NB + 31) / 32;
     int maxrows = 0;
     for (const auto& jb : jobs) maxrows = std::max(maxrows, jb.e - jb.s);
     auto postdiv = [&]() {
@@ -987,28 +985,45 @@ class PrecondT : public PrecBase {
       k_factor_postdiv<T><<<dim3(grid_for((long long)maxrows * Kmax, 256, 1024), (int)jobs.size()), 256, 0, st>>>(
           jobs_d.get(), B.get(), B2.get());
     };
-    auto panel_smem = [&](int dpf) { return factor_panel_smem<T, NB>(R, Kmax, dpf); };
-    // (a panel's rows in registers: K <= 32 R - NB with R <= 4, or 5 in FP32)
-    if (!ring_only && R <= (sizeof(T) == 4 ? 5 : 4) && panel_smem(1) <= 227 * 1024) {
-      const int dpf = panel_smem(2) <= 227 * 1024 ? 2 : 1;
-      const size_t psm = panel_smem(dpf);
-      // the chain's warp, and four trailing columns per other warp
-      const int nt = 32 * std::min(16, std::max(3, 1 + (Kmax - NB + 3) / 4));
+    // (a panel's rows in registers: K <= 32 R - NB with R <= 4, or 5 in FP32;
+    // FP64 bands whose ring does not fit with panels of 8 take panels of 4)
+    auto run_panel = [&](auto nbc) {
+      constexpr int NBP = decltype(nbc)::value;
+      const int R = (Kmax + NBP + 31) / 32;
+      auto need = [&](int dpf) { return factor_panel_smem<T, NBP>(R, Kmax, dpf); };
+      if (R > (sizeof(T) == 4 ? 5 : 4) || need(1) > 227 * 1024) return false;
+      const int dpf = need(2) <= 227 * 1024 ? 2 : 1;
+      // the chain's warp and three more for the next panel, four trailing columns per other warp
+      const int nt = 32 * std::min(16, std::max(5, 1 + (Kmax - NBP + 3) / 4));
       auto launch = [&](auto kern) {
-        SAPB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)psm));
-        kern<<<(int)jobs.size(), nt, psm, st>>>(jobs_d.get(), B.get(), B2.get(), boost ? 1 : 0, flag.get(), dpf);
+        SAPB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)need(dpf)));
+        kern<<<(int)jobs.size(), nt, need(dpf), st>>>(jobs_d.get(), B.get(), B2.get(), boost ? 1 : 0, flag.get(), dpf);
       };
-      SAPB_PROF("factor", st);  // the factor kernel and its post-divide pass
-      switch (R) {
-        case 1: launch(k_factor_panel<T, NB, 1>); break;
-        case 2: launch(k_factor_panel<T, NB, 2>); break;
-        case 3: launch(k_factor_panel<T, NB, 3>); break;
-        case 4: launch(k_factor_panel<T, NB, 4>); break;
-        default:
-          if constexpr (sizeof(T) == 4) launch(k_factor_panel<T, NB, 5>);
-          break;
+      if constexpr (NBP == 8) {
+        switch (R) {
+          case 1: launch(k_factor_panel<T, NBP, 1>); break;
+          case 2: launch(k_factor_panel<T, NBP, 2>); break;
+          case 3: launch(k_factor_panel<T, NBP, 3>); break;
+          case 4: launch(k_factor_panel<T, NBP, 4>); break;
+          default:
+            if constexpr (sizeof(T) == 4) launch(k_factor_panel<T, NBP, 5>);
+            break;
+        }
+      } else {
+        if (R != 4) return false;
+        launch(k_factor_panel<T, NBP, 4>);
       }
-      postdiv();
+      return true;
+    };
+    bool panel = false;
+    if (!ring_only) {
+      SAPB_PROF("factor", st);  // the factor kernel and its post-divide pass
+      panel = run_panel(std::integral_constant<int, 8>{});
+      if constexpr (sizeof(T) == 8) panel = panel || run_panel(std::integral_constant<int, 4>{});
+      if (panel) postdiv();
+    }
+    if (panel) {
+      // launched above
     } else if (smem <= 200 * 1024) {
       SAPB_CUDA(cudaFuncSetAttribute(k_factor_smem<T, D>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
       SAPB_PROF("factor", st);
