@@ -409,6 +409,31 @@ __device__ __forceinline__ T div_rcp_fast(T a, T b, T y, bool& ok) {
   return a == T(0) ? q0 : q;
 }
 
+// 1 / b without a branch: Newton's iteration on the hardware's approximation,
+// y <- y + y (1 - b y) with fused multiply-adds.  Once y is within one unit in
+// the last place, one more step gives the correctly rounded reciprocal unless
+// b's significand is all ones (Markstein, IBM J. Res. Dev. 34(1), 1990).  `ok`
+// is false for that significand and outside DivRange, where the caller must
+// use the division; with ok true the result equals T(1) / b.
+__device__ __forceinline__ float rcp_fast(float b, bool& ok) {
+  float y;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(b));
+#pragma unroll
+  for (int i = 0; i < 2; i++) y = fmaf(y, fmaf(-b, y, 1.f), y);
+  ok = DivRange<float>::mag(b) - DivRange<float>::lo < DivRange<float>::hi - DivRange<float>::lo &&
+       (__float_as_uint(b) & 0x7fffffu) != 0x7fffffu;
+  return y;
+}
+__device__ __forceinline__ double rcp_fast(double b, bool& ok) {
+  double y;
+  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(b));  // about 20 bits
+#pragma unroll
+  for (int i = 0; i < 3; i++) y = fma(y, fma(-b, y, 1.0), y);
+  ok = DivRange<double>::mag(b) - DivRange<double>::lo < DivRange<double>::hi - DivRange<double>::lo &&
+       (__double_as_longlong(b) & 0xfffffffffffffll) != 0xfffffffffffffll;
+  return y;
+}
+
 // boostValue (sap/device/factor_band_const.cuh:29-40): pivots with
 // |p| <= BURST_VALUE are replaced by +-BURST_NEW_VALUE.
 template <typename T>

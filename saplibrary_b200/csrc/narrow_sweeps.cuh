@@ -325,9 +325,13 @@ k_win_transfer(const PartDev* __restrict__ parts, const ChunkDev* __restrict__ c
 
 // Carry scan of one partition per CTA (see k_scan): the transfer matrices and
 // tails of NB chunks at a time come into shared memory by cp.async (they are
-// contiguous, and copied by all threads), one batch ahead of the chain, so that
-// a chain step is a K x K product out of shared memory: NC = 32-multiple >=
-// K G threads, G groups splitting its columns, synchronised among themselves.
+// contiguous, and copied by all threads), one batch ahead of the chain.  A
+// chain step is then a K x K product by the first K G threads: thread (g, u)
+// holds the KG values T(u, g KG ..) of the step in registers before the carry
+// they multiply is known, G partial sums per row meet in shared memory.  Up to
+// K = 32 one warp has whole rows (G = 1) and no barrier is left but its own.
+// What bounds it is the latency of a step: 0.41 us at K = 10 and 0.8 us at K =
+// 50 (FP64) with the matrix read after the carry.
 template <typename T>
 __host__ __device__ inline size_t scan_pad(size_t values) {  // to a multiple of 16 bytes
   constexpr size_t per = 16 / sizeof(T);
@@ -339,11 +343,14 @@ template <typename T>
 __host__ __device__ inline size_t scan_batch(int K, int NB) {
   return scan_pad<T>((size_t)K * K * NB + 4) + scan_pad<T>((size_t)K * NB + 4);
 }
-template <typename T>
-__global__ void __launch_bounds__(512)
+// values per thread and groups for half-bandwidth K
+constexpr int scan_kg(int K) { return K <= 16 ? 16 : K <= 32 ? 32 : K <= 64 ? 8 : K <= 128 ? 16 : 32; }
+constexpr int scan_groups(int K, int kg) { return (K + kg - 1) / kg; }
+template <typename T, int KG>
+__global__ void __launch_bounds__(sizeof(T) == 8 && KG == 32 ? 256 : 1024)
 k_win_scan(const PartDev* __restrict__ parts, const int* __restrict__ pchunk0, const int* __restrict__ pnchunk,
            const long long* __restrict__ koff, const long long* __restrict__ toff, const T* __restrict__ Tm,
-           const T* __restrict__ tails, T* __restrict__ carry, int which, int Gmax, int NC, int NB) {
+           const T* __restrict__ tails, T* __restrict__ carry, int which, int NB) {
   const PartDev p = parts[blockIdx.x];
   const int K = p.K, c0 = pchunk0[blockIdx.x], nc = pnchunk[blockIdx.x];
   if (nc <= 1) return;
@@ -351,16 +358,17 @@ k_win_scan(const PartDev* __restrict__ parts, const int* __restrict__ pchunk0, c
   extern __shared__ __align__(16) unsigned char win_raw[];
   T* st = reinterpret_cast<T*>(win_raw);
   const size_t SB = scan_batch<T>(K, NB), TO = scan_pad<T>((size_t)K * K * NB + 4);
-  T* sig = st + 2 * SB;  // K
-  T* red = sig + K;      // G * K
+  T* sig = st + 2 * SB;               // K, read up to a multiple of KG
+  const int G = scan_groups(K, KG), NC = (K * G + 31) / 32 * 32;
+  T* red = sig + G * KG;              // G * K
   const int tid = threadIdx.x, NT = blockDim.x, KK = K * K;
-  const int G = max(1, min(Gmax, NC / K));
   const int u = tid % K, g = tid / K;
   const bool act = g < G;
   const T* Tp = Tm + toff[c0];
   const T* tp = tails + koff[c0];
   T* cp = carry + koff[c0];
   constexpr int V = 16 / (int)sizeof(T);
+  for (int e = tid; e < G * KG; e += NT) sig[e] = T(0);
   // n contiguous values at src into dst + (src's offset within 16 bytes)
   auto fetch = [&](T* dst, const T* src, int n) {
     const int lead = (int)((reinterpret_cast<uintptr_t>(src) & 15) / sizeof(T));
@@ -385,6 +393,10 @@ k_win_scan(const PartDev* __restrict__ parts, const int* __restrict__ pchunk0, c
     }
     cp_async_commit();
   };
+  auto sync = [&] {
+    if (NC == 32) __syncwarp();
+    else asm volatile("bar.sync 1, %0;" ::"r"(NC) : "memory");
+  };
   issue(0);
   for (int b = 0; b * NB < nc - 1; b++) {
     cp_async_wait<0>();
@@ -395,26 +407,45 @@ k_win_scan(const PartDev* __restrict__ parts, const int* __restrict__ pchunk0, c
     batch(b, lo, cnt);
     const T* Tb = st + (b & 1) * SB + (reinterpret_cast<uintptr_t>(Tp + (long long)lo * KK) & 15) / sizeof(T);
     const T* tb = st + (b & 1) * SB + TO + (reinterpret_cast<uintptr_t>(tp + (long long)lo * K) & 15) / sizeof(T);
-    auto sync = [&] {
-      if (NC == 32) __syncwarp();
-      else asm volatile("bar.sync 1, %0;" ::"r"(NC) : "memory");
-    };
-    for (int q = 0; q < cnt; q++) {
+    T tv[KG], tl = T(0);
+    auto load = [&](int q) {
       const int j = dir > 0 ? q : cnt - 1 - q;  // chunk lo + j
-      T part = T(0);
-      if (act && b + q > 0) {
-        const T* tc = Tb + j * KK + g * K + u;
-#pragma unroll 4
-        for (int k = g; k < K; k += G, tc += G * K) part = fma(*tc, sig[k], part);
+      const T* tc = Tb + j * KK + g * KG * K + u;
+#pragma unroll
+      for (int k = 0; k < KG; k++) tv[k] = act && b + q > 0 && g * KG + k < K ? tc[k * K] : T(0);
+      tl = tid < K ? tb[j * K + tid] : T(0);
+    };
+    load(0);
+    for (int q = 0; q < cnt; q++) {
+      const int j = dir > 0 ? q : cnt - 1 - q;
+      const T* sg = sig + g * KG;
+      T acc[4] = {G == 1 ? tl : T(0), T(0), T(0), T(0)};
+      if (act) {
+#pragma unroll
+        for (int k = 0; k < KG; k++) acc[k & 3] = fma(tv[k], sg[k], acc[k & 3]);
       }
-      if (act) red[g * K + u] = part;
-      sync();
+      T v = (acc[0] + acc[1]) + (acc[2] + acc[3]);
+      const T tail = tl;
+      if (q + 1 < cnt) load(q + 1);
+      if (G > 1) {
+        if (act) red[g * K + u] = v;
+        sync();
+        if (tid < K) {
+          T s0 = tail, s1 = T(0);
+          int r = 0;
+          for (; r + 1 < G; r += 2) {
+            s0 += red[r * K + tid];
+            s1 += red[(r + 1) * K + tid];
+          }
+          if (r < G) s0 += red[r * K + tid];
+          v = s0 + s1;
+        }
+      } else {
+        sync();  // all lanes have read the carry
+      }
       if (tid < K) {
-        T acc = tb[j * K + tid];
-#pragma unroll 4
-        for (int r = 0; r < G; r++) acc += red[r * K + tid];
-        cp[(long long)(lo + j + dir) * K + tid] = acc;
-        sig[tid] = acc;
+        cp[(long long)(lo + j + dir) * K + tid] = v;
+        sig[tid] = v;
       }
       sync();
     }

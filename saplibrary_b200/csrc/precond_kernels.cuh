@@ -328,18 +328,21 @@ k_factor_panel(const FactorJob* __restrict__ jobs, T* __restrict__ B, T* __restr
     };
     load_panel();
     const int last = np - 1 - j;  // the panel's rows are 0 .. last
-    // fast path: each quotient from the pivot's reciprocal with Markstein's
-    // correction (div_rcp_fast, equal to the division inside its range),
-    // without branches; `bad` records a lane whose operands left the range
-    bool bad = false;
+    // fast path of a full panel: each quotient from the pivot's reciprocal with
+    // Markstein's correction (rcp_fast and div_rcp_fast, equal to the division
+    // inside their range), one block of code without branches, so that a
+    // pivot's shuffles and updates run beside the next reciprocal; `bad`
+    // records a lane whose operands left the range
+    bool bad = nb < NB;
+    if (nb == NB) {
 #pragma unroll
-    for (int k = 0; k < NB; k++) {
-      if (k < nb) {
+      for (int k = 0; k < NB; k++) {
         const int end = min(K + k, last);  // last row of the pivot's column
         T p = __shfl_sync(0xffffffffu, a[0][k], k);
-        if (do_boost) p = boost_pivot(p);
-        else zero_seen |= fabs((double)p) < 1e-7;
-        const T y = T(1) / p;
+        p = do_boost ? boost_pivot(p) : p;
+        bool pok;
+        const T y = rcp_fast(p, pok);
+        bad |= !pok;
         T u[NB];
 #pragma unroll
         for (int c = k + 1; c < NB; c++) u[c] = __shfl_sync(0xffffffffu, a[0][c], k);
@@ -358,7 +361,7 @@ k_factor_panel(const FactorJob* __restrict__ jobs, T* __restrict__ B, T* __restr
       }
     }
     if (__any_sync(0xffffffffu, bad)) {
-      // some quotient left the range: the panel again with the division
+      // a quotient left the range, or the last panel: with the division
       load_panel();
 #pragma unroll 1
       for (int k = 0; k < nb; k++) {
@@ -394,6 +397,10 @@ k_factor_panel(const FactorJob* __restrict__ jobs, T* __restrict__ B, T* __restr
 #pragma unroll
       for (int t = 0; t < R; t++)
         if (c < nb && (t + 1 < R || tail)) colp[32 * t] = a[t][c];
+    }
+    if (!do_boost) {  // the pivots as used
+      __syncwarp();
+      zero_seen |= lane < nb && fabs((double)win[wrap(s + min(lane, NB - 1)) * SP + K]) < 1e-7;
     }
   };
   // the panel at j0 (L columns in lp) applied to the NC columns from q0 past
@@ -466,7 +473,7 @@ k_factor_panel(const FactorJob* __restrict__ jobs, T* __restrict__ B, T* __restr
         update(std::integral_constant<int, CPW>{}, s0, lp, q0, nt);
     }
   }
-  if (zero_seen && tid == 0) atomicOr(zero_flag, 1);
+  if (zero_seen) atomicOr(zero_flag, 1);
   cp_async_wait<0>();
   __syncthreads();
   // the last panel: columns [j0 - NB, np) in slots from s0 - NB on

@@ -1054,6 +1054,12 @@ class PrecondT : public PrecBase {
       const auto& d = parts_h[p];
       int Kp = d.K;
       int m = std::min(4096, std::max(256, 8 * Kp));
+      // The window sweeps and their scan are chains of about 50 ns per row and
+      // 0.2 - 0.4 us per chunk, the rows passed four times and the chunks twice
+      // per sweep pair: shortest where m is about sqrt(rows per partition times
+      // their ratio).  At least 2 K rows, so that the transfer matrices stay
+      // below half of the factors' bytes.
+      if (window(maxK)) m = std::max({2 * Kp, 32, (int)std::sqrt(d.size * (3.0 + Kp / 24.0))});
       int nc = std::max(1, d.size / m);
       pc0.push_back((int)chunks_h.size());
       pnc.push_back(nc);
@@ -1151,9 +1157,8 @@ class PrecondT : public PrecBase {
   }
 
   // Transfer matrices of the register-window sweeps, and the carry scan's
-  // launch shape: about sqrt(K) column groups balance a group's share of the
-  // product against the sum over the groups; batches of as many chunks as fit
-  // twice in shared memory (one from K ~ 82 in FP64, ~ 116 in FP32 on).
+  // launch shape: batches of as many chunks as fit twice in shared memory
+  // (one from K ~ 82 in FP64, ~ 116 in FP32 on).
   int scanNT = 32, scanNB = 1;
   size_t scanSmem = 0;
   void build_window(int maxK, int nch) {
@@ -1172,9 +1177,9 @@ class PrecondT : public PrecBase {
           parts_d.get(), chunks_d.get(), toff_d.get(), pkd.get(), pku.get(), KP, T1.get(), T2.get(), first1_d.get(), first2_d.get());
     });
     SAPB_LAUNCHED();
-    scanG = std::max(1, std::min((int)std::lround(std::sqrt((double)maxK)), 512 / maxK));
-    scanNT = ((maxK * scanG + 31) / 32) * 32;
-    const size_t fixed = (size_t)(maxK + std::max(scanNT, maxK)) * sizeof(T);
+    const int kg = scan_kg(maxK), groups = scan_groups(maxK, kg);
+    scanNT = ((maxK * groups + 31) / 32) * 32;
+    const size_t fixed = (size_t)(groups * kg + scanNT) * sizeof(T);
     int longest = 1;
     for (size_t c = 0, run = 0; c < chunks_h.size(); c++) {
       run = c > 0 && chunks_h[c].part == chunks_h[c - 1].part ? run + 1 : 1;
@@ -1184,15 +1189,24 @@ class PrecondT : public PrecBase {
     scanNB = 1;
     while (scanNB < 64 && scanNB < longest && bytes(scanNB * 2) <= 200 * 1024) scanNB *= 2;
     scanSmem = bytes(scanNB);
-    allow_smem(k_win_scan<T>, scanSmem);
+    by_scan(maxK, [&](auto KG) { allow_smem(k_win_scan<T, KG()>, scanSmem); });
     SAPB_CUDA(cudaStreamSynchronize(st));
     t_assembly += ms_since(t0);
   }
+  template <class F>
+  static void by_scan(int k, F&& f) {
+    switch (scan_kg(k)) {
+      case 8: f(std::integral_constant<int, 8>{}); break;
+      case 16: f(std::integral_constant<int, 16>{}); break;
+      default: f(std::integral_constant<int, 32>{}); break;
+    }
+  }
   void window_scan(const T* Tm, const T* tails, T* carry, int which) {
     SAPB_PROF("scan", st);
-    k_win_scan<T><<<(int)parts_h.size(), std::max(scanNT, 256), scanSmem, st>>>(
-        parts_d.get(), pchunk0_d.get(), pnchunk_d.get(), koff_d.get(), toff_d.get(), Tm, tails, carry, which, scanG,
-        scanNT, scanNB);
+    by_scan(parts_maxK(), [&](auto KG) {
+      k_win_scan<T, KG()><<<(int)parts_h.size(), std::max(scanNT, 256), scanSmem, st>>>(
+          parts_d.get(), pchunk0_d.get(), pnchunk_d.get(), koff_d.get(), toff_d.get(), Tm, tails, carry, which, scanNB);
+    });
     SAPB_LAUNCHED();
   }
   void window_pair(const double* vin, double* zout, T* gout, int maxK, int nch) {

@@ -133,11 +133,11 @@ __global__ void k_sub_fill(T* __restrict__ dst, int ldd, long long sd, int m, in
 //
 // The whole block stays in shared memory (row-major, ld = n16 + 4), as 16 x 16
 // tiles, one warp per tile and product:
-//   * 16 pivots at a time: warp 0 factors the diagonal tile in registers and
-//     inverts its triangles (tile_lu), which take the tile's place in G; the
-//     panels U12 = L^-1 A12 and L21 = A21 U^-1 follow, then A22 -= L21 U12,
-//     where warp 0 takes the next diagonal tile and factors it at once while
-//     the other warps update the rest;
+//   * 16 pivots at a time: warp 0 factors the diagonal tile in registers; the
+//     panels U12 = L^-1 A12 and L21 = A21 U^-1 follow by substitution, 32
+//     columns or rows per warp, then A22 -= L21 U12, where warp 0 takes the
+//     next diagonal tile and factors it at once while the other warps update
+//     the rest and the last one inverts the tile's triangles in its place;
 //   * the inverses of the two triangular factors grow by doubling, 16 -> 32 ->
 //     64 -> 128: (L^-1)21 = -L22^-1 (L21 L11^-1), (U^-1)12 = -U11^-1 (U12
 //     U22^-1), all pairs and both triangles at once, in place of L21 and U12.
@@ -159,11 +159,11 @@ inline size_t leaf_smem(int n) {
 }
 enum { TILE_FULL = 0, TILE_UNIT_LOWER = 1, TILE_UPPER = 2 };
 // element (r, c) of a 16 x 16 tile of G read as full, unit lower or upper
-template <typename T>
-__device__ __forceinline__ T tile_el(const T* A, int ld, int r, int c, int tri) {
+template <int TRI, typename T>
+__device__ __forceinline__ T tile_el(const T* A, int ld, int r, int c) {
   const T v = A[r * ld + c];
-  if (tri == TILE_UNIT_LOWER) return r > c ? v : (r == c ? T(1) : T(0));
-  if (tri == TILE_UPPER) return r <= c ? v : T(0);
+  if constexpr (TRI == TILE_UNIT_LOWER) return r > c ? v : (r == c ? T(1) : T(0));
+  if constexpr (TRI == TILE_UPPER) return r <= c ? v : T(0);
   return v;
 }
 __device__ __forceinline__ unsigned to_tf32(float v) {
@@ -174,20 +174,20 @@ __device__ __forceinline__ unsigned to_tf32(float v) {
 // acc += A B for 16 x 16 tiles, one warp.  Lane (g, t) = (lane / 4, lane % 4)
 // holds rows g, g + 8 and columns 2t, 2t+1, 8+2t, 9+2t (the accumulator layout
 // of mma.m16n8k8): acc[4 h + 2 i + j] = (g + 8 i, 8 h + 2 t + j).
-template <typename T>
-__device__ __forceinline__ void tile_mac(const T* A, int triA, const T* B, int triB, int ld, bool tc, T acc[8]) {
+template <int TA = TILE_FULL, int TB = TILE_FULL, typename T>
+__device__ __forceinline__ void tile_mac(const T* A, const T* B, int ld, bool tc, T acc[8]) {
   const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
   if constexpr (sizeof(T) == 4) {
     if (tc) {
 #pragma unroll
       for (int k = 0; k < 16; k += 8) {
-        const unsigned a0 = to_tf32(tile_el(A, ld, g, k + t, triA)), a1 = to_tf32(tile_el(A, ld, g + 8, k + t, triA)),
-                       a2 = to_tf32(tile_el(A, ld, g, k + t + 4, triA)),
-                       a3 = to_tf32(tile_el(A, ld, g + 8, k + t + 4, triA));
+        const unsigned a0 = to_tf32(tile_el<TA>(A, ld, g, k + t)), a1 = to_tf32(tile_el<TA>(A, ld, g + 8, k + t)),
+                       a2 = to_tf32(tile_el<TA>(A, ld, g, k + t + 4)),
+                       a3 = to_tf32(tile_el<TA>(A, ld, g + 8, k + t + 4));
 #pragma unroll
         for (int h = 0; h < 2; h++) {
-          const unsigned b0 = to_tf32(tile_el(B, ld, k + t, 8 * h + g, triB)),
-                         b1 = to_tf32(tile_el(B, ld, k + t + 4, 8 * h + g, triB));
+          const unsigned b0 = to_tf32(tile_el<TB>(B, ld, k + t, 8 * h + g)),
+                         b1 = to_tf32(tile_el<TB>(B, ld, k + t + 4, 8 * h + g));
           asm("mma.sync.aligned.m16n8k8.row.col.f32.tf32.tf32.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, "
               "{%0,%1,%2,%3};"
               : "+f"(acc[4 * h]), "+f"(acc[4 * h + 1]), "+f"(acc[4 * h + 2]), "+f"(acc[4 * h + 3])
@@ -199,14 +199,22 @@ __device__ __forceinline__ void tile_mac(const T* A, int triA, const T* B, int t
   }
 #pragma unroll
   for (int k = 0; k < 16; k++) {
-    const T a0 = tile_el(A, ld, g, k, triA), a1 = tile_el(A, ld, g + 8, k, triA);
+    const T a0 = tile_el<TA>(A, ld, g, k), a1 = tile_el<TA>(A, ld, g + 8, k);
+    T bv[4];
+    if constexpr (TB == TILE_FULL && sizeof(T) == 4) {
+      const float2 p = *reinterpret_cast<const float2*>(B + k * ld + 2 * t),
+                   q = *reinterpret_cast<const float2*>(B + k * ld + 8 + 2 * t);
+      bv[0] = p.x, bv[1] = p.y, bv[2] = q.x, bv[3] = q.y;
+    } else {
+#pragma unroll
+      for (int h = 0; h < 4; h++) bv[h] = tile_el<TB>(B, ld, k, 8 * (h >> 1) + 2 * t + (h & 1));
+    }
 #pragma unroll
     for (int h = 0; h < 2; h++)
 #pragma unroll
       for (int j = 0; j < 2; j++) {
-        const T bv = tile_el(B, ld, k, 8 * h + 2 * t + j, triB);
-        acc[4 * h + j] = fma(a0, bv, acc[4 * h + j]);
-        acc[4 * h + 2 + j] = fma(a1, bv, acc[4 * h + 2 + j]);
+        acc[4 * h + j] = fma(a0, bv[2 * h + j], acc[4 * h + j]);
+        acc[4 * h + 2 + j] = fma(a1, bv[2 * h + j], acc[4 * h + 2 + j]);
       }
   }
 }
@@ -230,51 +238,92 @@ __device__ __forceinline__ void tile_sub(T* C, int ld, const T acc[8]) {
 #pragma unroll
       for (int j = 0; j < 2; j++) C[(g + 8 * i) * ld + 8 * h + 2 * t + j] -= acc[4 * h + 2 * i + j];
 }
-// One warp: LU of the 16 x 16 tile A (the first n pivots count for the zero
-// check), then A's strict lower part <- L^-1, its upper part <- U^-1.  Lane l
-// holds row l % 16; lanes 0..15 then solve for a column of L^-1, lanes 16..31
-// for a column of U^-1.
+// One warp: LU of the 16 x 16 tile A in place (the first n pivots count for the
+// zero check); 1 / pivot to rinv.  Lane l holds row l % 16.
 template <typename T>
-__device__ __forceinline__ void tile_lu(T* A, int ld, int n, int boost, int* zero_flag) {
+__device__ __forceinline__ void tile_lu(T* A, int ld, int n, int boost, int* zero_flag, T* rinv) {
   const unsigned full = 0xffffffffu;
   const int lane = threadIdx.x & 31, r = lane & 15;
   T a[16];
 #pragma unroll
   for (int c = 0; c < 16; c++) a[c] = A[r * ld + c];
-  bool zero = false;
+  T low = T(1);
 #pragma unroll
   for (int k = 0; k < 16; k++) {
     T p = __shfl_sync(full, a[k], k);
     if (boost) p = boost_pivot(p);
-    else zero |= k < n && fabs((double)p) < 1e-7;
+    else if (k < n) low = fmin(low, fabs(p));
     const T inv = T(1) / p;
+    if (lane == k) rinv[k] = inv;
     const T l = r > k ? a[k] * inv : T(0);
 #pragma unroll
     for (int c = k + 1; c < 16; c++) a[c] = fma(-l, __shfl_sync(full, a[c], k), a[c]);
     a[k] = r > k ? l : (r == k ? p : a[k]);
   }
-  if (zero && lane == 0) atomicOr(zero_flag, 1);
-  // both solves run in every lane (the shuffles need the whole warp)
-  T xl[16], xu[16];
+  if ((double)low < 1e-7 && lane == 0) atomicOr(zero_flag, 1);
+  if (lane < 16) {
+#pragma unroll
+    for (int c = 0; c < 16; c++) A[r * ld + c] = a[c];
+  }
+}
+// One warp: the LU in tile A replaced by L^-1 (strict lower part) and U^-1
+// (upper part).  Both come from one forward recurrence: lane c < 16 solves for
+// column c of L^-1 from row 0 down, lane 16 + c for column c of U^-1 from row
+// 15 up, which is the same with rows and columns reversed.
+template <typename T>
+__device__ __forceinline__ void tile_inverses(T* A, int ld) {
+  const unsigned full = 0xffffffffu;
+  const int lane = threadIdx.x & 31, r = lane & 15;
+  const bool up = lane >= 16;
+  T b[16], x[16];
+#pragma unroll
+  for (int k = 0; k < 16; k++) b[k] = A[r * ld + (up ? 15 - k : k)];
+  const int e = up ? 15 - r : r;  // the unit right-hand side
 #pragma unroll
   for (int i = 0; i < 16; i++) {
-    T v = i == r ? T(1) : T(0);
+    const int src = up ? 31 - i : i;  // row i, or row 15 - i, of the factor
+    T v = i == e ? T(1) : T(0);
 #pragma unroll
-    for (int k = 0; k < i; k++) v = fma(-__shfl_sync(full, a[k], i), xl[k], v);
-    xl[i] = v;
+    for (int k = 0; k < i; k++) v = fma(-__shfl_sync(full, b[k], src), x[k], v);
+    const T d = __shfl_sync(full, b[i], src);
+    x[i] = v / (up ? d : T(1));
   }
-#pragma unroll
-  for (int i = 15; i >= 0; i--) {
-    T v = i == r ? T(1) : T(0);
-#pragma unroll
-    for (int k = i + 1; k < 16; k++) v = fma(-__shfl_sync(full, a[k], i), xu[k], v);
-    xu[i] = v / __shfl_sync(full, a[i], i);
-  }
+  __syncwarp();
 #pragma unroll
   for (int i = 0; i < 16; i++) {
-    if (lane < 16 && i > r) A[i * ld + r] = xl[i];
-    if (lane >= 16 && i <= r) A[i * ld + r] = xu[i];
+    const int row = up ? 15 - i : i;
+    if (up ? row <= r : row > r) A[row * ld + r] = x[i];
   }
+}
+// One warp, 32 columns (lane's column at P, rows ld apart): P <- L^-1 P for the
+// unit lower triangle of tile A.
+template <typename T>
+__device__ __forceinline__ void panel_lower(const T* A, T* P, int ld) {
+  T x[16];
+#pragma unroll
+  for (int i = 0; i < 16; i++) x[i] = P[i * ld];
+#pragma unroll
+  for (int k = 0; k < 15; k++)
+#pragma unroll
+    for (int i = k + 1; i < 16; i++) x[i] = fma(-A[i * ld + k], x[k], x[i]);
+#pragma unroll
+  for (int i = 1; i < 16; i++) P[i * ld] = x[i];
+}
+// One warp, 32 rows (lane's row at P): P <- P U^-1 for the upper triangle of
+// tile A, whose reciprocal pivots are rinv.
+template <typename T>
+__device__ __forceinline__ void panel_upper(const T* A, const T* rinv, T* P, int ld) {
+  T x[16];
+#pragma unroll
+  for (int c = 0; c < 16; c++) x[c] = P[c];
+#pragma unroll
+  for (int k = 0; k < 16; k++) {
+    x[k] *= rinv[k];
+#pragma unroll
+    for (int c = k + 1; c < 16; c++) x[c] = fma(-x[k], A[k * ld + c], x[c]);
+  }
+#pragma unroll
+  for (int c = 0; c < 16; c++) P[c] = x[c];
 }
 template <typename T>
 __global__ void __launch_bounds__(kLeafThreads)
@@ -288,47 +337,57 @@ k_leaf(const T* __restrict__ M, int ldm, long long sm, T* __restrict__ Li, T* __
   const T* Mb = M + blockIdx.x * sm;
   T* Lb = Li + blockIdx.x * stride;
   T* Ub = Ui + blockIdx.x * stride;
-  for (int c = warp; c < n16; c += nw)
-    for (int r = lane; r < n16; r += 32)
-      G[r * ld + c] = (r < n && c < n) ? Mb[(long long)c * ldm + r] : (r == c ? T(1) : T(0));
+  for (int c0 = warp; c0 < n16; c0 += 4 * nw) {  // 16 loads in flight per thread
+    T v[4][4];
+#pragma unroll
+    for (int i = 0; i < 4; i++)
+#pragma unroll
+      for (int j = 0; j < 4; j++) {
+        const int c = c0 + i * nw, r = lane + 32 * j;
+        v[i][j] = (r < n && c < n) ? Mb[(long long)c * ldm + r] : (r == c ? T(1) : T(0));
+      }
+#pragma unroll
+    for (int i = 0; i < 4; i++)
+#pragma unroll
+      for (int j = 0; j < 4; j++) {
+        const int c = c0 + i * nw, r = lane + 32 * j;
+        if (c < n16 && r < n16) G[r * ld + c] = v[i][j];
+      }
+  }
+  __shared__ T rinv[16];
   __syncthreads();
   auto tile = [&](T* Z, int i, int j) { return Z + (16 * i) * ld + 16 * j; };
   auto apart = [&](int i, int j) { return tc && (i >> 1) != (j >> 1); };
-  if (warp == 0) tile_lu(tile(G, 0, 0), ld, n, boost, zero_flag);
+  if (warp == 0) tile_lu(tile(G, 0, 0), ld, n, boost, zero_flag, rinv);
   __syncthreads();
   for (int k = 0; k < nt; k++) {
-    const int m = nt - 1 - k;
-    for (int q = warp; q < 2 * m; q += nw) {  // panels, in place
-      const int j = k + 1 + (q >> 1);
-      T acc[8] = {};
-      T* P;
-      if (q & 1) {
-        P = tile(G, j, k);
-        tile_mac(P, TILE_FULL, tile(G, k, k), TILE_UPPER, ld, apart(j, k), acc);
-      } else {
-        P = tile(G, k, j);
-        tile_mac(tile(G, k, k), TILE_UNIT_LOWER, P, TILE_FULL, ld, apart(j, k), acc);
+    const int m = nt - 1 - k, half = (m + 1) / 2;  // panels: two tiles per warp
+    if (warp < 2 * half) {
+      const int o = 16 * (k + 1) + 32 * (warp % half) + lane;
+      if (o < n16) {
+        if (warp < half) panel_lower(tile(G, k, k), G + 16 * k * ld + o, ld);
+        else panel_upper(tile(G, k, k), rinv, G + o * ld + 16 * k, ld);
       }
-      __syncwarp();
-      tile_store(P, ld, acc, T(1));
     }
     __syncthreads();
     auto trail = [&](int i, int j) {
       T acc[8] = {};
       // (a pivot tile of another 32-block is a product of the recursion)
-      tile_mac(tile(G, i, k), TILE_FULL, tile(G, k, j), TILE_FULL, ld, tc && (apart(i, k) || apart(j, k)), acc);
+      tile_mac(tile(G, i, k), tile(G, k, j), ld, tc && (apart(i, k) || apart(j, k)), acc);
       tile_sub(tile(G, i, j), ld, acc);
     };
-    if (m > 0) {
-      if (warp == 0) {
+    if (warp == 0) {
+      if (m > 0) {
         trail(k + 1, k + 1);
         __syncwarp();
-        tile_lu(tile(G, k + 1, k + 1), ld, n - 16 * (k + 1), boost, zero_flag);
-      } else {
-        for (int q = warp; q < m * m; q += nw - 1) trail(k + 1 + q / m, k + 1 + q % m);
+        tile_lu(tile(G, k + 1, k + 1), ld, n - 16 * (k + 1), boost, zero_flag, rinv);
       }
-      __syncthreads();
+    } else if (warp == nw - 1) {
+      tile_inverses(tile(G, k, k), ld);
+    } else {
+      for (int q = warp; q < m * m; q += nw - 2) trail(k + 1 + q / m, k + 1 + q % m);
     }
+    __syncthreads();
   }
   // inverses by doubling: blocks of s tiles, pairs (2s tiles); the second of a
   // pair may be cut off by n
@@ -340,31 +399,28 @@ k_leaf(const T* __restrict__ M, int ldm, long long sm, T* __restrict__ Li, T* __
         const int e = q >> 1, pr = e / per, i = (e % per) / s, j = (e % per) % s, o = pr * 2 * s, o2 = o + s;
         const int s2 = min(s, nt - o2);  // tiles of the second block
         if (s2 <= 0) continue;
+        const bool t32 = tc && s > 1;
         T acc[8] = {};
         if (!up) {  // (i, j): rows o2 + i (i < s2), columns o + j
           if (i >= s2) continue;
           if (phase == 0) {  // T = L21 L11^-1
-            for (int k = j; k < s; k++)
-              tile_mac(tile(G, o2 + i, o + k), TILE_FULL, tile(G, o + k, o + j), k == j ? TILE_UNIT_LOWER : TILE_FULL,
-                       ld, tc && s > 1, acc);
+            tile_mac<TILE_FULL, TILE_UNIT_LOWER>(tile(G, o2 + i, o + j), tile(G, o + j, o + j), ld, t32, acc);
+            for (int k = j + 1; k < s; k++) tile_mac(tile(G, o2 + i, o + k), tile(G, o + k, o + j), ld, t32, acc);
             tile_store(tile(X, o2 + i, o + j), ld, acc, T(1));
           } else {  // (L^-1)21 = -L22^-1 T
-            for (int k = 0; k <= i; k++)
-              tile_mac(tile(G, o2 + i, o2 + k), k == i ? TILE_UNIT_LOWER : TILE_FULL, tile(X, o2 + k, o + j),
-                       TILE_FULL, ld, tc && s > 1, acc);
+            for (int k = 0; k < i; k++) tile_mac(tile(G, o2 + i, o2 + k), tile(X, o2 + k, o + j), ld, t32, acc);
+            tile_mac<TILE_UNIT_LOWER>(tile(G, o2 + i, o2 + i), tile(X, o2 + i, o + j), ld, t32, acc);
             tile_store(tile(G, o2 + i, o + j), ld, acc, T(-1));
           }
         } else {  // (i, j): rows o + i, columns o2 + j (j < s2)
           if (j >= s2) continue;
           if (phase == 0) {  // T = U12 U22^-1
-            for (int k = 0; k <= j; k++)
-              tile_mac(tile(G, o + i, o2 + k), TILE_FULL, tile(G, o2 + k, o2 + j), k == j ? TILE_UPPER : TILE_FULL, ld,
-                       tc && s > 1, acc);
+            for (int k = 0; k < j; k++) tile_mac(tile(G, o + i, o2 + k), tile(G, o2 + k, o2 + j), ld, t32, acc);
+            tile_mac<TILE_FULL, TILE_UPPER>(tile(G, o + i, o2 + j), tile(G, o2 + j, o2 + j), ld, t32, acc);
             tile_store(tile(X, o + i, o2 + j), ld, acc, T(1));
           } else {  // (U^-1)12 = -U11^-1 T
-            for (int k = i; k < s; k++)
-              tile_mac(tile(G, o + i, o + k), k == i ? TILE_UPPER : TILE_FULL, tile(X, o + k, o2 + j), TILE_FULL, ld,
-                       tc && s > 1, acc);
+            tile_mac<TILE_UPPER>(tile(G, o + i, o + i), tile(X, o + i, o2 + j), ld, t32, acc);
+            for (int k = i + 1; k < s; k++) tile_mac(tile(G, o + i, o + k), tile(X, o + k, o2 + j), ld, t32, acc);
             tile_store(tile(G, o + i, o2 + j), ld, acc, T(-1));
           }
         }

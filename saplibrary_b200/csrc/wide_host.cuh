@@ -281,7 +281,7 @@ class WideBand {
   DBuf<int> flag;
   // setup workspaces, kept (with everything above) across setups of the
   // same layout so that a repeated setup does not free and re-allocate
-  DBuf<T> Dw, Ww, X, Wt, S, Ws;
+  DBuf<T> Dw, Ww, X, X2, Wt, S, Ws;
   DBuf<T> Rw, Rs;  // recursion workspaces of the partition factors / the reduced system
   DBuf<int> nz_d, spk_cols[2], spk_pos[2], sflag;  // spike-tip setup scratch
 
@@ -289,7 +289,7 @@ class WideBand {
   size_t bytes_held() const {
     size_t b = 0;
     for (const DBuf<T>* d : {&Linv, &Uinv, &Uoff, &Loff, &Vc, &Wc, &Bc, &Cc, &SLi, &SUi, &Fb, &xv, &yv, &tv, &xbt, &fbt,
-                             &t1, &t2, &Dw, &Ww, &X, &Wt, &S, &Ws, &Rw, &Rs, &gws[0], &gws[1], &gws[2], &gws[3], &pws, &csL, &csU,
+                             &t1, &t2, &Dw, &Dw2, &Cu_, &Cl_, &Ww, &X, &X2, &Wt, &S, &Ws, &Rw, &Rs, &gws[0], &gws[1], &gws[2], &gws[3], &pws, &csL, &csU,
                              &csLo, &csUo})
       b += d->size() * sizeof(T);
     for (const DBuf<__half>* d : {&Lh, &Uh, &Loh, &Uoh}) b += d->size() * sizeof(__half);
@@ -576,6 +576,11 @@ class WideBand {
   void factor(bool boost) {
     Dw.alloc((size_t)P * BB);
     Ww.alloc((size_t)P * BB);
+    if (ahead_mode()) {
+      Dw2.alloc((size_t)P * BB);
+      Cu_.alloc((size_t)P * kc * kc);
+      Cl_.alloc((size_t)P * kc * kc);
+    }
     Rw.alloc((size_t)P * std::max(1LL, BlockLU<T>::rec_ws(bs, leaf_size<T>())));
     flag.alloc(1);
     const long long key = (((long long)P * 65537 + bs) * 65537 + nb) * 4 + (boost ? 2 : 0) + (tf32 ? 1 : 0);
@@ -640,20 +645,45 @@ class WideBand {
     lanes(lu);
     lu.rws = std::max(1LL, BlockLU<T>::rec_ws(bs, lu.leaf));
     lu.rw = Rw.get();
-    const Mat<T> D{Dw.get(), bs, BB}, Wm{Ww.get(), bs, BB};
+    const Mat<T> Wm{Ww.get(), bs, BB};
     lu.W = Wm;
-    for (int i = 0; i < nb; i++) {
+    // D_i, loaded into the L_ii^-1 slot, to a workspace; both inverses start from zero
+    auto take = [&](int i, const Mat<T>& D, cudaStream_t s) {
+      SAPB_PROF("wb_copy", s);
       const Mat<T> Li = blk(Linv, nb, i), Ui = blk(Uinv, nb, i);
-      {
-        SAPB_PROF("wb_copy", st);
-        // D_i, loaded into the L_ii^-1 slot, to the workspace; both inverses start from zero
-        k_take_block<T><<<dim3(grid1d(BB * (long long)sizeof(T) / 16, 256, std::max(8, 148 * 8 / P)), P), 256, 0, st>>>(
-            Li.p, Ui.p, Li.s, D.p, D.s, BB);
-        SAPB_LAUNCHED();
+      k_take_block<T><<<dim3(grid1d(BB * (long long)sizeof(T) / 16, 256, std::max(8, 148 * 8 / P)), P), 256, 0, s>>>(
+          Li.p, Ui.p, Li.s, D.p, D.s, BB);
+      SAPB_LAUNCHED();
+    };
+    const int c0 = bs - kc;
+    auto Ec = [&](int i) { return blk(Uoff, nb - 1, i).at(c0, 0); };  // the corners of U_{i,i+1} and L_{i+1,i}
+    auto Fc = [&](int i) { return blk(Loff, nb - 1, i).at(0, c0); };
+    // Small blocks: what a block row only passes on is off its chain.  The next
+    // row's D is taken ahead into a second workspace, and the corners stay in
+    // workspaces that the next Schur complement reads, their copies to the
+    // factor slots running beside it on the second lane.
+    const bool ahead = ahead_mode() && nb > 1;
+    const Mat<T> Db[2] = {Mat<T>{Dw.get(), bs, BB}, ahead ? Mat<T>{Dw2.get(), bs, BB} : Mat<T>{Dw.get(), bs, BB}};
+    const long long sC = (long long)kc * kc;
+    const Mat<T> Cu{Cu_.get(), kc, sC}, Cl{Cl_.get(), kc, sC};
+    if (ahead) take(0, Db[0], st);
+    for (int i = 0; i < nb; i++) {
+      const Mat<T> Li = blk(Linv, nb, i), Ui = blk(Uinv, nb, i), D = Db[i & 1];
+      if (ahead) {
+        lu.fork();
+        lu.lane2([&] {
+          if (i > 0) {
+            lu.copy(Cu, Ec(i - 1), kc, kc);
+            lu.copy(Cl, Fc(i - 1), kc, kc);
+          }
+          if (i + 1 < nb) take(i + 1, Db[(i + 1) & 1], lu.st);
+        });
+      } else {
+        take(i, D, st);
       }
       if (i > 0) {  // D_i -= L_{i,i-1} U_{i-1,i}: upper times lower, in the corner
         SAPB_PROF("wb_schur", st);
-        lu.prod_UL_acc(kc, T(-1), blk(Loff, nb - 1, i - 1).at(0, bs - kc), blk(Uoff, nb - 1, i - 1).at(bs - kc, 0), D);
+        lu.prod_UL_acc(kc, T(-1), ahead ? Cl : Fc(i - 1), ahead ? Cu : Ec(i - 1), D);
       }
       {
         SAPB_PROF("wb_rec", st);
@@ -665,19 +695,21 @@ class WideBand {
         // (upper times upper); D is free again as the second lane's scratch
         SAPB_PROF("wb_offdiag", st);
         lu.fork();
-        const int c0 = bs - kc;
-        const Mat<T> E = blk(Uoff, nb - 1, i).at(c0, 0), F = blk(Loff, nb - 1, i).at(0, c0);
-        lu.prod_LL(kc, T(1), Li.at(c0, c0), E, Wm);
-        lu.copy(Wm, E, kc, kc);
+        lu.prod_LL(kc, T(1), Li.at(c0, c0), Ec(i), ahead ? Cu : Wm);
+        if (!ahead) lu.copy(Wm, Ec(i), kc, kc);
         lu.lane2([&] {
-          lu.prod_UU(kc, T(1), F, Ui.at(c0, c0), D);
-          lu.copy(D, F, kc, kc);
+          lu.prod_UU(kc, T(1), Fc(i), Ui.at(c0, c0), ahead ? Cl : D);
+          if (!ahead) lu.copy(D, Fc(i), kc, kc);
         });
+        lu.join();
+      } else if (ahead) {
         lu.join();
       }
     }
   }
-
+  // blocks whose second workspace is small beside the factors
+  bool ahead_mode() const { return bs <= 512; }
+  DBuf<T> Dw2, Cu_, Cl_;
 
   // tri: 0 full, 1 lower, 2 upper (see k_tgemv).  Grids with fewer than
   // about 2.5 CTAs per SM split the columns over gridDim.z CTAs.
@@ -691,7 +723,8 @@ class WideBand {
   cudaEvent_t ev_fork = nullptr, ev_join = nullptr, ev_lane[kMaxLanes] = {};
   cudaStream_t lane_stream(int lane) const { return lane == 0 ? st : (lane == 1 ? st2 : st_more[lane - 2]); }
   // CTAs one GEMV launch aims at through its column split (about 2.5 of the
-  // three resident CTAs per SM); SAPB_GEMV_CTAS overrides
+  // three resident CTAs per SM; a split that keeps 15 interfaces of K = 2845
+  // below one full wave was slower, 167 against 134 us); SAPB_GEMV_CTAS overrides
   static int gemv_ctas() {
     const char* e = std::getenv("SAPB_GEMV_CTAS");
     return (e && std::atoi(e) > 0) ? std::atoi(e) : 370;
@@ -1092,7 +1125,14 @@ class WideBand {
       const int cs = std::min(ncol, cs_max);
       const long long sX = plen * cs;
       X.ensure((size_t)nI * sX);
-      Wt.ensure((size_t)nI * bs * cs);
+      // a second slab, while both fit the budget and the memory: every product
+      // then writes its block row of the other slab and no copy is needed
+      size_t fr = 0, tot = 0;
+      SAPB_CUDA(cudaMemGetInfo(&fr, &tot));
+      const double slab = (double)nI * (double)sX * sizeof(T);
+      const bool two = 2 * slab <= budget && (X2.size() >= (size_t)nI * sX || 3 * slab <= (double)fr);
+      if (two) X2.ensure((size_t)nI * sX);
+      else Wt.ensure((size_t)nI * bs * cs);
       BlockLU<T> ops;
       ops.h = h;
       ops.st = st;
@@ -1103,6 +1143,7 @@ class WideBand {
       const Mat<T> Wm{Wt.get(), bs, (long long)bs * cs};
       const int ib0 = std::max(0, minpos) / bs;
       auto Xb = [&](int i) { return Mat<T>{X.get() + (long long)i * bs, (int)plen, sX}; };
+      auto Yb = [&](int i) { return two ? Mat<T>{X2.get() + (long long)i * bs, (int)plen, sX} : Xb(i); };
       // factor blocks of partition t + which for interface t
       auto Fk = [&](DBuf<T>& a, int per, int i) {
         return Mat<T>{a.get() + (long long)which * per * BB + (long long)i * BB, bs, (long long)per * BB};
@@ -1120,15 +1161,15 @@ class WideBand {
         // U_{i,i+1} (lower) and U_ii^-1 (upper)
         for (int i = ib0; i < nb; i++) {
           if (i > ib0)
-            ops.prod_UF(kc, w, T(-1), Fk(Loff, nb - 1, i - 1).at(0, bs - kc), Xb(i - 1).at(bs - kc, 0), T(1), Xb(i));
-          ops.prod_LF(bs, w, T(1), Fk(Linv, nb, i), Xb(i), T(0), Wm);
-          ops.copy(Wm, Xb(i), bs, w);
+            ops.prod_UF(kc, w, T(-1), Fk(Loff, nb - 1, i - 1).at(0, bs - kc), Yb(i - 1).at(bs - kc, 0), T(1), Xb(i));
+          ops.prod_LF(bs, w, T(1), Fk(Linv, nb, i), Xb(i), T(0), two ? Yb(i) : Wm);
+          if (!two) ops.copy(Wm, Xb(i), bs, w);
         }
         for (int i = nb - 1; i >= ib0; i--) {
           if (i < nb - 1)
-            ops.prod_LF(kc, w, T(-1), Fk(Uoff, nb - 1, i).at(bs - kc, 0), Xb(i + 1), T(1), Xb(i).at(bs - kc, 0));
-          ops.prod_UF(bs, w, T(1), Fk(Uinv, nb, i), Xb(i), T(0), Wm);
-          ops.copy(Wm, Xb(i), bs, w);
+            ops.prod_LF(kc, w, T(-1), Fk(Uoff, nb - 1, i).at(bs - kc, 0), Xb(i + 1), T(1), Yb(i).at(bs - kc, 0));
+          ops.prod_UF(bs, w, T(1), Fk(Uinv, nb, i), Yb(i), T(0), two ? Xb(i) : Wm);
+          if (!two) ops.copy(Wm, Xb(i), bs, w);
         }
         k_spike_tips<T><<<dim3(w, nI), kt, 0, st>>>(X.get(), sX, plen, cols_d.get(), ncol, j0, pos_d.get(), K, ldK,
                                                      sK, which ? Wc.get() : Vc.get());
@@ -1215,8 +1256,9 @@ class WideBand {
     gemv(SLi.get(), ldK, sK, t1.get(), K, nullptr, 0, t2.get(), K, K, nI, 0, 1);  // t2 = L_S^-1 t1
     gemv(SUi.get(), ldK, sK, t2.get(), K, nullptr, 0, t1.get(), K, K, nI, 0, 2);  // z2 = U_S^-1 t2
     gemv(Vc.get(), ldK, sK, t1.get(), K, xb, s2, t2.get(), K, K, nI, 1, 0);       // z1 = xb - V z2
-    gemv(Bc.get(), ldK, sK, t1.get(), K, fb, s2, fb, s2, K, nI, 1, 0);            // f_b -= B z2
-    gemv(Cc.get(), ldK, sK, t2.get(), K, ft, s2, ft, s2, K, nI, 1, 0);            // f_t -= C z1
+    // the coupling blocks' entries lie within the half-bandwidth: B lower, C upper triangular
+    gemv(Bc.get(), ldK, sK, t1.get(), K, fb, s2, fb, s2, K, nI, 1, 1);            // f_b -= B z2
+    gemv(Cc.get(), ldK, sK, t2.get(), K, ft, s2, ft, s2, K, nI, 1, 2);            // f_t -= C z1
     k_scatter_idx<T><<<grid1d(m), 256, 0, st>>>(irow.get(), fbt.get(), m, F);
     SAPB_LAUNCHED();
   }

@@ -1,4 +1,4 @@
-// Checks sapb::div_rcp_fast (a / b from the reciprocal y = 1 / b with
+// Checks sapb::rcp_fast against T(1) / b and sapb::div_rcp_fast (a / b from the reciprocal y = 1 / b with
 // Markstein's correction, the division of the narrow band factorisation's
 // fast path) against the division operator on the GPU, in double and float:
 // wherever it reports ok, its quotient must equal a / b bit for bit.
@@ -67,6 +67,8 @@ __global__ void k_check(int mode_a, int mode_b, int edge, int spread, int per_th
     const T a = draw<T>(h1, mode_a, edge, spread), b = draw<T>(h2, mode_b, edge, spread);
     const T y = T(1) / b;
     bool ok;
+    const T y1 = sapb::rcp_fast(b, ok);
+    if (ok && B::to(y1) != B::to(y)) bad++;
     const T q1 = sapb::div_rcp_fast(a, b, y, ok), q2 = a / b;
     if (!ok) slow++;
     else if (B::to(q1) != B::to(q2) && !(q1 != q1 && q2 != q2)) bad++;
@@ -96,7 +98,41 @@ void run(int ma, int mb, int edge, int spread, unsigned long long seed, unsigned
   if (ma == 1 && mb == 1) tot[3] += h[1];  // matrix-like values outside the fast path
 }
 
+// every float, and doubles with significands next to powers of two and to all
+// ones (`near` = distance) at random exponents
+__global__ void k_rcp_floats(unsigned long long* counts) {
+  const unsigned long long t = blockIdx.x * (unsigned long long)blockDim.x + threadIdx.x;
+  unsigned long long bad = 0;
+  for (unsigned long long u = t; u < (1ull << 32); u += (unsigned long long)gridDim.x * blockDim.x) {
+    const float b = __uint_as_float((unsigned)u);
+    bool ok;
+    const float y = sapb::rcp_fast(b, ok);
+    if (ok && __float_as_uint(y) != __float_as_uint(1.f / b)) bad++;
+  }
+  atomicAdd(&counts[0], bad);
+}
+__global__ void k_rcp_doubles(unsigned long long* counts) {
+  const unsigned long long t = blockIdx.x * (unsigned long long)blockDim.x + threadIdx.x;
+  unsigned long long bad = 0;
+  for (int i = 0; i < 64; i++) {
+    const unsigned long long h = mix(t * 64 + i), top = 0xfffffffffffffull, near = (h >> 12) % 4096;
+    const unsigned long long m = (h & 1) ? near : ((h & 2) ? top - near : mix(h) & top);
+    const double b = __longlong_as_double((long long)((24 + (h >> 40) % 1998) << 52 | m));
+    bool ok;
+    const double y = sapb::rcp_fast(b, ok);
+    if (ok && y != 1.0 / b) bad++;
+  }
+  atomicAdd(&counts[1], bad);
+}
+
 int main() {
+  unsigned long long *rc, rh[2] = {1, 1};
+  cudaMalloc(&rc, 16);
+  cudaMemset(rc, 0, 16);
+  k_rcp_floats<<<148 * 8, 256>>>(rc);
+  k_rcp_doubles<<<148 * 8, 256>>>(rc);
+  cudaMemcpy(rh, rc, 16, cudaMemcpyDeviceToHost);
+  cudaFree(rc);
   unsigned long long d[4] = {0, 0, 0, 0}, f[4] = {0, 0, 0, 0};
   for (int m = 0; m < 3; m++)
     for (int n = 0; n < 3; n++) {
@@ -105,6 +141,8 @@ int main() {
       run<float>(m, n, 110, 30, 211 + 3 * m + n, f);
       run<float>(m, n, 0, 6, 311 + 3 * m + n, f);
     }
+  f[1] += rh[0];
+  d[1] += rh[1];
   printf("{\"double_pairs\": %llu, \"double_mismatches\": %llu, \"double_outside\": %llu, "
          "\"double_typical_outside\": %llu, \"float_pairs\": %llu, \"float_mismatches\": %llu, "
          "\"float_outside\": %llu, \"float_typical_outside\": %llu}\n",
