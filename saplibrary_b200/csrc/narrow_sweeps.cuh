@@ -292,6 +292,17 @@ k_win_pass3(const PartDev* __restrict__ parts, const ChunkDev* __restrict__ chun
                       first2[c] ? nullptr : carry2 + koff[c], rhs, out);
 }
 
+// Transfer matrices in memory: T(k, u) at [k * TS + u] for carry entry k and tail
+// entry u, rows padded to the scan's own thread layout (a compile-time stride up
+// to K = 64) and to a multiple of four rows, zero-filled (scan_rows x TS values).
+constexpr int scan_stride(int K) { return K <= 8 ? 8 : K <= 16 ? 16 : K <= 32 ? 32 : K <= 64 ? 64 : (K + 3) / 4 * 4; }
+constexpr int scan_rows(int K) { return (K + 3) / 4 * 4; }
+// carry entries per thread: TS * ceil(K / KG) threads take a step
+constexpr int scan_kg(int K) { return K <= 8 ? 2 : K <= 16 ? 8 : K <= 32 ? 32 : K <= 64 ? 8 : K <= 128 ? 16 : 32; }
+inline int scan_threads(int K) {
+  return K <= 32 ? 32 : (scan_stride(K) * ((K + scan_kg(K) - 1) / scan_kg(K)) + 31) / 32 * 32;
+}
+
 // Chunk transfer matrices (see k_transfer): a CTA's warps follow C unit
 // carries each through the chunk, sharing the staged coefficients; grid
 // (chunk, group of carries, solve).
@@ -299,7 +310,7 @@ template <typename T, int R1, int C>
 __global__ void __launch_bounds__(512)
 k_win_transfer(const PartDev* __restrict__ parts, const ChunkDev* __restrict__ chunks,
                const long long* __restrict__ toff, const T* __restrict__ pkd, const T* __restrict__ pku, int KP,
-               T* __restrict__ T1, T* __restrict__ T2, const int* __restrict__ first1,
+               T* __restrict__ T1, T* __restrict__ T2, int TS, const int* __restrict__ first1,
                const int* __restrict__ first2) {
   extern __shared__ __align__(16) unsigned char win_raw[];
   T* stage = reinterpret_cast<T*>(win_raw);
@@ -318,66 +329,64 @@ k_win_transfer(const PartDev* __restrict__ parts, const ChunkDev* __restrict__ c
     return v <= k && k < K ? -pk[(k - K) * ps + v + K - k - 1] : T(0);
   };
   auto out = [&](int c, int v, T x) {
-    if (v >= m - K && k0 + c < K) Tc[(long long)(k0 + c) * K + v - (m - K)] = x;
+    if (v >= m - K && k0 + c < K) Tc[(long long)(k0 + c) * TS + v - (m - K)] = x;
   };
+  // the padding of rows and columns (scan_rows x TS)
+  if (blockIdx.y == 0)
+    for (int e = threadIdx.x; e < scan_rows(K) * TS; e += blockDim.x)
+      if (e / TS >= K || e % TS >= K) Tc[e] = T(0);
   win_sweep<T, R1, C, false>(stage, pk, ps, K, m, nullptr, rhs, out);
 }
 
 // Carry scan of one partition per CTA (see k_scan): the transfer matrices and
 // tails of NB chunks at a time come into shared memory by cp.async (they are
-// contiguous, and copied by all threads), one batch ahead of the chain.  A
-// chain step is then a K x K product by the first K G threads: thread (g, u)
-// holds the KG values T(u, g KG ..) of the step in registers before the carry
-// they multiply is known, G partial sums per row meet in shared memory.  Up to
-// K = 32 one warp has whole rows (G = 1) and no barrier is left but its own.
-// What bounds it is the latency of a step: 0.41 us at K = 10 and 0.8 us at K =
-// 50 (FP64) with the matrix read after the carry.
+// contiguous), one batch ahead of the chain and by warps of their own where
+// there is room for them.  A chain step is a K x K product by NC threads:
+// thread (g, u) holds T(g KG .., u) of the step in registers before the carry
+// they multiply is known; up to K = 32 one warp takes the step (groups add by
+// shuffles, no barrier but its own), above it the groups' sums meet in shared
+// memory.  What bounds it is the instructions of a step, not its arithmetic:
+// with runtime strides and a test per element a step took 912 cycles at K = 10,
+// 1,193 at K = 64 (FP32), 1,408 at K = 50 (FP64).
 template <typename T>
 __host__ __device__ inline size_t scan_pad(size_t values) {  // to a multiple of 16 bytes
   constexpr size_t per = 16 / sizeof(T);
   return (values + per - 1) / per * per;
 }
-// values of one batch: NB matrices, NB tails, each with room for the offset of
-// an unaligned source
+// values of one batch: NB matrices, NB tails (these with room for the offset
+// of an unaligned source)
 template <typename T>
-__host__ __device__ inline size_t scan_batch(int K, int NB) {
-  return scan_pad<T>((size_t)K * K * NB + 4) + scan_pad<T>((size_t)K * NB + 4);
+inline size_t scan_batch(int K, int NB) {
+  return (size_t)scan_rows(K) * scan_stride(K) * NB + scan_pad<T>((size_t)K * NB + 4);
 }
-// values per thread and groups for half-bandwidth K
-constexpr int scan_kg(int K) { return K <= 16 ? 16 : K <= 32 ? 32 : K <= 64 ? 8 : K <= 128 ? 16 : 32; }
-constexpr int scan_groups(int K, int kg) { return (K + kg - 1) / kg; }
-template <typename T, int KG>
-__global__ void __launch_bounds__(sizeof(T) == 8 && KG == 32 ? 256 : 1024)
+// maxK: the widest partition's (its strides hold for all); TSC: scan_stride(maxK)
+// when it is a compile-time class, else 0
+template <typename T, int KG, int TSC>
+__global__ void __launch_bounds__(TSC == 32 ? 512 : 1024)
 k_win_scan(const PartDev* __restrict__ parts, const int* __restrict__ pchunk0, const int* __restrict__ pnchunk,
            const long long* __restrict__ koff, const long long* __restrict__ toff, const T* __restrict__ Tm,
-           const T* __restrict__ tails, T* __restrict__ carry, int which, int NB) {
+           const T* __restrict__ tails, T* __restrict__ carry, int which, int ts, int NC, int NB) {
   const PartDev p = parts[blockIdx.x];
   const int K = p.K, c0 = pchunk0[blockIdx.x], nc = pnchunk[blockIdx.x];
   if (nc <= 1) return;
   const int dir = (which == 1) ? dir1_of(p) : -dir1_of(p);
   extern __shared__ __align__(16) unsigned char win_raw[];
+  constexpr bool WARP = TSC > 0 && TSC <= 32;
+  const int TS = TSC ? TSC : ts, KR = scan_rows(K), KT = KR * TS;
+  const size_t TO = (size_t)KT * NB, SB = TO + scan_pad<T>((size_t)K * NB + 4);
   T* st = reinterpret_cast<T*>(win_raw);
-  const size_t SB = scan_batch<T>(K, NB), TO = scan_pad<T>((size_t)K * K * NB + 4);
-  T* sig = st + 2 * SB;               // K, read up to a multiple of KG
-  const int G = scan_groups(K, KG), NC = (K * G + 31) / 32 * 32;
-  T* red = sig + G * KG;              // G * K
-  const int tid = threadIdx.x, NT = blockDim.x, KK = K * K;
-  const int u = tid % K, g = tid / K;
-  const bool act = g < G;
+  T* sig = st + 2 * SB;                            // the carry, zeros up to KZ
+  const int G = (K + KG - 1) / KG, KZ = WARP ? 32 : G * KG;
+  T* red = sig + KZ;                               // G * TS
+  const int tid = threadIdx.x, NT = blockDim.x;
+  const int u = TSC ? tid % (TSC ? TSC : 1) : tid % ts, g = TSC ? tid / (TSC ? TSC : 1) : tid / ts;
+  const bool act = WARP || g < G;
   const T* Tp = Tm + toff[c0];
   const T* tp = tails + koff[c0];
   T* cp = carry + koff[c0];
   constexpr int V = 16 / (int)sizeof(T);
-  for (int e = tid; e < G * KG; e += NT) sig[e] = T(0);
-  // n contiguous values at src into dst + (src's offset within 16 bytes)
-  auto fetch = [&](T* dst, const T* src, int n) {
-    const int lead = (int)((reinterpret_cast<uintptr_t>(src) & 15) / sizeof(T));
-    const int a = min(n, lead ? V - lead : 0), m = (n - a) / V * V;
-    T* d = dst + lead;
-    for (int e = tid; e < a; e += NT) cp_async_val<T>(d + e, src + e);
-    for (int e = a + tid * V; e < a + m; e += NT * V) cp_async16(d + e, src + e);
-    for (int e = a + m + tid; e < n; e += NT) cp_async_val<T>(d + e, src + e);
-  };
+  for (int e = tid; e < KZ; e += NT) sig[e] = T(0);
+  const int lt = NT > NC ? tid - NC : tid, LT = NT > NC ? NT - NC : NT;  // the copying threads
   // batch b: steps b NB .. ; chunks [lo, lo + cnt) of the partition
   auto batch = [&](int b, int& lo, int& cnt) {
     const int s0 = b * NB;
@@ -387,14 +396,17 @@ k_win_scan(const PartDev* __restrict__ parts, const int* __restrict__ pchunk0, c
   auto issue = [&](int b) {
     int lo, cnt;
     batch(b, lo, cnt);
-    if (cnt > 0) {
-      fetch(st + (b & 1) * SB, Tp + (long long)lo * KK, cnt * KK);
-      fetch(st + (b & 1) * SB + TO, tp + (long long)lo * K, cnt * K);
+    if (cnt > 0 && lt >= 0) {
+      T* d = st + (b & 1) * SB;
+      const T* src = Tp + (long long)lo * KT;
+      for (int e = lt * V; e < cnt * KT; e += LT * V) cp_async16(d + e, src + e);
+      const T* ts_ = tp + (long long)lo * K;
+      for (int e = lt; e < cnt * K; e += LT) cp_async_val<T>(d + TO + e, ts_ + e);
     }
     cp_async_commit();
   };
   auto sync = [&] {
-    if (NC == 32) __syncwarp();
+    if constexpr (WARP) __syncwarp();
     else asm volatile("bar.sync 1, %0;" ::"r"(NC) : "memory");
   };
   issue(0);
@@ -405,48 +417,76 @@ k_win_scan(const PartDev* __restrict__ parts, const int* __restrict__ pchunk0, c
     if (tid >= NC) continue;
     int lo, cnt;
     batch(b, lo, cnt);
-    const T* Tb = st + (b & 1) * SB + (reinterpret_cast<uintptr_t>(Tp + (long long)lo * KK) & 15) / sizeof(T);
-    const T* tb = st + (b & 1) * SB + TO + (reinterpret_cast<uintptr_t>(tp + (long long)lo * K) & 15) / sizeof(T);
+    const int dj = dir > 0 ? 1 : -1;
+    int j = dir > 0 ? 0 : cnt - 1;  // chunk lo + j
+    const T* tq = st + (b & 1) * SB + (long long)j * KT + g * KG * TS + u;
+    const T* lq = st + (b & 1) * SB + TO + j * K + (u < K ? u : 0);
+    T* cq = cp + (long long)(lo + j + dj) * K + u;
     T tv[KG], tl = T(0);
-    auto load = [&](int q) {
-      const int j = dir > 0 ? q : cnt - 1 - q;  // chunk lo + j
-      const T* tc = Tb + j * KK + g * KG * K + u;
+    auto load = [&] {
 #pragma unroll
-      for (int k = 0; k < KG; k++) tv[k] = act && b + q > 0 && g * KG + k < K ? tc[k * K] : T(0);
-      tl = tid < K ? tb[j * K + tid] : T(0);
+      for (int k = 0; k < KG; k += KG < 4 ? KG : 4)
+        if (act && g * KG + k < KR) {
+#pragma unroll
+          for (int i = 0; i < (KG < 4 ? KG : 4); i++) tv[k + i] = tq[(k + i) * TS];
+        }
+      tl = *lq;
     };
-    load(0);
-    for (int q = 0; q < cnt; q++) {
-      const int j = dir > 0 ? q : cnt - 1 - q;
-      const T* sg = sig + g * KG;
-      T acc[4] = {G == 1 ? tl : T(0), T(0), T(0), T(0)};
-      if (act) {
 #pragma unroll
-        for (int k = 0; k < KG; k++) acc[k & 3] = fma(tv[k], sg[k], acc[k & 3]);
+    for (int k = 0; k < KG; k++) tv[k] = T(0);
+    load();
+    for (int q = 0; q < cnt; q++) {
+      T acc[4] = {T(0), T(0), T(0), T(0)};
+      if (b + q > 0) {  // (no carry enters the first chunk)
+        const T* sg = sig + g * KG;
+#pragma unroll
+        for (int k = 0; k < KG; k += KG < 4 ? KG : 4)
+          if (act && g * KG + k < KR) {
+            T x[4];
+            if constexpr (KG % 4 == 0 && sizeof(T) == 4) {
+              const float4 f = *reinterpret_cast<const float4*>(sg + k);
+              x[0] = f.x, x[1] = f.y, x[2] = f.z, x[3] = f.w;
+            } else if constexpr (KG % 4 == 0) {
+              const double2 f = *reinterpret_cast<const double2*>(sg + k), h = *reinterpret_cast<const double2*>(sg + k + 2);
+              x[0] = f.x, x[1] = f.y, x[2] = h.x, x[3] = h.y;
+            } else {
+#pragma unroll
+              for (int i = 0; i < KG; i++) x[i] = sg[i];
+            }
+#pragma unroll
+            for (int i = 0; i < (KG < 4 ? KG : 4); i++) acc[i] = fma(tv[k + i], x[i], acc[i]);
+          }
       }
       T v = (acc[0] + acc[1]) + (acc[2] + acc[3]);
       const T tail = tl;
-      if (q + 1 < cnt) load(q + 1);
-      if (G > 1) {
-        if (act) red[g * K + u] = v;
+      tq += (long long)dj * KT;
+      lq += dj * K;
+      if (q + 1 < cnt) load();
+      if constexpr (WARP) {
+#pragma unroll
+        for (int off = TSC; off < 32; off *= 2) v += __shfl_xor_sync(0xffffffffu, v, off);
+        v += tail;
+        sync();  // all lanes have read the carry
+      } else {
+        if (act) red[g * TS + u] = v;
         sync();
-        if (tid < K) {
+        if (g == 0 && u < K) {
           T s0 = tail, s1 = T(0);
           int r = 0;
+#pragma unroll 4
           for (; r + 1 < G; r += 2) {
-            s0 += red[r * K + tid];
-            s1 += red[(r + 1) * K + tid];
+            s0 += red[r * TS + u];
+            s1 += red[(r + 1) * TS + u];
           }
-          if (r < G) s0 += red[r * K + tid];
+          if (r < G) s0 += red[r * TS + u];
           v = s0 + s1;
         }
-      } else {
-        sync();  // all lanes have read the carry
       }
-      if (tid < K) {
-        cp[(long long)(lo + j + dir) * K + tid] = v;
-        sig[tid] = v;
+      if (g == 0 && u < K) {
+        *cq = v;
+        sig[u] = v;
       }
+      cq += dj * K;
       sync();
     }
   }

@@ -1071,7 +1071,7 @@ class PrecondT : public PrecBase {
         koff.push_back(ko);
         toff.push_back(to);
         ko += Kp;
-        to += (long long)Kp * Kp;
+        to += window(maxK) ? (long long)scan_rows(Kp) * scan_stride(maxK) : (long long)Kp * Kp;
         bool down1 = !d.ul;
         first1.push_back(down1 ? (c == 0) : (c == nc - 1));
         first2.push_back(down1 ? (c == nc - 1) : (c == 0));
@@ -1159,7 +1159,7 @@ class PrecondT : public PrecBase {
   // Transfer matrices of the register-window sweeps, and the carry scan's
   // launch shape: batches of as many chunks as fit twice in shared memory
   // (one from K ~ 82 in FP64, ~ 116 in FP32 on).
-  int scanNT = 32, scanNB = 1;
+  int scanNC = 32, scanNB = 1;
   size_t scanSmem = 0;
   void build_window(int maxK, int nch) {
     auto t0 = Clock::now();
@@ -1174,12 +1174,12 @@ class PrecondT : public PrecBase {
       allow_smem(k_win_pass2<T, R1()>, smem);
       allow_smem(k_win_pass3<T, R1()>, smem);
       kern<<<dim3(nch, (maxK + C * warps - 1) / (C * warps), 2), 32 * warps, smem, st>>>(
-          parts_d.get(), chunks_d.get(), toff_d.get(), pkd.get(), pku.get(), KP, T1.get(), T2.get(), first1_d.get(), first2_d.get());
+          parts_d.get(), chunks_d.get(), toff_d.get(), pkd.get(), pku.get(), KP, T1.get(), T2.get(),
+          scan_stride(maxK), first1_d.get(), first2_d.get());
     });
     SAPB_LAUNCHED();
-    const int kg = scan_kg(maxK), groups = scan_groups(maxK, kg);
-    scanNT = ((maxK * groups + 31) / 32) * 32;
-    const size_t fixed = (size_t)(groups * kg + scanNT) * sizeof(T);
+    scanNC = scan_threads(maxK);
+    const size_t fixed = (size_t)(64 + (maxK + 31) / 32 * 32 + std::max(scanNC, 32)) * sizeof(T);
     int longest = 1;
     for (size_t c = 0, run = 0; c < chunks_h.size(); c++) {
       run = c > 0 && chunks_h[c].part == chunks_h[c - 1].part ? run + 1 : 1;
@@ -1189,23 +1189,27 @@ class PrecondT : public PrecBase {
     scanNB = 1;
     while (scanNB < 64 && scanNB < longest && bytes(scanNB * 2) <= 200 * 1024) scanNB *= 2;
     scanSmem = bytes(scanNB);
-    by_scan(maxK, [&](auto KG) { allow_smem(k_win_scan<T, KG()>, scanSmem); });
+    by_scan(maxK, [&](auto KG, auto TS) { allow_smem(k_win_scan<T, KG(), TS()>, scanSmem); });
     SAPB_CUDA(cudaStreamSynchronize(st));
     t_assembly += ms_since(t0);
   }
   template <class F>
   static void by_scan(int k, F&& f) {
-    switch (scan_kg(k)) {
-      case 8: f(std::integral_constant<int, 8>{}); break;
-      case 16: f(std::integral_constant<int, 16>{}); break;
-      default: f(std::integral_constant<int, 32>{}); break;
-    }
+    using std::integral_constant;
+    if (k <= 8) f(integral_constant<int, 2>{}, integral_constant<int, 8>{});
+    else if (k <= 16) f(integral_constant<int, 8>{}, integral_constant<int, 16>{});
+    else if (k <= 32) f(integral_constant<int, 32>{}, integral_constant<int, 32>{});
+    else if (k <= 64) f(integral_constant<int, 8>{}, integral_constant<int, 64>{});
+    else if (k <= 128) f(integral_constant<int, 16>{}, integral_constant<int, 0>{});
+    else f(integral_constant<int, 32>{}, integral_constant<int, 0>{});
   }
   void window_scan(const T* Tm, const T* tails, T* carry, int which) {
     SAPB_PROF("scan", st);
-    by_scan(parts_maxK(), [&](auto KG) {
-      k_win_scan<T, KG()><<<(int)parts_h.size(), std::max(scanNT, 256), scanSmem, st>>>(
-          parts_d.get(), pchunk0_d.get(), pnchunk_d.get(), koff_d.get(), toff_d.get(), Tm, tails, carry, which, scanNB);
+    const int maxK = parts_maxK();
+    by_scan(maxK, [&](auto KG, auto TS) {
+      k_win_scan<T, KG(), TS()><<<(int)parts_h.size(), std::min(TS() == 32 ? 512 : 1024, scanNC + 256), scanSmem, st>>>(
+          parts_d.get(), pchunk0_d.get(), pnchunk_d.get(), koff_d.get(), toff_d.get(), Tm, tails, carry, which,
+          scan_stride(maxK), scanNC, scanNB);
     });
     SAPB_LAUNCHED();
   }
