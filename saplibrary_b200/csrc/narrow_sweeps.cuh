@@ -14,8 +14,11 @@ namespace sapb {
 // K x K stages of the carry scan still fit in shared memory.
 template <typename T>
 constexpr int kWinMaxK = sizeof(T) == 8 ? 112 : 160;
-// 32-row register slots a lane needs for half-bandwidth K
-constexpr int win_slots(int K) { return (31 + K) / 32 + 1; }
+// Lanes that hold a chunk's window: the warp, or half of it (two chunks per
+// warp in the passes) up to K = 16, where most of 32 lanes would be past the
+// band; and the register slots a lane then needs
+constexpr int win_lanes(int K) { return K <= 16 ? 16 : 32; }
+constexpr int win_slots(int K, int LW = 32) { return (LW - 1 + K) / LW + 1; }
 
 // Packed factors: for every band row c its K coefficients towards the rows
 // below (pkd: factor entry (c+t, c) at [c][t-1]) and towards the rows above
@@ -27,15 +30,15 @@ __host__ __device__ inline int pack_stride(int K) {
   return (K + per - 1) / per * per;
 }
 
-// Coefficient staging: kStageRows packed rows per stage, kStages stages, one
-// window group of 32 rows in all (some 1,000 cycles ahead of its use).  A row
-// occupies 32 R1 values of shared memory, zeros after its K coefficients, so
-// that lanes left and right of the coefficients read zeros without a test.
+// Coefficient staging: kStageRows packed rows per stage, kStages stages (32
+// rows, some 1,000 cycles ahead of their use).  A row occupies LW R1 values of
+// shared memory, zeros after its K coefficients, so that lanes left and right
+// of the coefficients read zeros without a test.
 constexpr int kStageRows = 8;
 constexpr int kStages = 4;
-static_assert(kStageRows * kStages == 32, "the stages hold one group of 32 rows");
+constexpr int kRingRows = kStageRows * kStages;
 template <typename T>
-constexpr size_t win_smem(int R1) { return (size_t)(32 * 32 * R1 + 32) * sizeof(T); }
+constexpr size_t win_smem(int R1, int LW = 32) { return (size_t)(32 / LW) * (kRingRows * LW * R1 + 32) * sizeof(T); }
 
 // Forward substitution with a unit triangular band factor over the rows
 // v = 0 .. m-1 in processing order, C right-hand sides per warp:
@@ -57,22 +60,28 @@ constexpr size_t win_smem(int R1) { return (size_t)(32 * 32 * R1 + 32) * sizeof(
 // rhs(c, v) is called once per row, by the lane that holds it, at least 32
 // rows ahead of out(c, v, x), which is called once per row.  The staging area
 // (win_smem) is cleared on entry.
-// SOLO: the CTA is one warp.
-template <typename T, int R1, int C, bool SOLO, typename Rhs, typename Out>
+// SOLO: the CTA is one warp.  LW < 32 (SOLO, C = 1): every LW lanes have a sweep
+// of their own -- all arguments are theirs -- over windows of LW rows.
+template <typename T, int R1, int C, bool SOLO, int LW = 32, typename Rhs, typename Out>
 __device__ __forceinline__ void win_sweep(T* sm, const T* __restrict__ pk, long long pstep, int K, int m,
                                           const T* __restrict__ cr, Rhs rhs, Out out) {
-  constexpr int RS = 32 * R1, V = 16 / (int)sizeof(T), SR = kStageRows;
-  const int lane = threadIdx.x & 31, warp = SOLO ? 0 : threadIdx.x >> 5, nwarp = SOLO ? 1 : blockDim.x >> 5;
+  constexpr int RS = LW * R1, V = 16 / (int)sizeof(T), SR = kStageRows;
+  static_assert(LW == 32 || (SOLO && C == 1 && LW % SR == 0), "window lanes");
+  const int lane = threadIdx.x & (LW - 1), warp = SOLO ? 0 : threadIdx.x >> 5, nwarp = SOLO ? 1 : blockDim.x >> 5;
   const unsigned full = 0xffffffffu;
   const int nv = pack_stride<T>(K) / V;  // 16-byte pieces of a row, at most 64
   auto sync = [] {
     if constexpr (SOLO) __syncwarp();
     else __syncthreads();
   };
-  for (int e = threadIdx.x; e < (32 * RS + 32) / V; e += blockDim.x)
+  constexpr int AREA = kRingRows * RS + 32;
+  for (int e = threadIdx.x; e < AREA * (32 / LW) / V; e += blockDim.x)
     reinterpret_cast<uint4*>(sm)[e] = make_uint4(0, 0, 0, 0);
   sync();
-  T* stage = sm + 32;
+  T* stage = sm + (LW < 32 ? (threadIdx.x & 31) / LW * AREA : 0) + 32;
+  int m_all = m;  // the longest sweep of the warp
+#pragma unroll
+  for (int off = LW; off < 32; off *= 2) m_all = max(m_all, __shfl_xor_sync(full, m_all, off));
   const T* next = pk + lane * V;  // the lane's piece of the next row to stage
   auto issue = [&](int s0, int slot) {  // rows s0 .. s0 + SR - 1
     T* dst = stage + slot * SR * RS + lane * V;
@@ -82,7 +91,7 @@ __device__ __forceinline__ void win_sweep(T* sm, const T* __restrict__ pk, long 
 #pragma unroll
           for (int r = 0; r < SR; r++) cp_async16(dst + r * RS, next + r * pstep);
         }
-        if (lane + 32 < nv) {
+        if (LW == 32 && lane + 32 < nv) {
 #pragma unroll
           for (int r = 0; r < SR; r++) cp_async16(dst + r * RS + 32 * V, next + r * pstep + 32 * V);
         }
@@ -95,7 +104,7 @@ __device__ __forceinline__ void win_sweep(T* sm, const T* __restrict__ pk, long 
       }
     } else {
       for (int r = warp; r < SR; r += nwarp)
-        for (int e = lane; e < nv; e += 32) {
+        for (int e = lane; e < nv; e += LW) {
           T* d = dst + r * RS + (e - lane) * V;
           if (s0 + r < m) {
             cp_async16(d, next + r * pstep + (e - lane) * V);
@@ -115,7 +124,7 @@ __device__ __forceinline__ void win_sweep(T* sm, const T* __restrict__ pk, long 
   for (int t = 0; t < R1; t++)
 #pragma unroll
     for (int c = 0; c < C; c++) {
-      const int v = lane + 32 * t;
+      const int v = lane + LW * t;
       w[c][t] = v < m ? rhs(c, v) : T(0);
     }
   if (cr) {
@@ -125,39 +134,40 @@ __device__ __forceinline__ void win_sweep(T* sm, const T* __restrict__ pk, long 
       const T x = cr[k];
 #pragma unroll
       for (int t = 0; t + 1 < R1; t++)
-        if (lane + 32 * t <= k) w[0][t] = fma(-src[k * pstep - k + 32 * t], x, w[0][t]);
+        if (lane + LW * t <= k) w[0][t] = fma(-src[k * pstep - k + LW * t], x, w[0][t]);
     }
   }
-  for (int base = 0; base < m; base += 32) {
+  int slot = 0;
+  for (int base = 0; base < m_all; base += LW) {
     T nw[C];
 #pragma unroll
     for (int c = 0; c < C; c++) {
-      const int v = base + 32 * R1 + lane;
+      const int v = base + LW * R1 + lane;
       nw[c] = v < m ? rhs(c, v) : T(0);
     }
     // (one stage of code: an unrolled group does not stay in the instruction
     // cache a single warp runs from)
 #pragma unroll 1
-    for (int h = 0; h < 32; h += SR) {
+    for (int h = 0; h < LW; h += SR, slot = (slot + 1) % kStages) {
       cp_async_wait<kStages - 2>();
       sync();
-      issue(base + h + (kStages - 1) * SR, h == 0 ? kStages - 1 : h / SR - 1);
+      issue(base + h + (kStages - 1) * SR, (slot + kStages - 1) % kStages);
 #pragma unroll
       for (int b4 = 0; b4 < SR; b4 += 4) {
         const int i = h + b4;
-        const T* row = stage + i * RS;     // the four source rows
+        const T* row = stage + (slot * SR + b4) * RS;  // the four source rows
         const T* cl = row + lane - i - 1;  // lane's coefficients of row i (zeros outside 0..K-1)
         const T l10 = row[0], l20 = row[1], l30 = row[2], l21 = row[RS], l31 = row[RS + 1], l32 = row[2 * RS];
         T cf[4][R1];
 #pragma unroll
         for (int r = 0; r < 4; r++)
 #pragma unroll
-          for (int t = 0; t < R1; t++) cf[r][t] = cl[r * RS - r + 32 * t];
+          for (int t = 0; t < R1; t++) cf[r][t] = cl[r * RS - r + LW * t];
 #pragma unroll
         for (int c = 0; c < C; c++) {
-          const T x0 = __shfl_sync(full, w[c][0], i);
-          T x1 = __shfl_sync(full, w[c][0], i + 1), x2 = __shfl_sync(full, w[c][0], i + 2),
-            x3 = __shfl_sync(full, w[c][0], i + 3);
+          const T x0 = __shfl_sync(full, w[c][0], i, LW);
+          T x1 = __shfl_sync(full, w[c][0], i + 1, LW), x2 = __shfl_sync(full, w[c][0], i + 2, LW),
+            x3 = __shfl_sync(full, w[c][0], i + 3, LW);
           x1 = fma(-l10, x0, x1);
           x2 = fma(-l21, x1, fma(-l20, x0, x2));
           x3 = fma(-l32, x2, fma(-l31, x1, fma(-l30, x0, x3)));
@@ -211,17 +221,23 @@ __global__ void k_pack(const PartDev* __restrict__ parts, const T* __restrict__ 
 // The three passes of a chunked partition sweep (see precond_kernels.cuh), one
 // warp per chunk.  Apply of a 200,000-row half-bandwidth 64 FP32 band in 32
 // partitions: see k_win_scan.
-template <typename T, int R1>
+// The chunk of this lane's window (past the last one: a sweep of no rows).
+template <int LW>
+__device__ __forceinline__ int win_chunk() {
+  return (int)blockIdx.x * (32 / LW) + (LW < 32 ? (int)threadIdx.x / LW : 0);
+}
+template <typename T, int R1, int LW>
 __global__ void __launch_bounds__(32)
 k_win_pass1(const PartDev* __restrict__ parts, const ChunkDev* __restrict__ chunks, const long long* __restrict__ koff,
             const T* __restrict__ pkd, const T* __restrict__ pku, int KP, const double* __restrict__ vin, T* F,
-            T* __restrict__ tails, const int* __restrict__ gin, const T* __restrict__ sin) {
+            T* __restrict__ tails, const int* __restrict__ gin, const T* __restrict__ sin, int nch) {
   extern __shared__ __align__(16) unsigned char win_raw[];
   T* stage = reinterpret_cast<T*>(win_raw);
-  const ChunkDev ch = chunks[blockIdx.x];
+  const int ci = win_chunk<LW>(), c = min(ci, nch - 1);
+  const ChunkDev ch = chunks[c];
   const PartDev p = parts[ch.part];
-  const int K = p.K, m = ch.b - ch.a, dir = dir1_of(p), o = dir > 0 ? ch.a : ch.b - 1;
-  T* tl = tails + koff[blockIdx.x];
+  const int K = p.K, m = ci < nch ? ch.b - ch.a : 0, dir = dir1_of(p), o = dir > 0 ? ch.a : ch.b - 1;
+  T* tl = tails + koff[c];
   auto rhs = [&](int, int v) -> T {
     const int row = o + dir * v;
     if (!vin) return F[row];
@@ -234,27 +250,28 @@ k_win_pass1(const PartDev* __restrict__ parts, const ChunkDev* __restrict__ chun
   auto out = [&](int, int v, T x) {
     if (v >= m - K) tl[v - (m - K)] = x;
   };
-  win_sweep<T, R1, 1, true>(stage, (dir > 0 ? pkd : pku) + (long long)o * KP, dir * KP, K, m, nullptr, rhs, out);
+  win_sweep<T, R1, 1, true, LW>(stage, (dir > 0 ? pkd : pku) + (long long)o * KP, dir * KP, K, m, nullptr, rhs, out);
 }
 
-template <typename T, int R1>
+template <typename T, int R1, int LW>
 __global__ void __launch_bounds__(32)
 k_win_pass2(const PartDev* __restrict__ parts, const ChunkDev* __restrict__ chunks, const int* __restrict__ first1,
             const long long* __restrict__ koff, const T* __restrict__ pkd, const T* __restrict__ pku, int KP,
-            const T* __restrict__ piv, const T* __restrict__ F, const T* __restrict__ carry1, T* Y, T* __restrict__ tails2) {
+            const T* __restrict__ piv, const T* __restrict__ F, const T* __restrict__ carry1, T* Y,
+            T* __restrict__ tails2, int nch) {
   extern __shared__ __align__(16) unsigned char win_raw[];
   T* stage = reinterpret_cast<T*>(win_raw);
-  const int c = blockIdx.x;
+  const int ci = win_chunk<LW>(), c = min(ci, nch - 1);
   const ChunkDev ch = chunks[c];
   const PartDev p = parts[ch.part];
-  const int K = p.K, m = ch.b - ch.a, dir = dir1_of(p), o = dir > 0 ? ch.a : ch.b - 1;
+  const int K = p.K, m = ci < nch ? ch.b - ch.a : 0, dir = dir1_of(p), o = dir > 0 ? ch.a : ch.b - 1;
   {
     auto rhs = [&](int, int v) -> T { return F[o + dir * v]; };
     auto out = [&](int, int v, T x) {
       const int row = o + dir * v;
       Y[row] = x / piv[row];
     };
-    win_sweep<T, R1, 1, true>(stage, (dir > 0 ? pkd : pku) + (long long)o * KP, dir * KP, K, m,
+    win_sweep<T, R1, 1, true, LW>(stage, (dir > 0 ? pkd : pku) + (long long)o * KP, dir * KP, K, m,
                         first1[c] ? nullptr : carry1 + koff[c], rhs, out);
   }
   const int dir2 = -dir, o2 = dir2 > 0 ? ch.a : ch.b - 1;
@@ -263,21 +280,21 @@ k_win_pass2(const PartDev* __restrict__ parts, const ChunkDev* __restrict__ chun
   auto out = [&](int, int v, T x) {
     if (v >= m - K) tl[v - (m - K)] = x;
   };
-  win_sweep<T, R1, 1, true>(stage, (dir2 > 0 ? pkd : pku) + (long long)o2 * KP, dir2 * KP, K, m, nullptr, rhs, out);
+  win_sweep<T, R1, 1, true, LW>(stage, (dir2 > 0 ? pkd : pku) + (long long)o2 * KP, dir2 * KP, K, m, nullptr, rhs, out);
 }
 
-template <typename T, int R1>
+template <typename T, int R1, int LW>
 __global__ void __launch_bounds__(32)
 k_win_pass3(const PartDev* __restrict__ parts, const ChunkDev* __restrict__ chunks, const int* __restrict__ first2,
             const long long* __restrict__ koff, const T* __restrict__ pkd, const T* __restrict__ pku, int KP,
             const T* __restrict__ Y, const T* __restrict__ carry2, double* __restrict__ zout, T* __restrict__ gout,
-            const int* __restrict__ sout, const T* __restrict__ cout) {
+            const int* __restrict__ sout, const T* __restrict__ cout, int nch) {
   extern __shared__ __align__(16) unsigned char win_raw[];
   T* stage = reinterpret_cast<T*>(win_raw);
-  const int c = blockIdx.x;
+  const int ci = win_chunk<LW>(), c = min(ci, nch - 1);
   const ChunkDev ch = chunks[c];
   const PartDev p = parts[ch.part];
-  const int K = p.K, m = ch.b - ch.a, dir = -dir1_of(p), o = dir > 0 ? ch.a : ch.b - 1;
+  const int K = p.K, m = ci < nch ? ch.b - ch.a : 0, dir = -dir1_of(p), o = dir > 0 ? ch.a : ch.b - 1;
   auto rhs = [&](int, int v) -> T { return Y[o + dir * v]; };
   auto out = [&](int, int v, T x) {
     const int row = o + dir * v;
@@ -288,7 +305,7 @@ k_win_pass3(const PartDev* __restrict__ parts, const ChunkDev* __restrict__ chun
       gout[row] = x;
     }
   };
-  win_sweep<T, R1, 1, true>(stage, (dir > 0 ? pkd : pku) + (long long)o * KP, dir * KP, K, m,
+  win_sweep<T, R1, 1, true, LW>(stage, (dir > 0 ? pkd : pku) + (long long)o * KP, dir * KP, K, m,
                       first2[c] ? nullptr : carry2 + koff[c], rhs, out);
 }
 

@@ -906,6 +906,13 @@ class PrecondT : public PrecBase {
       default: f(std::integral_constant<int, 6>{}); break;
     }
   }
+  // the same for the passes: slots and lanes per window
+  template <class F>
+  static void by_pass(int k, F&& f) {
+    using std::integral_constant;
+    if (win_lanes(k) == 16) return f(integral_constant<int, win_slots(16, 16)>{}, integral_constant<int, 16>{});
+    by_window(k, [&](auto R1) { f(R1, integral_constant<int, 32>{}); });
+  }
   template <class Kern>
   static void allow_smem(Kern kern, size_t bytes) {
     if (bytes > 48 * 1024)
@@ -1170,9 +1177,6 @@ class PrecondT : public PrecBase {
       auto kern = k_win_transfer<T, R1(), C>;
       constexpr size_t smem = win_smem<T>(R1());
       allow_smem(kern, smem);
-      allow_smem(k_win_pass1<T, R1()>, smem);
-      allow_smem(k_win_pass2<T, R1()>, smem);
-      allow_smem(k_win_pass3<T, R1()>, smem);
       kern<<<dim3(nch, (maxK + C * warps - 1) / (C * warps), 2), 32 * warps, smem, st>>>(
           parts_d.get(), chunks_d.get(), toff_d.get(), pkd.get(), pku.get(), KP, T1.get(), T2.get(),
           scan_stride(maxK), first1_d.get(), first2_d.get());
@@ -1214,29 +1218,30 @@ class PrecondT : public PrecBase {
     SAPB_LAUNCHED();
   }
   void window_pair(const double* vin, double* zout, T* gout, int maxK, int nch) {
-    by_window(maxK, [&](auto R1) {
-      constexpr size_t smem = win_smem<T>(R1());
+    by_pass(maxK, [&](auto R1, auto LW) {
+      constexpr size_t smem = win_smem<T>(R1(), LW());
+      const int grid = (nch + 32 / LW() - 1) / (32 / LW());
       {
         SAPB_PROF("pass1", st);
-        k_win_pass1<T, R1()><<<nch, 32, smem, st>>>(parts_d.get(), chunks_d.get(), koff_d.get(), pkd.get(), pku.get(),
+        k_win_pass1<T, R1(), LW()><<<grid, 32, smem, st>>>(parts_d.get(), chunks_d.get(), koff_d.get(), pkd.get(), pku.get(),
                                                     KP, vin, F.get(), tails1.get(), reordered ? gin_d.get() : nullptr,
-                                                    in_scale());
+                                                    in_scale(), nch);
         SAPB_LAUNCHED();
       }
       window_scan(T1.get(), tails1.get(), carry1.get(), 1);
       {
         SAPB_PROF("pass2", st);
-        k_win_pass2<T, R1()><<<nch, 32, smem, st>>>(parts_d.get(), chunks_d.get(), first1_d.get(), koff_d.get(),
+        k_win_pass2<T, R1(), LW()><<<grid, 32, smem, st>>>(parts_d.get(), chunks_d.get(), first1_d.get(), koff_d.get(),
                                                     pkd.get(), pku.get(), KP, piv.get(), F.get(), carry1.get(),
-                                                    Y.get(), tails2.get());
+                                                    Y.get(), tails2.get(), nch);
         SAPB_LAUNCHED();
       }
       window_scan(T2.get(), tails2.get(), carry2.get(), 2);
       {
         SAPB_PROF("pass3", st);
-        k_win_pass3<T, R1()><<<nch, 32, smem, st>>>(parts_d.get(), chunks_d.get(), first2_d.get(), koff_d.get(),
+        k_win_pass3<T, R1(), LW()><<<grid, 32, smem, st>>>(parts_d.get(), chunks_d.get(), first2_d.get(), koff_d.get(),
                                                     pkd.get(), pku.get(), KP, Y.get(), carry2.get(), zout, gout,
-                                                    reordered ? sout_d.get() : nullptr, out_scale());
+                                                    reordered ? sout_d.get() : nullptr, out_scale(), nch);
         SAPB_LAUNCHED();
       }
     });
