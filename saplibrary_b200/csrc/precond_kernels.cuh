@@ -303,7 +303,8 @@ k_factor_panel(const FactorJob* __restrict__ jobs, T* __restrict__ B, T* __restr
     return (long long)col * SW + pos;
   };
   auto wrap = [&](int s) { return s >= W ? s - W : s; };  // for 0 <= s < 2 W
-  const bool tail = lane + 32 * (R - 1) < K + NB;  // the last row slot of this lane is in use
+  // rows a panel touches (a partition narrower than the widest has fewer than 32 R)
+  auto on = [&](int t) { return lane + 32 * t < K + NB; };
   for (int e = tid; e < NB; e += blockDim.x) win[e - NB] = T(0);
   for (int e = tid; e < W * (NB - 1); e += blockDim.x) win[(e / (NB - 1)) * SP + SW + e % (NB - 1)] = T(0);
   if (warp != 0) {  // columns [0, K + NB), then one panel's new columns per group; all in slots == column
@@ -323,7 +324,7 @@ k_factor_panel(const FactorJob* __restrict__ jobs, T* __restrict__ B, T* __restr
       for (int c = 0; c < NB; c++) {
         const T* colp = win + wrap(s + c) * SP + K - c + lane;  // row j + lane + 32 t
 #pragma unroll
-        for (int t = 0; t < R; t++) a[t][c] = (c < nb && (t + 1 < R || tail)) ? colp[32 * t] : T(0);
+        for (int t = 0; t < R; t++) a[t][c] = (c < nb && on(t)) ? colp[32 * t] : T(0);
       }
     };
     load_panel();
@@ -396,7 +397,7 @@ k_factor_panel(const FactorJob* __restrict__ jobs, T* __restrict__ B, T* __restr
       T* colp = win + wrap(s + c) * SP + K - c + lane;
 #pragma unroll
       for (int t = 0; t < R; t++)
-        if (c < nb && (t + 1 < R || tail)) colp[32 * t] = a[t][c];
+        if (c < nb && on(t)) colp[32 * t] = a[t][c];
     }
     if (!do_boost) {  // the pivots as used
       __syncwarp();
@@ -413,7 +414,7 @@ k_factor_panel(const FactorJob* __restrict__ jobs, T* __restrict__ B, T* __restr
     for (int i = 0; i < NC; i++) {
       colp[i] = win + wrap(s0 + NB + q0 + i) * SP + K - NB - q0 - i + lane;
 #pragma unroll
-      for (int t = 0; t < R; t++) x[i][t] = (q0 + i < nt && (t + 1 < R || tail)) ? colp[i][32 * t] : T(0);
+      for (int t = 0; t < R; t++) x[i][t] = (q0 + i < nt && on(t)) ? colp[i][32 * t] : T(0);
     }
 #pragma unroll
     for (int k = 0; k < NB; k++) {
@@ -431,7 +432,7 @@ k_factor_panel(const FactorJob* __restrict__ jobs, T* __restrict__ B, T* __restr
     for (int i = 0; i < NC; i++)
 #pragma unroll
       for (int t = 0; t < R; t++)
-        if (q0 + i < nt && (t + 1 < R || tail)) colp[i][32 * t] = x[i][t];
+        if (q0 + i < nt && on(t)) colp[i][32 * t] = x[i][t];
   };
   // (K < NB: the next panel reaches past the columns the current one touches,
   // into those of the newest group)

@@ -38,3 +38,39 @@ def test_window_apply_matches_oracle(n, K, P, fact, dtype):
     s.precond(torch.tensor(v, device="cuda"), z)
     z, zo = z.cpu().numpy(), o.apply(v)
     assert np.linalg.norm(z - zo) / np.linalg.norm(zo) <= TOL[dtype]
+
+
+def uneven_band(n, widths, seed):
+    """Diagonally dominant CSR whose half-bandwidth changes along the matrix
+    (sparse inside the band, its outermost diagonals kept)."""
+    rng = np.random.default_rng(seed)
+    rows, cols = [np.arange(n)], [np.arange(n)]
+    for i, k in enumerate(widths):
+        a, e = n * i // len(widths), n * (i + 1) // len(widths)
+        for d in {1, k} | set(rng.integers(1, k + 1, 4).tolist()):
+            r = np.arange(a, min(e, n - d))
+            rows += [r, r + d]
+            cols += [r + d, r]
+    key = np.unique(np.concatenate(rows) * np.int64(n) + np.concatenate(cols))
+    r, c = key // n, (key % n).astype(np.int32)
+    v = rng.uniform(-1.0, 1.0, r.size)
+    v[r == c] = 0.0
+    v[r == c] = 1.5 * np.bincount(r, weights=np.abs(v), minlength=n)
+    return np.concatenate([[0], np.cumsum(np.bincount(r, minlength=n))]).astype(np.int32), c, v
+
+
+@pytest.mark.parametrize("dtype", ["double", "float"])
+@pytest.mark.parametrize("n,widths,P", [(8003, (3, 60, 9, 33), 8), (6001, (70, 2), 6), (5003, (12, 90, 5), 9)])
+def test_partitions_of_uneven_width(n, widths, P, dtype):
+    rp, ci, v = uneven_band(n, widths, n)
+    s = sap.Solver(P, sap.Options(), prec=dtype)
+    s.setup(sap.CsrMatrix(rp, ci, v))
+    ks = s.getReorder("ks")
+    assert ks.max() >= 2 * max(ks.min(), 1) and s.blockLayout()[0] == 0
+    o = oracle.SparsePrecond(P, dtype=dtype)
+    assert o.setup(rp, ci, v) == 0
+    x = np.random.default_rng(1).standard_normal(n)
+    z = torch.empty(n, dtype=torch.float64, device="cuda")
+    s.precond(torch.tensor(x, device="cuda"), z)
+    z, zo = z.cpu().numpy(), o.apply(x)
+    assert np.linalg.norm(z - zo) / np.linalg.norm(zo) <= TOL[dtype]
