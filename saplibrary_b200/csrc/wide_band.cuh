@@ -239,55 +239,39 @@ __device__ __forceinline__ void tile_sub(T* C, int ld, const T acc[8]) {
       for (int j = 0; j < 2; j++) C[(g + 8 * i) * ld + 8 * h + 2 * t + j] -= acc[4 * h + 2 * i + j];
 }
 // One warp: LU of the 16 x 16 tile A in place (the first n pivots count for the
-// zero check); 1 / pivot to rinv.  Lane l holds row l % 16.  FAST: reciprocals
-// without a branch (rcp_fast); false, with nothing written, when one left its
-// range.
-template <bool FAST, typename T>
-__device__ __forceinline__ bool tile_lu_body(T* A, int ld, int n, int boost, int* zero_flag, T* rinv) {
+// zero check); 1 / pivot to rinv.  Lane l holds row l % 16.
+template <typename T>
+__device__ __forceinline__ void tile_lu(T* A, int ld, int n, int boost, int* zero_flag, T* rinv) {
   const unsigned full = 0xffffffffu;
   const int lane = threadIdx.x & 31, r = lane & 15;
-  T a[16], y[16];
+  T a[16];
 #pragma unroll
   for (int c = 0; c < 16; c++) a[c] = A[r * ld + c];
   T low = T(1);
-  bool bad = false;
 #pragma unroll
   for (int k = 0; k < 16; k++) {
     T p = __shfl_sync(full, a[k], k);
-    p = boost ? boost_pivot(p) : p;
-    low = !boost && k < n ? fmin(low, fabs(p)) : low;
-    if constexpr (FAST) {
-      bool ok;
-      y[k] = rcp_fast(p, ok);
-      bad |= !ok;
-    } else {
-      y[k] = T(1) / p;
-    }
-    const T l = r > k ? a[k] * y[k] : T(0);
+    if (boost) p = boost_pivot(p);
+    else if (k < n) low = fmin(low, fabs(p));
+    const T inv = T(1) / p;
+    if (lane == k) rinv[k] = inv;
+    const T l = r > k ? a[k] * inv : T(0);
 #pragma unroll
     for (int c = k + 1; c < 16; c++) a[c] = fma(-l, __shfl_sync(full, a[c], k), a[c]);
     a[k] = r > k ? l : (r == k ? p : a[k]);
   }
-  if (__any_sync(full, bad)) return false;
   if ((double)low < 1e-7 && lane == 0) atomicOr(zero_flag, 1);
+  if (lane < 16) {
 #pragma unroll
-  for (int c = 0; c < 16; c++) {
-    if (lane == 16) rinv[c] = y[c];
-    if (lane < 16) A[r * ld + c] = a[c];
+    for (int c = 0; c < 16; c++) A[r * ld + c] = a[c];
   }
-  return true;
 }
+// One warp: the LU in tile A replaced by L^-1 (strict lower part) and U^-1
+// (upper part).  Both come from one forward recurrence: lane c < 16 solves for
+// column c of L^-1 from row 0 down, lane 16 + c for column c of U^-1 from row
+// 15 up, which is the same with rows and columns reversed.
 template <typename T>
-__device__ __forceinline__ void tile_lu(T* A, int ld, int n, int boost, int* zero_flag, T* rinv) {
-  if (!tile_lu_body<true>(A, ld, n, boost, zero_flag, rinv)) tile_lu_body<false>(A, ld, n, boost, zero_flag, rinv);
-}
-// One warp: the LU in tile A (reciprocal pivots rinv) replaced by L^-1 (strict
-// lower part) and U^-1 (upper part).  Both come from one forward recurrence:
-// lane c < 16 solves for column c of L^-1 from row 0 down, lane 16 + c for
-// column c of U^-1 from row 15 up, which is the same with rows and columns
-// reversed.  FAST: quotients by div_rcp_fast, as in tile_lu_body.
-template <bool FAST, typename T>
-__device__ __forceinline__ bool tile_inverses_body(T* A, int ld, const T* rinv) {
+__device__ __forceinline__ void tile_inverses(T* A, int ld) {
   const unsigned full = 0xffffffffu;
   const int lane = threadIdx.x & 31, r = lane & 15;
   const bool up = lane >= 16;
@@ -296,33 +280,20 @@ __device__ __forceinline__ bool tile_inverses_body(T* A, int ld, const T* rinv) 
   for (int k = 0; k < 16; k++) b[k] = A[r * ld + (up ? 15 - k : k)];
   const int e = up ? 15 - r : r;  // the unit right-hand side
 #pragma unroll
-  for (int i = 0; i < 16; i++) x[i] = i == e ? T(1) : T(0);
-  bool bad = false;
+  for (int i = 0; i < 16; i++) {
+    const int src = up ? 31 - i : i;  // row i, or row 15 - i, of the factor
+    T v = i == e ? T(1) : T(0);
 #pragma unroll
-  for (int k = 0; k < 16; k++) {
-    const T d = __shfl_sync(full, b[k], up ? 31 - k : k);  // the pivot, for U
-    if constexpr (FAST) {
-      bool ok;
-      const T q = div_rcp_fast(x[k], d, rinv[15 - k], ok);
-      bad |= up && !ok;
-      x[k] = up ? q : x[k];
-    } else {
-      x[k] = up ? x[k] / d : x[k];
-    }
-#pragma unroll
-    for (int i = k + 1; i < 16; i++) x[i] = fma(-__shfl_sync(full, b[k], up ? 31 - i : i), x[k], x[i]);
+    for (int k = 0; k < i; k++) v = fma(-__shfl_sync(full, b[k], src), x[k], v);
+    const T d = __shfl_sync(full, b[i], src);
+    x[i] = v / (up ? d : T(1));
   }
-  if (__any_sync(full, bad)) return false;
+  __syncwarp();
 #pragma unroll
   for (int i = 0; i < 16; i++) {
     const int row = up ? 15 - i : i;
     if (up ? row <= r : row > r) A[row * ld + r] = x[i];
   }
-  return true;
-}
-template <typename T>
-__device__ __forceinline__ void tile_inverses(T* A, int ld, const T* rinv) {
-  if (!tile_inverses_body<true>(A, ld, rinv)) tile_inverses_body<false>(A, ld, rinv);
 }
 // One warp, 32 columns (lane's column at P, rows ld apart): P <- L^-1 P for the
 // unit lower triangle of tile A.
@@ -412,7 +383,7 @@ k_leaf(const T* __restrict__ M, int ldm, long long sm, T* __restrict__ Li, T* __
         tile_lu(tile(G, k + 1, k + 1), ld, n - 16 * (k + 1), boost, zero_flag, rinv[(k + 1) & 1]);
       }
     } else if (warp == nw - 1) {
-      tile_inverses(tile(G, k, k), ld, rinv[k & 1]);
+      tile_inverses(tile(G, k, k), ld);
     } else {
       for (int q = warp; q < m * m; q += nw - 2) trail(k + 1 + q / m, k + 1 + q % m);
     }
