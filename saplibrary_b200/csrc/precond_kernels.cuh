@@ -282,6 +282,32 @@ template <typename T, int NB>
 inline size_t factor_panel_smem(int R, int K, int dpf) {
   return (NB + (size_t)(K + NB * (1 + dpf)) * (2 * K + NB) + 2 * NB * 32 * R) * sizeof(T);
 }
+// One warp: the panel of nb columns (first slot s, rows 0 .. last) factored in
+// place in the ring with the division, pivot by pivot; L columns to lp.  Kept
+// out of the chain's code, which it follows rarely.
+template <typename T>
+__device__ __noinline__ void factor_panel_div(T* win, T* lp, int K, int SP, int W, int LR, int s, int nb, int last,
+                                              int do_boost) {
+  const int lane = threadIdx.x & 31;
+  auto at = [&](int c, int r) -> T& { return win[(s + c >= W ? s + c - W : s + c) * SP + K - c + r]; };
+  for (int k = 0; k < nb; k++) {
+    T p = at(k, k);
+    if (do_boost) p = boost_pivot(p);
+    __syncwarp();
+    if (lane == 0) at(k, k) = p;
+    for (int r = lane; r < LR; r += 32) {
+      T l = T(0);
+      if (r > k && r <= min(K + k, last)) {
+        l = at(k, r) / p;
+        at(k, r) = l;
+        for (int c = k + 1; c < nb; c++)
+          if (c - k <= K) at(c, r) -= l * at(c, k);
+      }
+      lp[k * LR + r] = l;
+    }
+    __syncwarp();
+  }
+}
 template <typename T, int NB, int R>
 __global__ void __launch_bounds__(512)
 k_factor_panel(const FactorJob* __restrict__ jobs, T* __restrict__ B, T* __restrict__ B2,
@@ -319,15 +345,12 @@ k_factor_panel(const FactorJob* __restrict__ jobs, T* __restrict__ B, T* __restr
   // warp 0: the panel of columns j .. j+nb-1 (first slot s) factored in registers
   auto factor = [&](int j, int s, int nb, T* lp) {
     T a[R][NB];
-    auto load_panel = [&]() {
 #pragma unroll
-      for (int c = 0; c < NB; c++) {
-        const T* colp = win + wrap(s + c) * SP + K - c + lane;  // row j + lane + 32 t
+    for (int c = 0; c < NB; c++) {
+      const T* colp = win + wrap(s + c) * SP + K - c + lane;  // row j + lane + 32 t
 #pragma unroll
-        for (int t = 0; t < R; t++) a[t][c] = (c < nb && on(t)) ? colp[32 * t] : T(0);
-      }
-    };
-    load_panel();
+      for (int t = 0; t < R; t++) a[t][c] = (c < nb && on(t)) ? colp[32 * t] : T(0);
+    }
     const int last = np - 1 - j;  // the panel's rows are 0 .. last
     // fast path of a full panel: each quotient from the pivot's reciprocal with
     // Markstein's correction (rcp_fast and div_rcp_fast, equal to the division
@@ -363,41 +386,15 @@ k_factor_panel(const FactorJob* __restrict__ jobs, T* __restrict__ B, T* __restr
     }
     if (__any_sync(0xffffffffu, bad)) {
       // a quotient left the range, or the last panel: with the division
-      load_panel();
-#pragma unroll 1
-      for (int k = 0; k < nb; k++) {
-        const int end = min(K + k, last);
-        T p = T(0);
+      factor_panel_div(win, lp, K, SP, W, LR, s, nb, last, do_boost);
+    } else {
 #pragma unroll
-        for (int c = 0; c < NB; c++)
-          if (c == k) p = __shfl_sync(0xffffffffu, a[0][c], k);
-        if (do_boost) p = boost_pivot(p);
-        T u[NB];
+      for (int c = 0; c < NB; c++) {
+        T* colp = win + wrap(s + c) * SP + K - c + lane;
 #pragma unroll
-        for (int c = 0; c < NB; c++) u[c] = __shfl_sync(0xffffffffu, a[0][c], k);
-#pragma unroll
-        for (int t = 0; t < R; t++) {
-          const bool in = (t > 0 || lane > k) && lane + 32 * t <= end;
-          T l = T(0);
-#pragma unroll
-          for (int c = 0; c < NB; c++)
-            if (c == k) l = a[t][c] / p;
-          l = in ? l : T(0);
-          lp[k * LR + lane + 32 * t] = l;
-#pragma unroll
-          for (int c = 0; c < NB; c++) {
-            if (c > k) a[t][c] -= l * u[c];
-            else if (c == k) a[t][c] = t == 0 && lane == k ? p : (in ? l : a[t][c]);
-          }
-        }
+        for (int t = 0; t < R; t++)
+          if (on(t)) colp[32 * t] = a[t][c];
       }
-    }
-#pragma unroll
-    for (int c = 0; c < NB; c++) {
-      T* colp = win + wrap(s + c) * SP + K - c + lane;
-#pragma unroll
-      for (int t = 0; t < R; t++)
-        if (c < nb && on(t)) colp[32 * t] = a[t][c];
     }
     if (!do_boost) {  // the pivots as used
       __syncwarp();
