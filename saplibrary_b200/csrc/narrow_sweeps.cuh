@@ -219,8 +219,9 @@ __global__ void k_pack(const PartDev* __restrict__ parts, const T* __restrict__ 
 }
 
 // The three passes of a chunked partition sweep (see precond_kernels.cuh), one
-// warp per chunk.  Apply of a 200,000-row half-bandwidth 64 FP32 band in 32
-// partitions: see k_win_scan.
+// warp (up to K = 16 half a warp) per chunk.  About 50 ns per row: 1,000,000
+// rows, K = 10, FP64, passes 1 / 2 / 3 65 / 140 / 66 us with a CTA per chunk and
+// a barrier per row, 51 / 105 / 51 us with a warp per chunk.
 // The chunk of this lane's window (past the last one: a sweep of no rows).
 template <int LW>
 __device__ __forceinline__ int win_chunk() {
@@ -322,7 +323,8 @@ inline int scan_threads(int K) {
 
 // Chunk transfer matrices (see k_transfer): a CTA's warps follow C unit
 // carries each through the chunk, sharing the staged coefficients; grid
-// (chunk, group of carries, solve).
+// (chunk, group of carries, solve).  200,000 rows, K = 50, FP64: 5.7 -> 0.6 ms
+// against one thread per carry with its window in shared memory.
 template <typename T, int R1, int C>
 __global__ void __launch_bounds__(512)
 k_win_transfer(const PartDev* __restrict__ parts, const ChunkDev* __restrict__ chunks,
@@ -364,7 +366,10 @@ k_win_transfer(const PartDev* __restrict__ parts, const ChunkDev* __restrict__ c
 // shuffles, no barrier but its own), above it the groups' sums meet in shared
 // memory.  What bounds it is the instructions of a step, not its arithmetic:
 // with runtime strides and a test per element a step took 912 cycles at K = 10,
-// 1,193 at K = 64 (FP32), 1,408 at K = 50 (FP64).
+// 1,193 at K = 64 (FP32), 1,408 at K = 50 (FP64); now 0.31 us at K = 10 and 0.54
+// us at K = 64 (1.15 and 3.2 us with every load in the chain).  At K = 50 in FP64
+// a batch is two chunks and its transfer sets the pace (0.83 us); a ring of six
+// single-chunk stages gained 8 % there and lost 35 % in FP32.
 template <typename T>
 __host__ __device__ inline size_t scan_pad(size_t values) {  // to a multiple of 16 bytes
   constexpr size_t per = 16 / sizeof(T);
@@ -552,7 +557,7 @@ k_win_spikes_luul(const PartDev* __restrict__ parts, const T* __restrict__ pkd, 
 // scratch, and the interface rows read back.  iface null: the constant band
 // (the bottom K rows of partition i, the top K rows of partition i+1, the
 // former through the corner alone).  A 60,013-row half-bandwidth 37 FP32
-// band in 16 partitions: 24.6 ms with one thread per column.
+// band in 16 partitions: 24.6 ms with one thread per column, 0.36 ms now.
 template <typename T, int R1, int C>
 __global__ void __launch_bounds__(256)
 k_win_spikes_lu(const PartDev* __restrict__ parts, const T* __restrict__ pkd, const T* __restrict__ pku,

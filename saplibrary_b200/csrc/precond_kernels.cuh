@@ -277,7 +277,10 @@ k_factor_smem(const FactorJob* __restrict__ jobs, T* __restrict__ B, T* __restri
 // no test, those outside its band being zeros of the padding (or, past the
 // partition's end, elements that meet zeros of Lp and stay as they are).
 // 200,000 rows, K = 50, P = 10, FP64: 15.1 ms with one phase after the other,
-// 10.4 ms with look-ahead and a test per element.
+// 10.4 ms with look-ahead and a test per element, 6.9 ms now (FP32, K = 20, P =
+// 64, 400,000 rows: 2.43 -> 1.29 ms); rows below the first 32 on further warps
+// behind a second barrier (11.5 ms) and one rolled pivot step (9.9 ms) were
+// slower.
 template <typename T, int NB>
 inline size_t factor_panel_smem(int R, int K, int dpf) {
   return (NB + (size_t)(K + NB * (1 + dpf)) * (2 * K + NB) + 2 * NB * 32 * R) * sizeof(T);

@@ -143,7 +143,9 @@ __global__ void k_sub_fill(T* __restrict__ dst, int ldd, long long sd, int m, in
 //     U22^-1), all pairs and both triangles at once, in place of L21 and U12.
 // What bounds it is this chain of phases in one CTA per partition; larger
 // leaves replace whole levels of the recursion, whose products cost a launch
-// each (about 5 us, six on the chain of every level).
+// each (about 5 us, six on the chain of every level).  128 and 96 rows, 32
+// partitions: 47 us, against some 120 us for 32-row leaves (12 us each) and the
+// products of the two levels above them; 62 us with the inverses on the chain.
 //
 // tc: products between tiles of different 32-blocks run on the tensor cores
 // in TF32 (mma.sync, FP32 accumulation), like the products of the recursion
@@ -798,7 +800,7 @@ __global__ void __launch_bounds__(kGemvWarps * 32, 3) k_sweep(const MT* __restri
 // With blocks of a few hundred rows a step of the sweep moves some 100 KB per
 // CTA, so what bounds the schedules above is the latency of a step: the first
 // loads after each barrier, the partial sums and the barrier in global memory
-// (10.4 us per step at 448-row blocks, 32 partitions).  Here every CTA keeps
+// (10.4 us per step at 448-row blocks, 32 partitions; 2.6 us here).  Here every CTA keeps
 // its share of the next step's factor block on the way into registers while
 // the current step's sums are exchanged: the loads do not depend on the chain.
 // Columns go round the 16 C warps of the cluster (column c to warp c mod 16 C),
