@@ -906,9 +906,14 @@ k_sweep_cluster(const MT* __restrict__ Li, const MT* __restrict__ Ui, const MT* 
   const std::true_type LO{};
   const std::false_type UP{};
   static_assert(ROWS <= kGemvWarps * 32, "one row per thread");
+  // another CTA's shared memory may be written only once that CTA runs: all
+  // have arrived before the first exchange, the first block's loads meanwhile
+  // in flight
+  cluster.barrier_arrive();
   load(LO, Li + bd * BB, scaled ? csL + bd * bs : nullptr, 0, bs, 0, bs);
   if (tid < bs) xs[tid] = xp[tid];
   __syncthreads();
+  cluster.barrier_wait();
   for (int i = 0; i < nb; i++) {  // y_i = L_ii^-1 (x_i - L_{i,i-1} y_{i-1})
     const bool more = i + 1 < nb;
     T cv = T(0);

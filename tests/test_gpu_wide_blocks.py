@@ -45,6 +45,30 @@ def test_block_path_apply_matches_oracle(prec, n, K, P):
         s.setup(sap.BandedMatrix.from_array(band, n, K))
 
 
+@pytest.mark.parametrize("prec,K", [("float", 157), ("double", 109)])
+def test_cluster_sweep_of_single_block_rows(prec, K, monkeypatch):
+    # one block per partition: the first exchange between the CTAs of a cluster
+    # comes right after the launch, and more clusters than the chip holds start
+    # in waves; every application gives the same bits
+    bs = {"float": 448, "double": 320}[prec]
+    P = 120
+    n = P * bs - 7
+    monkeypatch.setenv("SAPB_BLOCK_SIZE", str(bs))
+    band = sap.generate_band_host(n, K, 1.0, 1, seed=K)
+    _, s = setup(n, K, P, prec, band)
+    assert s.blockLayout()[:2] == (bs, 1)
+    o = oracle.Precond(P, fact=sap.LU_UL, dtype=prec)
+    assert o.setup_banded(band, n, K) == 0
+    v = np.random.default_rng(K).standard_normal(n)
+    vd, z = torch.tensor(v, device="cuda"), torch.empty(n, dtype=torch.float64, device="cuda")
+    s.precond(vd, z)
+    first, zo = z.cpu().numpy(), o.apply(v)
+    assert np.linalg.norm(first - zo) / np.linalg.norm(zo) <= TOL[prec]
+    for _ in range(50):
+        s.precond(vd, z)
+        assert np.array_equal(z.cpu().numpy(), first)
+
+
 @pytest.mark.parametrize("prec", ["tf32", "tf32_f16"])
 @pytest.mark.parametrize("n,K,P", [(5003, 160, 2), (20011, 200, 19), (9001, 300, 3), (9007, 447, 2), (12011, 460, 3)])
 def test_tf32_blocks_solve(prec, n, K, P):
