@@ -694,6 +694,9 @@ class WideBand {
         // its diagonal) and, on the second lane, L_{i+1,i} = F_i U_ii^-1
         // (upper times upper); D is free again as the second lane's scratch
         SAPB_PROF("wb_offdiag", st);
+        // the corners are copied out before they are written again (a block of
+        // one leaf has no join of its own in rec)
+        if (ahead) lu.join();
         lu.fork();
         lu.prod_LL(kc, T(1), Li.at(c0, c0), Ec(i), ahead ? Cu : Wm);
         if (!ahead) lu.copy(Wm, Ec(i), kc, kc);

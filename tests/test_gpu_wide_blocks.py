@@ -45,6 +45,30 @@ def test_block_path_apply_matches_oracle(prec, n, K, P):
         s.setup(sap.BandedMatrix.from_array(band, n, K))
 
 
+@pytest.mark.parametrize("prec,n,K,P", [("double", 9001, 20, 3), ("double", 20011, 50, 4), ("double", 24001, 96, 40),
+                                        ("float", 9001, 32, 2), ("float", 20011, 70, 40), ("float", 30011, 128, 3)])
+def test_blocks_of_one_leaf(prec, n, K, P, monkeypatch):
+    # many block rows whose factorisation is one leaf, without a recursion whose
+    # joins would order the copies of one row's corners before the next row's
+    # products: direct, captured and replayed factorisations give the same bits
+    monkeypatch.setenv("SAPB_WIDE_MIN_K", "16")
+    band = sap.generate_band_host(n, K, 1.0, 1, seed=n + K)
+    A, s = setup(n, K, P, prec, band)
+    bs, nb, _ = s.blockLayout()
+    assert bs <= (96 if prec == "double" else 128) and nb > 5
+    o = oracle.Precond(P, fact=sap.LU_UL, dtype=prec)
+    assert o.setup_banded(band, n, K) == 0
+    v = np.random.default_rng(K).standard_normal(n)
+    z = torch.empty(n, dtype=torch.float64, device="cuda")
+    zo, first = o.apply(v), None
+    for _ in range(8):
+        s.precond(torch.tensor(v, device="cuda"), z)
+        first = z.cpu().numpy() if first is None else first
+        assert np.linalg.norm(first - zo) / np.linalg.norm(zo) <= TOL[prec]
+        assert np.array_equal(z.cpu().numpy(), first)
+        s.setup(A)
+
+
 @pytest.mark.parametrize("prec,K", [("float", 157), ("double", 109)])
 def test_cluster_sweep_of_single_block_rows(prec, K, monkeypatch):
     # one block per partition: the first exchange between the CTAs of a cluster
