@@ -151,6 +151,26 @@ class DevicePool {
   size_t free_bytes_ = 0;
 };
 
+// Lets a kernel take `bytes` of dynamic shared memory on the current device.
+// The limit belongs to the kernel, not to a solver: one kernel serves several
+// widths and lengths, from any thread, so it is only ever raised.
+inline void allow_smem_of(const void* kernel, size_t bytes) {
+  if (bytes <= 40 * 1024) return;  // allowed by default, beside a kernel's static arrays
+  static std::mutex mu;
+  static std::map<std::pair<int, const void*>, size_t> limit;
+  int dev = 0;
+  SAPB_CUDA(cudaGetDevice(&dev));
+  std::lock_guard<std::mutex> lk(mu);
+  size_t& l = limit[{dev, kernel}];
+  if (bytes <= l) return;
+  SAPB_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
+  l = bytes;
+}
+template <class... A>
+inline void allow_smem(void (*kernel)(A...), size_t bytes) {
+  allow_smem_of(reinterpret_cast<const void*>(kernel), bytes);
+}
+
 // Owning device buffer, its memory from the pool.
 template <typename T>
 class DBuf {

@@ -913,11 +913,6 @@ class PrecondT : public PrecBase {
     if (win_lanes(k) == 16) return f(integral_constant<int, win_slots(16, 16)>{}, integral_constant<int, 16>{});
     by_window(k, [&](auto R1) { f(R1, integral_constant<int, 32>{}); });
   }
-  template <class Kern>
-  static void allow_smem(Kern kern, size_t bytes) {
-    if (bytes > 48 * 1024)
-      SAPB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
-  }
   // columns per warp of the spike sweeps, warps per CTA, CTAs per tip
   static constexpr int kSpikeCols = 1;
   static int spike_warps(int k) { return std::min(8, (k + kSpikeCols - 1) / kSpikeCols); }
@@ -1003,7 +998,7 @@ class PrecondT : public PrecBase {
       // the chain's warp and three more for the next panel, four trailing columns per other warp
       const int nt = 32 * std::min(16, std::max(5, 1 + (Kmax - NBP + 3) / 4));
       auto launch = [&](auto kern) {
-        SAPB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)need(dpf)));
+        allow_smem(kern, need(dpf));
         kern<<<(int)jobs.size(), nt, need(dpf), st>>>(jobs_d.get(), B.get(), B2.get(), boost ? 1 : 0, flag.get(), dpf);
       };
       if constexpr (NBP == 8) {
@@ -1032,7 +1027,7 @@ class PrecondT : public PrecBase {
     if (panel) {
       // launched above
     } else if (smem <= 200 * 1024) {
-      SAPB_CUDA(cudaFuncSetAttribute(k_factor_smem<T, D>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+      allow_smem(k_factor_smem<T, D>, smem);
       SAPB_PROF("factor", st);
       k_factor_smem<T, D><<<(int)jobs.size(), NT, smem, st>>>(jobs_d.get(), B.get(), B2.get(), boost ? 1 : 0,
                                                              flag.get(), G);
@@ -1116,7 +1111,7 @@ class PrecondT : public PrecBase {
       gring.alloc((size_t)nch * maxK * tthreads);
       tsmem = 0;
     } else {
-      SAPB_CUDA(cudaFuncSetAttribute(k_transfer<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)std::max<size_t>(tsmem, 1024)));
+      allow_smem(k_transfer<T>, std::max<size_t>(tsmem, 1024));
     }
     SAPB_PROF("transfer", st);
     k_transfer<T><<<nch, tthreads, tsmem, st>>>(parts_d.get(), chunks_d.get(), toff_d.get(), B.get(), T1.get(), 1, gring.get(), first1_d.get());
@@ -1125,9 +1120,9 @@ class PrecondT : public PrecBase {
     SAPB_LAUNCHED();
     size_t s1 = (size_t)(maxK + maxChunk) * sizeof(T);
     if (2 * s1 > 220 * 1024) throw Error(SAP_ERR_UNSUPPORTED, "sweep chunk does not fit in shared memory");
-    SAPB_CUDA(cudaFuncSetAttribute(k_pass2<T, 16>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(2 * s1)));
-    SAPB_CUDA(cudaFuncSetAttribute(k_pass1<T, 16>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)s1));
-    SAPB_CUDA(cudaFuncSetAttribute(k_pass3<T, 16>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)s1));
+    allow_smem(k_pass2<T, 16>, 2 * s1);
+    allow_smem(k_pass1<T, 16>, s1);
+    allow_smem(k_pass3<T, 16>, s1);
     SAPB_CUDA(cudaStreamSynchronize(st));
     t_assembly += ms_since(t0);
   }

@@ -504,8 +504,7 @@ class WideBand {
       gemm_err.zero(st);
     }
     if (tc_on()) umma::prepare();  // kernel attributes, before any capture
-    SAPB_CUDA(cudaFuncSetAttribute(k_leaf<T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                   (int)leaf_smem<T>(leaf_max<T>)));
+    allow_smem(k_leaf<T>, leaf_smem<T>(leaf_max<T>));
     int maxsz = 0;
     for (int v : psize) maxsz = std::max(maxsz, v);
     nb = std::max(1, (maxsz + bs - 1) / bs);
@@ -872,7 +871,7 @@ class WideBand {
     constexpr int W = kGemvWarps * C, JM = (kClusterMaxBs + W - 1) / W, NT = (kClusterMaxBs + 32 * V - 1) / (32 * V);
     auto kern = k_sweep_cluster<T, V, MT, C, JM, NT>;
     const size_t smem = (size_t)(kGemvWarps + 2 * C + 1) * 32 * V * NT * sizeof(T);
-    SAPB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    allow_smem(kern, smem);
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(P * C);
     cfg.blockDim = dim3(kGemvWarps * 32);

@@ -74,3 +74,42 @@ def test_partitions_of_uneven_width(n, widths, P, dtype):
     s.precond(torch.tensor(x, device="cuda"), z)
     z, zo = z.cpu().numpy(), o.apply(x)
     assert np.linalg.norm(z - zo) / np.linalg.norm(zo) <= TOL[dtype]
+
+
+def band_solver(n, K, P, dtype):
+    band = sap.generate_band_host(n, K, 1.0, 1, seed=n + K)
+    s = sap.Solver(P, sap.Options(performReorder=False, variableBandwidth=False, applyScaling=False,
+                                  factMethod=sap.LU_UL), prec=dtype)
+    s.setup(sap.BandedMatrix.from_array(band, n, K))
+    return s
+
+
+def band_apply(s, v):
+    z = torch.empty(v.size, dtype=torch.float64, device="cuda")
+    s.precond(torch.tensor(v, device="cuda"), z)
+    return z.cpu().numpy()
+
+
+# pairs that share a kernel and need different amounts of shared memory: the
+# scan's width classes (9..16, 33..64, 65..128) and batch lengths, the reduced
+# systems, the panel kernel's row counts
+@pytest.mark.parametrize("dtype,one,two", [
+    ("double", (200003, 16, 2), (20011, 10, 2)), ("double", (200003, 16, 2), (2003, 16, 2)),
+    ("double", (90001, 60, 4), (9001, 40, 4)), ("double", (60013, 107, 3), (20011, 90, 3)),
+    ("float", (60013, 120, 2), (20011, 70, 4)), ("float", (60013, 155, 3), (20021, 129, 3)),
+])
+def test_two_live_solvers(dtype, one, two):
+    for first, second in ((one, two), (two, one)):
+        n, K, P = first
+        s1 = band_solver(n, K, P, dtype)
+        v = np.random.default_rng(K).standard_normal(n)
+        z = band_apply(s1, v)
+        s2 = band_solver(*second, dtype)
+        w = np.random.default_rng(second[1]).standard_normal(second[0])
+        z2 = band_apply(s2, w)
+        assert np.array_equal(band_apply(s1, v), z)
+        assert np.array_equal(band_apply(s2, w), z2)
+        o = oracle.Precond(P, fact=sap.LU_UL, dtype=dtype)
+        assert o.setup_banded(sap.generate_band_host(n, K, 1.0, 1, seed=n + K), n, K) == 0
+        zo = o.apply(v)
+        assert np.linalg.norm(z - zo) / np.linalg.norm(zo) <= TOL[dtype]
