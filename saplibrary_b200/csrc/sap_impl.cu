@@ -2046,6 +2046,9 @@ int sap_banded_create(int n, int k, const double* data, int memspace, sap_banded
     h->b.A.alloc(cnt);
     SAPB_CUDA(cudaMemcpy(h->b.A.get(), data, cnt * sizeof(double),
                          memspace == SAP_DEVICE ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice));
+    // (a copy on the device returns before it is done, and the solvers' streams
+    // do not wait for the default one)
+    SAPB_CUDA(cudaStreamSynchronize(nullptr));
     *out = h.release();
   });
 }
@@ -2059,6 +2062,7 @@ int sap_banded_generate(int n, int k, double d, int dist, uint64_t seed, sap_ban
     m->b.n = n; m->b.K = k;
     m->b.A.alloc(h.size());
     SAPB_CUDA(cudaMemcpy(m->b.A.get(), h.data(), h.size() * sizeof(double), cudaMemcpyHostToDevice));
+    SAPB_CUDA(cudaStreamSynchronize(nullptr));
     *out = m.release();
   });
 }

@@ -221,3 +221,25 @@ def test_blas_dots_match_numpy(n):
     torch.cuda.synchronize()
     ref = [float(np.dot(x.cpu().numpy(), y.cpu().numpy())) for x, y in zip(xs, ys)]
     assert np.allclose(out.cpu().numpy(), ref, rtol=1e-12, atol=1e-12)
+
+
+def test_band_copied_on_the_device_is_complete_when_it_is_set_up():
+    # the copy of 6 GB outlasts the call that starts it, and the setup on the
+    # solver's own stream follows at once
+    n, K = 4_000_000, 96
+    g = torch.Generator(device="cuda")
+    g.manual_seed(1)
+    band = torch.empty(n, 2 * K + 1, dtype=torch.float64, device="cuda").uniform_(-1.0, 1.0, generator=g)
+    band[:, K] = 2 * K + 1
+    v = torch.ones(n, dtype=torch.float64, device="cuda")
+    z = []
+    for wait in (False, True):
+        torch.cuda.synchronize()
+        s = sap.Solver(148, banded_opts(ptype=sap.Block), prec="float")
+        A = sap.BandedMatrix.from_array(band, n, K)
+        if wait:
+            torch.cuda.synchronize()
+        s.setup(A)
+        z.append(torch.empty_like(v))
+        s.precond(v, z[-1])
+    assert bool(torch.isfinite(z[0]).all()) and torch.equal(z[0], z[1])
