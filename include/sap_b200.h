@@ -297,6 +297,11 @@ void* sap_solver_stream(const sap_solver* s);
  * used), and the bytes of one factor value read by the apply's sweeps (8, 4,
  * or 2 for the FP16 copies of SAP_PREC_TF32_F16). */
 int sap_solver_block_layout(const sap_solver* s, int* block_size, int* blocks_per_partition, int* value_bytes);
+/* Returns the memory that the library keeps for reuse to the driver: the device
+ * blocks of destroyed solvers and finished setups (at most 2 GiB) and the
+ * page-locked host blocks of destroyed CSR matrices (at most 2 GiB).  Live
+ * handles keep theirs.  May be called at any time from any thread. */
+int sap_trim_memory(void);
 /* Number of this library's own kernels enqueued since load (all handles). */
 int64_t sap_kernel_launch_count(void);
 /* Number of cuBLAS calls (batched GEMMs of the wide-band path) since load. */

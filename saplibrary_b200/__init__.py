@@ -87,6 +87,7 @@ _vp, _i, _d = ctypes.c_void_p, ctypes.c_int, ctypes.c_double
 _pp = ctypes.POINTER(ctypes.c_void_p)
 _sig = {
     "sap_last_error": (ctypes.c_char_p, []),
+    "sap_trim_memory": (_i, []),
     "sap_kernel_launch_count": (ctypes.c_int64, []),
     "sap_library_call_count": (ctypes.c_int64, []),
     "sap_mm_read_csr": (_i, [ctypes.c_char_p, ctypes.POINTER(_i), ctypes.POINTER(_i), ctypes.POINTER(ctypes.c_int64),
@@ -169,6 +170,12 @@ def _ptr(a):
             raise ValueError("tensor must be contiguous")
         return ctypes.c_void_p(a.data_ptr()), DEVICE
     raise TypeError("expected a numpy array or a CUDA tensor")
+
+
+def trim_memory() -> None:
+    """Return the memory kept for reuse (device blocks of destroyed solvers,
+    page-locked host blocks of destroyed matrices) to the driver."""
+    _check(_lib.sap_trim_memory())
 
 
 def kernel_launch_count() -> int:

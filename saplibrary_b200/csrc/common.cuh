@@ -4,6 +4,7 @@
 
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <atomic>
 #include <cstdlib>
 #include <map>
@@ -60,19 +61,73 @@ struct ProfScope {
 };
 #define SAPB_PROF(name, stream) ::sapb::ProfScope _sapb_prof_scope(name, stream)
 
+// The streams that ever touch a group of device buffers (a solver's own ones).
+// The buffers a thread allocates inside a HomeScope belong to its home, those
+// allocated outside of one have none.
+struct StreamHome {
+  std::vector<cudaStream_t> streams;
+  void add(cudaStream_t s) { streams.push_back(s); }
+  void remove(cudaStream_t s) { streams.erase(std::remove(streams.begin(), streams.end(), s), streams.end()); }
+  // all work on the streams is done; false when that cannot be told
+  bool wait() const {
+    bool ok = true;
+    for (cudaStream_t s : streams) ok = cudaStreamSynchronize(s) == cudaSuccess && ok;
+    if (!ok) (void)cudaGetLastError();  // nobody's next launch failed
+    return ok;
+  }
+};
+// A home without streams: for buffers that only calls touch which wait for their
+// work before they return.
+inline const std::shared_ptr<StreamHome>& idle_home() {
+  static const auto* h = new std::shared_ptr<StreamHome>(std::make_shared<StreamHome>());
+  return *h;
+}
+class HomeScope {
+ public:
+  explicit HomeScope(std::shared_ptr<StreamHome> h) : old_(std::move(h)) { std::swap(old_, current()); }
+  ~HomeScope() { std::swap(old_, current()); }
+  HomeScope(const HomeScope&) = delete;
+  HomeScope& operator=(const HomeScope&) = delete;
+  static std::shared_ptr<StreamHome>& current() {
+    static thread_local std::shared_ptr<StreamHome> h;
+    return h;
+  }
+
+ private:
+  std::shared_ptr<StreamHome> old_;
+};
+
 // Device blocks kept for reuse (DBuf): cudaMalloc and cudaFree cost some 0.2 ms
 // each whatever the size, and a setup, or a solver made for one batch of
 // systems, makes dozens of them (24 systems in four stacks: 568 of each, 0.2 s
 // of a 0.21 s call).  A block is taken by the next request on its device that
-// fills at least half of it.  give() waits for the device, as cudaFree does,
-// so a block in the pool has no work of any stream left on it.  The pool holds
-// at most kMaxFreeBytes (1 % of the memory), larger blocks go straight back,
-// and an allocation that fails empties it and tries again.
+// fills at least half of it.  Only blocks with a home are kept: give() waits for
+// the home's streams, so that a kept block has no work left on it, and never for
+// the device, which would break a graph capture open in another thread.  The
+// pool holds at most kMaxFreeBytes (1 % of the memory), larger blocks go
+// straight back, an allocation that fails empties it and tries again, and
+// sap_trim_memory() empties it on request.
 class DevicePool {
  public:
   static DevicePool& instance() {
     static DevicePool* pool = new DevicePool();  // no driver call during static teardown
     return *pool;
+  }
+  // an allocation that is not kept
+  void* take_plain(size_t bytes) {
+    void* p = nullptr;
+    cudaError_t e = cudaMalloc(&p, bytes);
+    if (e == cudaErrorMemoryAllocation) {
+      (void)cudaGetLastError();  // not sticky
+      trim();
+      e = cudaMalloc(&p, bytes);
+      if (e != cudaSuccess) (void)cudaGetLastError();
+    }
+    SAPB_CUDA(e);
+    return p;
+  }
+  static void give_plain(void* p) {
+    if (p && cudaFree(p) != cudaSuccess) (void)cudaGetLastError();
   }
   void* take(size_t bytes) {
     bytes = rounded(bytes);
@@ -89,55 +144,54 @@ class DevicePool {
         return p;
       }
     }
-    void* p = nullptr;
-    cudaError_t e = cudaMalloc(&p, bytes);
-    if (e == cudaErrorMemoryAllocation) {
-      (void)cudaGetLastError();  // not sticky
-      trim();
-      e = cudaMalloc(&p, bytes);
-    }
-    SAPB_CUDA(e);
+    void* p = take_plain(bytes);
     std::lock_guard<std::mutex> lk(mu_);
     used_[p] = {dev, bytes};
     return p;
   }
-  void give(void* p) {
+  void give(void* p, const StreamHome& home) {
     if (!p) return;
     Key k;
     {
       std::lock_guard<std::mutex> lk(mu_);
       auto it = used_.find(p);
-      if (it == used_.end()) return;
       k = it->second;
       used_.erase(it);
     }
-    int dev = -1;
-    const bool here = cudaGetDevice(&dev) == cudaSuccess && dev == k.first;
-    // (work on a block of another device cannot be waited for from here)
-    if (here && k.second <= kMaxFreeBytes / 2 && cudaDeviceSynchronize() == cudaSuccess) {
-      std::lock_guard<std::mutex> lk(mu_);
-      if (free_bytes_ + k.second <= kMaxFreeBytes) {
+    bool kept = false;
+    if (k.second <= kMaxFreeBytes / 2 && home.wait()) try {
+        std::lock_guard<std::mutex> lk(mu_);
         free_.emplace(k, p);
         free_bytes_ += k.second;
-        return;
+        kept = true;
+      } catch (const std::bad_alloc&) {  // (give() runs in destructors)
       }
-    }
-    cudaFree(p);
+    if (kept) shrink(kMaxFreeBytes);
+    else give_plain(p);
   }
   // every kept block back to the driver
-  void trim() {
-    std::multimap<Key, void*> all;
-    {
-      std::lock_guard<std::mutex> lk(mu_);
-      all.swap(free_);
-      free_bytes_ = 0;
-    }
-    for (auto& b : all) cudaFree(b.second);
-  }
+  void trim() { shrink(0); }
 
  private:
   using Key = std::pair<int, size_t>;  // device, bytes
   static constexpr size_t kMaxFreeBytes = size_t(1) << 31;
+  // kept blocks beyond `bytes` back to the driver, the largest first: a small
+  // one saves as much time as a large one
+  void shrink(size_t bytes) {
+    while (true) {
+      void* p;
+      {
+        std::lock_guard<std::mutex> lk(mu_);
+        if (free_bytes_ <= bytes || free_.empty()) return;
+        auto big = std::max_element(free_.begin(), free_.end(),
+                                    [](const auto& a, const auto& b) { return a.first.second < b.first.second; });
+        p = big->second;
+        free_bytes_ -= big->first.second;
+        free_.erase(big);
+      }
+      give_plain(p);
+    }
+  }
   // small blocks in powers of two, others in steps of 1 MB
   static size_t rounded(size_t b) {
     if (b > (size_t(1) << 20)) return (b + (size_t(1) << 20) - 1) >> 20 << 20;
@@ -171,7 +225,8 @@ inline void allow_smem(void (*kernel)(A...), size_t bytes) {
   allow_smem_of(reinterpret_cast<const void*>(kernel), bytes);
 }
 
-// Owning device buffer, its memory from the pool.
+// Owning device buffer; its memory from the pool when it is allocated inside a
+// HomeScope.
 template <typename T>
 class DBuf {
  public:
@@ -186,7 +241,10 @@ class DBuf {
     if (n == n_ && p_) return;
     release();
     n_ = n;
-    if (n) p_ = static_cast<T*>(DevicePool::instance().take(n * sizeof(T)));
+    if (!n) return;
+    DevicePool& pool = DevicePool::instance();
+    home_ = HomeScope::current();
+    p_ = static_cast<T*>(home_ ? pool.take(n * sizeof(T)) : pool.take_plain(n * sizeof(T)));
   }
   // grow-only: at least n elements (a smaller request keeps the buffer)
   void ensure(size_t n) {
@@ -211,7 +269,9 @@ class DBuf {
     if (n_) SAPB_CUDA(cudaMemcpyAsync(h.data(), p_, n_ * sizeof(T), cudaMemcpyDeviceToHost, s));
   }
   void release() {
-    DevicePool::instance().give(p_);
+    if (home_) DevicePool::instance().give(p_, *home_);
+    else DevicePool::give_plain(p_);
+    home_.reset();
     p_ = nullptr;
     n_ = 0;
   }
@@ -219,9 +279,10 @@ class DBuf {
   size_t size() const { return n_; }
 
  private:
-  void swap(DBuf& o) { std::swap(p_, o.p_); std::swap(n_, o.n_); }
+  void swap(DBuf& o) { std::swap(p_, o.p_); std::swap(n_, o.n_); std::swap(home_, o.home_); }
   T* p_ = nullptr;
   size_t n_ = 0;
+  std::shared_ptr<StreamHome> home_;
 };
 
 // Allocator whose value construction leaves trivially constructible elements
@@ -301,15 +362,23 @@ class PinnedPool {
     free_.emplace(it->second, p);
     free_bytes_ += it->second;
     used_.erase(it);
-    while (free_bytes_ > kMaxFreeBytes && !free_.empty()) {
-      auto big = std::prev(free_.end());
-      free_bytes_ -= big->first;
-      cudaFreeHost(big->second);
-      free_.erase(big);
-    }
+    shrink(kMaxFreeBytes);
+  }
+  // every free block back to the driver
+  void trim() {
+    std::lock_guard<std::mutex> lk(mu_);
+    shrink(0);
   }
 
  private:
+  void shrink(size_t bytes) {
+    while (free_bytes_ > bytes && !free_.empty()) {
+      auto big = std::prev(free_.end());
+      free_bytes_ -= big->first;
+      if (cudaFreeHost(big->second) != cudaSuccess) (void)cudaGetLastError();
+      free_.erase(big);
+    }
+  }
   static constexpr size_t kMaxFreeBytes = size_t(1) << 31;
   std::mutex mu_;
   std::multimap<size_t, void*> free_;

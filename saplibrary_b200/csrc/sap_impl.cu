@@ -10,6 +10,7 @@
 #include <cmath>
 #include <cstdlib>
 #include <cstring>
+#include <exception>
 #include <limits>
 #include <memory>
 #include <mutex>
@@ -79,8 +80,7 @@ struct Csr {
   int n = 0, nnz = 0;
   // host copies (reordering runs on the host), page-locked blocks from a
   // pool: the uploads run at full speed and repeated copies reuse warm
-  // pages.  Declared before the device buffers, so that they go back to the
-  // pool only after those are freed (cudaFree waits for copies in flight).
+  // pages.  (sap_csr_create waits for the uploads.)
   PinnedHostVec<int> rp_h, ci_h;
   PinnedHostVec<double> v_h;
   DBuf<int> rp, ci;
@@ -120,6 +120,7 @@ struct Spmv {
                                                          x, y);
       SAPB_LAUNCHED();
     } else {
+      HomeScope none(nullptr);  // what the caller's code allocates is not the solver's
       fn(ctx, x, y, (void*)s);
     }
   }
@@ -1382,6 +1383,7 @@ class Solver {
   int P_req = 1;
   int prec_dtype = SAP_PREC_FLOAT;
   cudaStream_t st = nullptr;
+  std::shared_ptr<StreamHome> home = std::make_shared<StreamHome>();
   std::unique_ptr<PrecBase> pcp;
   PrecBase& pc() { return *pcp; }
   Monitor mon;
@@ -1409,6 +1411,8 @@ class Solver {
 
   Solver(int P, const sap_options& o, int dtype) : opts(o), P_req(P), prec_dtype(dtype) {
     SAPB_CUDA(cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking));
+    home->add(st);
+    HomeScope hs(home);
     if (dtype == SAP_PREC_DOUBLE) pcp = std::make_unique<PrecondT<double>>();
     else pcp = std::make_unique<PrecondT<float>>();
     pcp->tf32 = dtype == SAP_PREC_TF32 || dtype == SAP_PREC_TF32_F16;
@@ -1430,6 +1434,8 @@ class Solver {
     if (pinned) cudaFreeHost(pinned);
     if (st) {
       cudaStreamSynchronize(st);
+      pcp.reset();
+      home->remove(st);  // (the other buffers are idle)
       cudaStreamDestroy(st);
     }
   }
@@ -1983,6 +1989,19 @@ struct sap_spmv { Spmv op; cudaStream_t st = nullptr; };
     return SAP_ERR_CUDA;                                 \
   }
 
+// A call that runs a solver: its allocations belong to the solver, and where it
+// fails halfway, the work it has started is done before it returns (the caller's
+// vectors and matrices may be released then).
+struct SolverCall {
+  Solver& S;
+  HomeScope hs;
+  const int thrown = std::uncaught_exceptions();
+  explicit SolverCall(Solver& s) : S(s), hs(s.home) {}
+  ~SolverCall() {
+    if (std::uncaught_exceptions() > thrown) S.home->wait();
+  }
+};
+
 #define SAP_REQUIRE(cond, msg) \
   do { if (!(cond)) throw sapb::Error(SAP_ERR_INVALID_ARGUMENT, msg); } while (0)
 
@@ -1991,6 +2010,13 @@ extern "C" {
 const char* sap_last_error(void) { return g_last_error.c_str(); }
 int64_t sap_kernel_launch_count(void) { return g_launches.load(); }
 int64_t sap_library_call_count(void) { return g_lib_calls.load(); }
+
+int sap_trim_memory(void) {
+  SAP_TRY({
+    DevicePool::instance().trim();
+    PinnedPool::instance().trim();
+  });
+}
 
 int sap_profile_select(const char* name) {
   SAP_TRY({
@@ -2040,6 +2066,7 @@ int sap_options_default(sap_options* o) {
 int sap_banded_create(int n, int k, const double* data, int memspace, sap_banded** out) {
   SAP_TRY({
     SAP_REQUIRE(out && data && n > 0 && k >= 0 && k < n, "invalid banded matrix arguments");
+    HomeScope hs(idle_home());
     auto h = std::make_unique<sap_banded>();
     h->b.n = n; h->b.K = k;
     size_t cnt = (size_t)n * (2 * k + 1);
@@ -2058,6 +2085,7 @@ int sap_banded_generate(int n, int k, double d, int dist, uint64_t seed, sap_ban
     SAP_REQUIRE(out && n > 0 && k >= 0 && k < n && dist >= 0 && dist <= 2, "invalid generator arguments");
     std::vector<double> h((size_t)n * (2 * k + 1), 0.0);
     sapb::generate_band(n, k, d, dist, seed, h.data());
+    HomeScope hs(idle_home());
     auto m = std::make_unique<sap_banded>();
     m->b.n = n; m->b.K = k;
     m->b.A.alloc(h.size());
@@ -2080,6 +2108,7 @@ int sap_banded_copy_out(const sap_banded* A, double* dst, int memspace) {
     SAP_REQUIRE(A && dst, "null argument");
     SAPB_CUDA(cudaMemcpy(dst, A->b.A.get(), A->b.A.size() * sizeof(double),
                          memspace == SAP_DEVICE ? cudaMemcpyDeviceToDevice : cudaMemcpyDeviceToHost));
+    SAPB_CUDA(cudaStreamSynchronize(nullptr));  // the matrix may be released next
   });
 }
 
@@ -2096,6 +2125,7 @@ int sap_banded_destroy(sap_banded* A) { delete A; return SAP_OK; }
 int sap_csr_create(int n, int nnz, const int* rp, const int* ci, const double* v, int memspace, sap_csr** out) {
   SAP_TRY({
     SAP_REQUIRE(out && rp && ci && v && n > 0 && nnz >= 0, "invalid CSR arguments");
+    HomeScope hs(idle_home());
     auto h = std::make_unique<sap_csr>();
     h->c.n = n; h->c.nnz = nnz;
     h->c.rp_h.resize(n + 1); h->c.ci_h.resize(nnz); h->c.v_h.resize(nnz);
@@ -2129,7 +2159,7 @@ int sap_csr_create(int n, int nnz, const int* rp, const int* ci, const double* v
       h->c.nblk = (int)blk.size() - 1;
       h->c.blk.upload(blk, nullptr);
     }
-    SAPB_CUDA(cudaDeviceSynchronize());
+    SAPB_CUDA(cudaStreamSynchronize(nullptr));
     *out = h.release();
   });
 }
@@ -2273,6 +2303,7 @@ int sap_solver_setup_banded(sap_solver* h, const sap_banded* A) {
   SAP_TRY({
     SAP_REQUIRE(h && A, "null argument");
     Solver& S = *h->s;
+    SolverCall call(S);
     auto t0 = Clock::now();
     PrecBase& pc = S.pc();
     pc.reordered = false;
@@ -2289,6 +2320,7 @@ int sap_solver_setup_csr(sap_solver* h, const sap_csr* A) {
   SAP_TRY({
     SAP_REQUIRE(h && A, "null argument");
     Solver& S = *h->s;
+    SolverCall call(S);
     auto t0 = Clock::now();
     PrecBase& pc = S.pc();
     if (!S.opts.performReorder) {
@@ -2313,6 +2345,7 @@ int sap_solver_update(sap_solver* h, const double* entries, int64_t nnz, int mem
   SAP_TRY({
     SAP_REQUIRE(h && entries, "null argument");
     Solver& S = *h->s;
+    SolverCall call(S);
     if (!S.setup_done) throw Error(SAP_ILLEGAL_UPDATE, "Illegal call to update() before setup().");
     if (!S.opts.trackReordering)
       throw Error(SAP_ILLEGAL_UPDATE, "Illegal call to update() with reordering tracking disabled.");
@@ -2344,6 +2377,7 @@ int sap_solver_solve(sap_solver* h, sap_spmv* spmv, const double* b, double* x, 
   SAP_TRY({
     SAP_REQUIRE(h && spmv && b && x, "null argument");
     Solver& S = *h->s;
+    SolverCall call(S);
     if (!S.setup_done) throw Error(SAP_ILLEGAL_SOLVE, "Illegal call to solve() before setup().");
     SAP_REQUIRE(spmv->op.n == S.n, "operator size differs from the preconditioner's");
     int L = 0;
@@ -2380,6 +2414,7 @@ int sap_precond_apply(sap_solver* h, const double* v, double* z) {
   SAP_TRY({
     SAP_REQUIRE(h && v && z, "null argument");
     Solver& S = *h->s;
+    SolverCall call(S);
     if (!S.setup_done) throw Error(SAP_ILLEGAL_SOLVE, "preconditioner used before setup().");
     S.pc().apply(v, z);
     SAPB_CUDA(cudaStreamSynchronize(S.st));
@@ -2428,6 +2463,18 @@ int sap_batch_banded_solve(int m, const int* n, const int* k, const double* cons
       SAP_REQUIRE(ntot < 2147483647LL, "stacked system too large");
       const size_t W = 2 * (size_t)K + 1;
       std::vector<double> bb((size_t)ntot), xx((size_t)ntot, 0.0);
+      sap_options o = *opts;
+      o.absTol = opts->relTol;
+      o.relTol = 0;
+      o.performReorder = 0;
+      o.variableBandwidth = 0;
+      o.applyScaling = 0;
+      sap_solver* sv_new = nullptr;
+      int rc = sap_solver_create(Ptot, &o, prec_dtype, &sv_new);
+      if (rc != SAP_OK) return rc;
+      std::unique_ptr<sap_solver> sv(sv_new);
+      Solver& S = *sv->s;
+      HomeScope hs(S.home);  // the stack is used on the solver's streams only
       // the stack on the device: every system copied into its rows, then
       // scaled, with the entries outside its own columns dropped so that no
       // system reaches into its neighbours
@@ -2438,39 +2485,30 @@ int sap_batch_banded_solve(int m, const int* n, const int* k, const double* cons
       for (size_t q = g0; q < g1; q++) {
         const int i = order[q];
         const long long off = seg[q - g0];
-        SAPB_CUDA(cudaMemcpy(Ah->b.A.get() + (size_t)off * W, bands[i], sizeof(double) * (size_t)n[i] * W,
-                             cudaMemcpyHostToDevice));
-        k_stack_rows<<<grid_for((long long)n[i] * (long long)W, 256), 256>>>(Ah->b.A.get() + (size_t)off * W, n[i], K,
-                                                                             scale[q - g0]);
+        SAPB_CUDA(cudaMemcpyAsync(Ah->b.A.get() + (size_t)off * W, bands[i], sizeof(double) * (size_t)n[i] * W,
+                                  cudaMemcpyHostToDevice, S.st));
+        k_stack_rows<<<grid_for((long long)n[i] * (long long)W, 256), 256, 0, S.st>>>(
+            Ah->b.A.get() + (size_t)off * W, n[i], K, scale[q - g0]);
         SAPB_LAUNCHED();
         const double sc = scale[q - g0];
         for (int r = 0; r < n[i]; r++) bb[off + r] = b[i][r] * sc;
       }
-      SAPB_CUDA(cudaDeviceSynchronize());
-      sap_options o = *opts;
-      o.absTol = opts->relTol;
-      o.relTol = 0;
-      o.performReorder = 0;
-      o.variableBandwidth = 0;
-      o.applyScaling = 0;
-      sap_banded* A = Ah.release();
-      sap_spmv* op = nullptr;
-      sap_solver* sv = nullptr;
-      int rc = sap_spmv_banded_create(A, &op);
-      if (rc == SAP_OK) rc = sap_solver_create(Ptot, &o, prec_dtype, &sv);
-      if (rc == SAP_OK) rc = sap_solver_setup_banded(sv, A);
+      sap_spmv op;
+      op.op.kind = 0;
+      op.op.band = &Ah->b;
+      op.op.n = (int)ntot;
+      rc = sap_solver_setup_banded(sv.get(), Ah.get());
       int conv = 0;
-      if (rc == SAP_OK) rc = sap_solver_solve(sv, op, bb.data(), xx.data(), SAP_HOST, &conv);
+      if (rc == SAP_OK) rc = sap_solver_solve(sv.get(), &op, bb.data(), xx.data(), SAP_HOST, &conv);
       if (rc == SAP_OK) {
         // per-system residual norms of the scaled stack = relative residuals
-        Solver& S = *sv->s;
         DBuf<double> xd, rd, sq;
         DBuf<long long> segd;
         xd.upload(xx, S.st);
         rd.alloc((size_t)ntot);
         sq.alloc(g1 - g0);
         segd.upload(seg, S.st);
-        op->op.apply(xd.get(), rd.get(), S.st);
+        op.op.apply(xd.get(), rd.get(), S.st);
         DBuf<double> bd;
         bd.upload(bb, S.st);
         k_axpby<<<grid_for(ntot, 256), 256, 0, S.st>>>((int)ntot, 1.0, bd.get(), -1.0, rd.get(), rd.get());
@@ -2488,9 +2526,6 @@ int sap_batch_banded_solve(int m, const int* n, const int* k, const double* cons
           std::memcpy(x[i], xx.data() + seg[q - g0], sizeof(double) * n[i]);
         }
       }
-      if (sv) sap_solver_destroy(sv);
-      if (op) sap_spmv_destroy(op);
-      if (A) sap_banded_destroy(A);
       if (rc != SAP_OK) return rc;
       g0 = g1;
     }

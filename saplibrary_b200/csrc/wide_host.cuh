@@ -306,9 +306,11 @@ class WideBand {
       if (x) cudaStreamSynchronize(x);
     if (h) cublasDestroy(h);
     if (h2) cublasDestroy(h2);
-    if (st2) cudaStreamDestroy(st2);
-    for (cudaStream_t x : st_more)
-      if (x) cudaStreamDestroy(x);
+    for (cudaStream_t x : {st2, st_more[0], st_more[1]}) {
+      if (!x) continue;
+      if (home) home->remove(x);
+      cudaStreamDestroy(x);
+    }
     if (ev_fork) cudaEventDestroy(ev_fork);
     if (ev_join) cudaEventDestroy(ev_join);
     if (ev_half) cudaEventDestroy(ev_half);
@@ -480,10 +482,13 @@ class WideBand {
     psize_h = psize;
     if (!h) cublas_check(cublasCreate(&h), "cublasCreate");
     if (!st2) {
+      home = HomeScope::current();  // the solver's buffers are used on these streams too
       SAPB_CUDA(cudaStreamCreateWithFlags(&st2, cudaStreamNonBlocking));
       SAPB_CUDA(cudaEventCreateWithFlags(&ev_fork, cudaEventDisableTiming));
       SAPB_CUDA(cudaEventCreateWithFlags(&ev_join, cudaEventDisableTiming));
       for (cudaStream_t& x : st_more) SAPB_CUDA(cudaStreamCreateWithFlags(&x, cudaStreamNonBlocking));
+      if (home)
+        for (cudaStream_t x : {st2, st_more[0], st_more[1]}) home->add(x);
       for (cudaEvent_t& e : ev_lane) SAPB_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
       SAPB_CUDA(cudaEventCreateWithFlags(&ev_half, cudaEventDisableTiming));
     }
@@ -722,6 +727,8 @@ class WideBand {
   DBuf<T> gws[kMaxLanes];          // column-split partial sums
   DBuf<unsigned> gctr[kMaxLanes];  // column-split arrival counters (zero between launches)
   cudaStream_t st2 = nullptr, st_more[kMaxLanes - 2] = {};
+  static_assert(kMaxLanes == 4, "two streams beside st and st2");
+  std::shared_ptr<StreamHome> home;
   cudaEvent_t ev_fork = nullptr, ev_join = nullptr, ev_lane[kMaxLanes] = {};
   cudaStream_t lane_stream(int lane) const { return lane == 0 ? st : (lane == 1 ? st2 : st_more[lane - 2]); }
   // CTAs one GEMV launch aims at through its column split (about 2.5 of the
