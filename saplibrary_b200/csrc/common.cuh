@@ -137,7 +137,7 @@ class DevicePool {
       std::lock_guard<std::mutex> lk(mu_);
       auto it = free_.lower_bound({dev, bytes});
       if (it != free_.end() && it->first.first == dev && it->first.second / 2 <= bytes) {
-        void* p = it->second;
+        void* p = it->second.p;
         used_[p] = it->first;
         free_bytes_ -= it->first.second;
         free_.erase(it);
@@ -161,7 +161,7 @@ class DevicePool {
     bool kept = false;
     if (k.second <= kMaxFreeBytes / 2 && home.wait()) try {
         std::lock_guard<std::mutex> lk(mu_);
-        free_.emplace(k, p);
+        free_.emplace(k, Block{p, given_++});
         free_bytes_ += k.second;
         kept = true;
       } catch (const std::bad_alloc&) {  // (give() runs in destructors)
@@ -175,19 +175,23 @@ class DevicePool {
  private:
   using Key = std::pair<int, size_t>;  // device, bytes
   static constexpr size_t kMaxFreeBytes = size_t(1) << 31;
-  // kept blocks beyond `bytes` back to the driver, the largest first: a small
-  // one saves as much time as a large one
+  struct Block {
+    void* p;
+    unsigned long long age;  // position in the order of give()
+  };
+  // kept blocks beyond `bytes` back to the driver, the longest unused first (they
+  // are left from other sizes; what a program uses again and again stays)
   void shrink(size_t bytes) {
     while (true) {
       void* p;
       {
         std::lock_guard<std::mutex> lk(mu_);
         if (free_bytes_ <= bytes || free_.empty()) return;
-        auto big = std::max_element(free_.begin(), free_.end(),
-                                    [](const auto& a, const auto& b) { return a.first.second < b.first.second; });
-        p = big->second;
-        free_bytes_ -= big->first.second;
-        free_.erase(big);
+        auto old = std::min_element(free_.begin(), free_.end(),
+                                    [](const auto& a, const auto& b) { return a.second.age < b.second.age; });
+        p = old->second.p;
+        free_bytes_ -= old->first.second;
+        free_.erase(old);
       }
       give_plain(p);
     }
@@ -200,7 +204,8 @@ class DevicePool {
     return r;
   }
   std::mutex mu_;
-  std::multimap<Key, void*> free_;
+  std::multimap<Key, Block> free_;
+  unsigned long long given_ = 0;
   std::unordered_map<void*, Key> used_;
   size_t free_bytes_ = 0;
 };

@@ -116,3 +116,22 @@ def test_kept_memory_is_returned_on_request():
     assert free() < before - (64 << 20)
     sap.trim_memory()
     assert free() >= before - (32 << 20)
+
+
+def test_kept_memory_is_bounded():
+    ns = (300_007, 500_009, 700_001, 900_001, 1_100_009)
+    As = [sap.BandedMatrix.from_array(sap.generate_band_host(n, 30, 1.0, 1, seed=n), n, 30) for n in ns]
+
+    def use(A):
+        s = sap.Solver(16, options(), prec="double")
+        s.setup(A)
+
+    use(As[0])
+    sap.trim_memory()
+    torch.cuda.synchronize()
+    before = torch.cuda.mem_get_info()[0]
+    for A in As + As[:1]:  # 4 GB of buffers in blocks of many sizes
+        use(A)
+        torch.cuda.synchronize()
+        assert torch.cuda.mem_get_info()[0] >= before - (2 << 30) - (64 << 20)
+    sap.trim_memory()
