@@ -769,7 +769,7 @@ class PrecondT : public PrecBase {
       for (auto& d : parts_h) maxsz = std::max(maxsz, d.size);
       scratch.alloc((size_t)2 * (P - 1) * maxsz * K);
       if (K > 1024) throw Error(SAP_ERR_UNSUPPORTED, "coupling width above 1024 is not supported by the spike kernel");
-      if (window(K) && window(parts_maxK())) {
+      if (packed && window(K)) {
         spikes_lu(iface_d.get(), maxsz);
       } else {
         k_spikes_var<T><<<dim3(P - 1, 2), ((K + 31) / 32) * 32, 0, st>>>(
@@ -857,7 +857,7 @@ class PrecondT : public PrecBase {
       const T* b2 = B2.get() ? B2.get() : B.get();
       int maxsz = 0;
       for (auto& p : parts_h) maxsz = std::max(maxsz, p.size);
-      if (lu_ul && window(K)) {
+      if (lu_ul && packed) {
         pack_corners(b2);
         by_window(K, [&](auto R1) {
           auto kern = k_win_spikes_luul<T, R1(), kSpikeCols>;
@@ -872,7 +872,7 @@ class PrecondT : public PrecBase {
         k_spikes_luul<T><<<dim3(P - 1, 2), ((K + 31) / 32) * 32, 0, st>>>(parts_d.get(), P, B.get(), b2, offd.get(),
                                                                         V.get(), W.get(), K);
         SAPB_LAUNCHED();
-      } else if (window(K)) {
+      } else if (packed) {
         scratch.alloc(spike_scratch(P - 1, K, maxsz, false));
         spikes_lu(nullptr, maxsz);
       } else {
@@ -895,7 +895,8 @@ class PrecondT : public PrecBase {
   }
 
   // The register-window kernels (narrow_sweeps.cuh) take half-bandwidths up
-  // to kWinMaxK; f gets their slot count as a compile-time constant.
+  // to kWinMaxK, the sweeps among them where the factors are packed
+  // (pack_factors); f gets their slot count as a compile-time constant.
   static bool window(int k) { return k <= kWinMaxK<T>; }
   template <class F>
   static void by_window(int k, F&& f) {
@@ -1045,6 +1046,20 @@ class PrecondT : public PrecBase {
     pack_factors();
   }
 
+  // Chunks of a partition's sweeps.  The window sweeps and their scan are chains
+  // of about 50 ns per row and 0.2 - 0.4 us per chunk, the rows passed four times
+  // and the chunks twice per sweep pair: shortest where a chunk has about
+  // sqrt(rows per partition times their ratio) rows.  At least 2 K rows, so that
+  // a transfer matrix stays below its chunk's factors.
+  static int chunk_count(const PartDev& d, bool packed) {
+    const int m = packed ? std::max({2 * d.K, 32, (int)std::sqrt(d.size * (3.0 + d.K / 24.0))})
+                         : std::min(4096, std::max(256, 8 * d.K));
+    return std::max(1, d.size / m);
+  }
+  // values of one chunk's transfer matrix
+  static long long transfer_values(int Kp, int maxK, bool packed) {
+    return packed ? (long long)scan_rows(Kp) * scan_stride(maxK) : (long long)Kp * Kp;
+  }
   void build_sweeps() {
     int maxK = parts_maxK();
     if (maxK > 1024) throw Error(SAP_ERR_UNSUPPORTED, "half-bandwidth above 1024 is not supported by the sweep kernels");
@@ -1056,14 +1071,7 @@ class PrecondT : public PrecBase {
     for (int p = 0; p < (int)parts_h.size(); p++) {
       const auto& d = parts_h[p];
       int Kp = d.K;
-      int m = std::min(4096, std::max(256, 8 * Kp));
-      // The window sweeps and their scan are chains of about 50 ns per row and
-      // 0.2 - 0.4 us per chunk, the rows passed four times and the chunks twice
-      // per sweep pair: shortest where m is about sqrt(rows per partition times
-      // their ratio).  At least 2 K rows, so that the transfer matrices stay
-      // below half of the factors' bytes.
-      if (window(maxK)) m = std::max({2 * Kp, 32, (int)std::sqrt(d.size * (3.0 + Kp / 24.0))});
-      int nc = std::max(1, d.size / m);
+      const int nc = chunk_count(d, packed);
       pc0.push_back((int)chunks_h.size());
       pnc.push_back(nc);
       int base = d.size / nc, rem = d.size % nc, a = d.start;
@@ -1074,7 +1082,7 @@ class PrecondT : public PrecBase {
         koff.push_back(ko);
         toff.push_back(to);
         ko += Kp;
-        to += window(maxK) ? (long long)scan_rows(Kp) * scan_stride(maxK) : (long long)Kp * Kp;
+        to += transfer_values(Kp, maxK, packed);
         bool down1 = !d.ul;
         first1.push_back(down1 ? (c == 0) : (c == nc - 1));
         first2.push_back(down1 ? (c == nc - 1) : (c == 0));
@@ -1100,7 +1108,7 @@ class PrecondT : public PrecBase {
     sweepThreads = std::max(32, ((maxK + 31) / 32) * 32);
     scanG = std::max(1, std::min(maxK, 512 / std::max(1, maxK)));
     const int nch = (int)chunks_h.size();
-    if (window(maxK)) {
+    if (packed) {
       build_window(maxK, nch);
       return;
     }
@@ -1133,12 +1141,45 @@ class PrecondT : public PrecBase {
   // B for the last partition, else in b2.
   DBuf<T> pkd, pku, piv, pkd2, pku2, piv2;
   int KP = 0;
+  bool packed = false;
+  // The packed copies take as much memory as the factors themselves, and the
+  // window kernels' transfer matrices up to half of that again.  A band that
+  // does not leave room for them, and for the vectors of a solve, runs on the
+  // kernels that read the factors in place (SAPB_NARROW_PACK=0: every band does).
+  bool pack_fits(int maxK) {
+    const char* e = std::getenv("SAPB_NARROW_PACK");
+    if (e && std::atoi(e) == 0) return false;
+    if (pkd.size() == (size_t)n * KP && piv.size() == (size_t)n) return true;  // held already
+    double need = (2.0 * KP + 1.0) * n * sizeof(T);
+    for (const auto& d : parts_h)
+      need += 2.0 * chunk_count(d, true) * transfer_values(d.K, maxK, true) * sizeof(T);
+    if (need < 256e6) return true;  // (an allocation that fails is caught)
+    const int vectors = o.solverType == SAP_FGMRES ? 104 : 20;
+    need += (3.0 * sizeof(T) + vectors * sizeof(double)) * n + 3.0 * (P - 1) * K * K * sizeof(T);
+    size_t fr = 0, tot = 0;
+    SAPB_CUDA(cudaMemGetInfo(&fr, &tot));
+    if (need > 0.92 * (double)fr) {
+      DevicePool::instance().trim();
+      SAPB_CUDA(cudaMemGetInfo(&fr, &tot));
+    }
+    return need <= 0.92 * (double)fr;
+  }
   void pack_factors() {
-    if (!window(parts_maxK())) return;
-    KP = pack_stride<T>(parts_maxK());
-    pkd.alloc((size_t)n * KP);
-    pku.alloc((size_t)n * KP);
-    piv.alloc(n);
+    const int maxK = parts_maxK();
+    KP = pack_stride<T>(maxK);
+    packed = window(maxK) && pack_fits(maxK);
+    if (packed) try {
+        pkd.alloc((size_t)n * KP);
+        pku.alloc((size_t)n * KP);
+        piv.alloc(n);
+      } catch (const Error& e) {
+        if (e.code != SAP_ERR_OUT_OF_MEMORY) throw;
+        packed = false;
+      }
+    if (!packed) {
+      for (DBuf<T>* b : {&pkd, &pku, &piv, &pkd2, &pku2, &piv2}) b->release();
+      return;
+    }
     const int np = (int)parts_h.size();
     k_pack<T><<<dim3(grid_for(((long long)n / np + 1) * 32, 256, std::max(1, 148 * 32 / np)), (unsigned)np), 256, 0, st>>>(
         parts_d.get(), B.get(), -1, KP, pkd.get(), pku.get(), piv.get());
@@ -1200,8 +1241,8 @@ class PrecondT : public PrecBase {
     else if (k <= 16) f(integral_constant<int, 8>{}, integral_constant<int, 16>{});
     else if (k <= 32) f(integral_constant<int, 32>{}, integral_constant<int, 32>{});
     else if (k <= 64) f(integral_constant<int, 8>{}, integral_constant<int, 64>{});
-    else if (k <= 128) f(integral_constant<int, 16>{}, integral_constant<int, 0>{});
-    else f(integral_constant<int, 32>{}, integral_constant<int, 0>{});
+    else if (kWinMaxK<T> <= 128 || k <= 128) f(integral_constant<int, 16>{}, integral_constant<int, 0>{});
+    else if constexpr (kWinMaxK<T> > 128) f(integral_constant<int, 32>{}, integral_constant<int, 0>{});
   }
   void window_scan(const T* Tm, const T* tails, T* carry, int which) {
     SAPB_PROF("scan", st);
@@ -1247,7 +1288,7 @@ class PrecondT : public PrecBase {
   void sweep_pair(const double* vin, double* zout, T* gout) {
     const int nch = (int)chunks_h.size();
     const int maxK = parts_maxK();
-    if (window(maxK)) return window_pair(vin, zout, gout, maxK, nch);
+    if (packed) return window_pair(vin, zout, gout, maxK, nch);
     const size_t s1 = (size_t)(maxK + maxChunk) * sizeof(T);
     const int NT = sweepThreads;
     const int scanNT = ((maxK * scanG + 31) / 32) * 32;

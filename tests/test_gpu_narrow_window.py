@@ -113,3 +113,59 @@ def test_two_live_solvers(dtype, one, two):
         assert o.setup_banded(sap.generate_band_host(n, K, 1.0, 1, seed=n + K), n, K) == 0
         zo = o.apply(v)
         assert np.linalg.norm(z - zo) / np.linalg.norm(zo) <= TOL[dtype]
+
+
+@pytest.mark.parametrize("dtype", ["double", "float"])
+@pytest.mark.parametrize("n,K,P", [(1003, 2, 5), (12011, 64, 5), (18001, 107, 3), (700, 5, 60)])
+def test_factors_read_in_place(n, K, P, dtype, monkeypatch):
+    # the kernels of bands without room for packed factors, first and after a
+    # setup that packed them
+    band = sap.generate_band_host(n, K, 1.0, 1, seed=n + K)
+    A = sap.BandedMatrix.from_array(band, n, K)
+    v = np.random.default_rng(K).standard_normal(n)
+    for fact, kind in ((sap.LU_UL, sap.Spike), (sap.LU_only, sap.Spike), (sap.LU_UL, sap.Block)):
+        o = oracle.Precond(P, fact=fact, ptype=kind, dtype=dtype)
+        assert o.setup_banded(band, n, K) == 0
+        zo = o.apply(v)
+        s = sap.Solver(P, sap.Options(performReorder=False, variableBandwidth=False, applyScaling=False,
+                                      factMethod=fact, precondType=kind), prec=dtype)
+        for pack in ("0", "1", "0"):
+            monkeypatch.setenv("SAPB_NARROW_PACK", pack)
+            s.setup(A)
+            assert np.linalg.norm(band_apply(s, v) - zo) / np.linalg.norm(zo) <= TOL[dtype]
+    rp, ci, w = uneven_band(n, (K, max(1, K // 3)), n)
+    s = sap.Solver(P, sap.Options(), prec=dtype)
+    s.setup(sap.CsrMatrix(rp, ci, w))
+    o = oracle.SparsePrecond(P, dtype=dtype)
+    assert o.setup(rp, ci, w) == 0
+    zo = o.apply(v)
+    assert np.linalg.norm(band_apply(s, v) - zo) / np.linalg.norm(zo) <= TOL[dtype]
+
+
+def test_band_that_leaves_no_room_for_packed_factors():
+    n, K, P = 4_000_000, 60, 148
+    g = torch.Generator(device="cuda")
+    g.manual_seed(1)
+    band = torch.empty(n, 2 * K + 1, dtype=torch.float64, device="cuda").uniform_(-1.0, 1.0, generator=g)
+    band[:, K] = 2 * K + 1
+    A = sap.BandedMatrix.from_array(band, n, K)  # 3.9 GB, as much as its factors
+    del band
+    v = torch.ones(n, dtype=torch.float64, device="cuda")
+    opts = sap.Options(performReorder=False, variableBandwidth=False, applyScaling=False, precondType=sap.Block)
+
+    def solve():
+        s = sap.Solver(P, opts, prec="double")
+        s.setup(A)
+        z = torch.empty_like(v)
+        s.precond(v, z)
+        return z
+
+    z = solve()
+    sap.trim_memory()
+    torch.cuda.empty_cache()
+    torch.cuda.synchronize()
+    rest = torch.empty(torch.cuda.mem_get_info()[0] - 6_500_000_000, dtype=torch.uint8, device="cuda")
+    z2 = solve()
+    del rest
+    torch.cuda.empty_cache()
+    assert float((z2 - z).norm() / z.norm()) <= 1e-10
