@@ -267,7 +267,8 @@ class PrecondT : public PrecBase {
     return o.safeFactorization || K >= 70;
   }
 
-  void wide_check_memory(int kmax) {
+  // (returns the memory that the factors leave)
+  double wide_check_memory(int kmax) {
     size_t fr = 0, tot = 0;
     SAPB_CUDA(cudaMemGetInfo(&fr, &tot));
     if (wide) fr += wide->bytes_held();  // reused (or released) by the new setup
@@ -281,6 +282,7 @@ class PrecondT : public PrecBase {
     if (need > 0.92 * (double)fr)
       throw Error(SAP_ERR_OUT_OF_MEMORY, "wide-band factors need " + std::to_string(need / 1e9) + " GB, " +
                                              std::to_string((double)fr / 1e9) + " GB free");
+    return (double)fr - need;
   }
 
   // Interface unknowns of the variable band: the last K first-level rows of
@@ -298,7 +300,7 @@ class PrecondT : public PrecBase {
   }
 
   void wide_init(int kmax) {
-    wide_check_memory(kmax);
+    const double room = wide_check_memory(kmax);
     std::vector<int> ps(P), pz(P);
     for (int p = 0; p < P; p++) {
       ps[p] = parts_h[p].start;
@@ -307,6 +309,7 @@ class PrecondT : public PrecBase {
     if (!wide) wide = std::make_unique<WideBand<T>>();
     wide->init(st, n, WideBand<T>::block_size(kmax, tf32 && sizeof(T) == 4 && WideBand<T>::tc_gemm_enabled()), kmax,
                ps, pz, tf32, h16);
+    wide->room = room;
     wide_active = true;
   }
 

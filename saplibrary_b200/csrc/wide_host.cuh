@@ -325,6 +325,7 @@ class WideBand {
   cudaGraphExec_t fgraph = nullptr;
   long long fgraph_key = -1;
   int fgraph_cut = 0, fgraph_leaf = 0, fgraph_kc = 0;
+  bool fgraph_ahead = false;
   // SAPB_FACTOR_GRAPH=0 runs the factorization's launches directly every time
   static bool graph_enabled() {
     const char* e = std::getenv("SAPB_FACTOR_GRAPH");
@@ -580,16 +581,16 @@ class WideBand {
   void factor(bool boost) {
     Dw.alloc((size_t)P * BB);
     Ww.alloc((size_t)P * BB);
-    if (ahead_mode()) {
-      Dw2.alloc((size_t)P * BB);
-      Cu_.alloc((size_t)P * kc * kc);
-      Cl_.alloc((size_t)P * kc * kc);
-    }
+    const bool ahead = ahead_mode();
+    Dw2.alloc(ahead ? (size_t)P * BB : 0);
+    Cu_.alloc(ahead ? (size_t)P * kc * kc : 0);
+    Cl_.alloc(ahead ? (size_t)P * kc * kc : 0);
     Rw.alloc((size_t)P * std::max(1LL, BlockLU<T>::rec_ws(bs, leaf_size<T>())));
     flag.alloc(1);
     const long long key = (((long long)P * 65537 + bs) * 65537 + nb) * 4 + (boost ? 2 : 0) + (tf32 ? 1 : 0);
-    if (key != fgraph_key || kc != fgraph_kc || factor_cut() != fgraph_cut || leaf_size<T>() != fgraph_leaf) {
+    if (key != fgraph_key || kc != fgraph_kc || ahead != fgraph_ahead || factor_cut() != fgraph_cut || leaf_size<T>() != fgraph_leaf) {
       fgraph_kc = kc;
+      fgraph_ahead = ahead;
       fgraph_cut = factor_cut();
       fgraph_leaf = leaf_size<T>();
       if (fgraph) cudaGraphExecDestroy(fgraph);
@@ -666,7 +667,7 @@ class WideBand {
     // row's D is taken ahead into a second workspace, and the corners stay in
     // workspaces that the next Schur complement reads, their copies to the
     // factor slots running beside it on the second lane.
-    const bool ahead = ahead_mode() && nb > 1;
+    const bool ahead = Dw2.size() > 0;
     const Mat<T> Db[2] = {Mat<T>{Dw.get(), bs, BB}, ahead ? Mat<T>{Dw2.get(), bs, BB} : Mat<T>{Dw.get(), bs, BB}};
     const long long sC = (long long)kc * kc;
     const Mat<T> Cu{Cu_.get(), kc, sC}, Cl{Cl_.get(), kc, sC};
@@ -714,8 +715,16 @@ class WideBand {
       }
     }
   }
-  // blocks whose second workspace is small beside the factors
-  bool ahead_mode() const { return bs <= 512; }
+  // Whether the second workspaces are taken: for blocks of at most 512 rows, where
+  // the copies they save lie on the chain, and where they need no more than a
+  // quarter of the memory that the factors leave (the spikes want the rest).
+  // SAPB_FACTOR_AHEAD=0 does without.
+  bool ahead_mode() const {
+    const char* e = std::getenv("SAPB_FACTOR_AHEAD");
+    if (e && std::atoi(e) == 0) return false;
+    return bs <= 512 && nb > 1 && (double)P * (BB + 2.0 * kc * kc) * sizeof(T) <= 0.25 * room;
+  }
+  double room = 0;  // memory beside the factors (set by the owner before factor())
   DBuf<T> Dw2, Cu_, Cl_;
 
   // tri: 0 full, 1 lower, 2 upper (see k_tgemv).  Grids with fewer than

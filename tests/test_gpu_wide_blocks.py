@@ -67,6 +67,27 @@ def test_blocks_of_one_leaf(prec, n, K, P, monkeypatch):
         assert np.linalg.norm(first - zo) / np.linalg.norm(zo) <= TOL[prec]
         assert np.array_equal(z.cpu().numpy(), first)
         s.setup(A)
+    # and without the second workspaces (a captured factorisation is replaced)
+    monkeypatch.setenv("SAPB_FACTOR_AHEAD", "0")
+    for _ in range(3):
+        s.setup(A)
+        s.precond(torch.tensor(v, device="cuda"), z)
+        assert np.array_equal(z.cpu().numpy(), first)
+
+
+@pytest.mark.parametrize("prec,n,K,P", [("double", 9001, 130, 4), ("float", 9001, 300, 3), ("tf32", 20011, 200, 19)])
+def test_second_workspaces_change_no_bit(prec, n, K, P, monkeypatch):
+    band = sap.generate_band_host(n, K, 1.0, 1, seed=n + K)
+    A, s = setup(n, K, P, prec, band)
+    assert s.blockLayout()[1] > 1
+    v = torch.tensor(np.random.default_rng(K).standard_normal(n), device="cuda")
+    out = []
+    for ahead in ("1", "0", "0", "0", "1", "1", "1"):  # direct, captured, replayed in turn
+        monkeypatch.setenv("SAPB_FACTOR_AHEAD", ahead)
+        s.setup(A)
+        out.append(torch.empty_like(v))
+        s.precond(v, out[-1])
+    assert all(torch.equal(z, out[0]) for z in out)
 
 
 @pytest.mark.parametrize("prec,K", [("float", 157), ("double", 109)])
