@@ -300,6 +300,7 @@ class PrecondT : public PrecBase {
   }
 
   void wide_init(int kmax) {
+    drop_packed();  // of an earlier setup on the narrow path
     const double room = wide_check_memory(kmax);
     std::vector<int> ps(P), pz(P);
     for (int p = 0; p < P; p++) {
@@ -1167,6 +1168,10 @@ class PrecondT : public PrecBase {
     }
     return need <= 0.92 * (double)fr;
   }
+  void drop_packed() {
+    packed = false;
+    for (DBuf<T>* b : {&pkd, &pku, &piv, &pkd2, &pku2, &piv2}) b->release();
+  }
   void pack_factors() {
     const int maxK = parts_maxK();
     KP = pack_stride<T>(maxK);
@@ -1179,10 +1184,7 @@ class PrecondT : public PrecBase {
         if (e.code != SAP_ERR_OUT_OF_MEMORY) throw;
         packed = false;
       }
-    if (!packed) {
-      for (DBuf<T>* b : {&pkd, &pku, &piv, &pkd2, &pku2, &piv2}) b->release();
-      return;
-    }
+    if (!packed) return drop_packed();
     const int np = (int)parts_h.size();
     k_pack<T><<<dim3(grid_for(((long long)n / np + 1) * 32, 256, std::max(1, 148 * 32 / np)), (unsigned)np), 256, 0, st>>>(
         parts_d.get(), B.get(), -1, KP, pkd.get(), pku.get(), piv.get());

@@ -169,3 +169,31 @@ def test_band_that_leaves_no_room_for_packed_factors():
     del rest
     torch.cuda.empty_cache()
     assert float((z2 - z).norm() / z.norm()) <= 1e-10
+
+
+def test_wide_setup_drops_the_packed_factors_of_a_narrow_one():
+    n, K = 2_000_003, 60
+    narrow = sap.BandedMatrix.from_array(sap.generate_band_host(n, K, 1.0, 1, seed=1), n, K)
+    wide = sap.BandedMatrix.from_array(sap.generate_band_host(5003, 130, 1.0, 1, seed=2), 5003, 130)
+    opts = sap.Options(performReorder=False, variableBandwidth=False, applyScaling=False, precondType=sap.Block)
+
+    def free():
+        sap.trim_memory()
+        torch.cuda.synchronize()
+        return torch.cuda.mem_get_info()[0]
+
+    s = sap.Solver(8, opts, prec="double")
+    s.setup(narrow)
+    held = free()
+    s.setup(wide)
+    assert s.blockLayout()[0] > 0
+    # at least the packed factors (2 n K values) and the band (n (2 K + 1)) are gone
+    assert free() - held >= 8 * n * (4 * K) - (1 << 29)
+    z = band_apply(s, np.ones(5003))
+    s2 = sap.Solver(8, opts, prec="double")
+    s2.setup(wide)
+    assert np.array_equal(band_apply(s2, np.ones(5003)), z)
+    s.setup(narrow)
+    z = band_apply(s, np.ones(n))
+    s2.setup(narrow)
+    assert np.array_equal(band_apply(s2, np.ones(n)), z)
