@@ -8,10 +8,11 @@
 namespace sapb {
 
 // Largest half-bandwidth of the register-window kernels: the narrow path's
-// own range (FP32 up to 155, FP64 up to 107; wider bands take the block path,
-// and the shared-memory kernels of precond_kernels.cuh only when
-// SAPB_WIDE_MIN_K keeps such a band on the narrow path).  At these widths two
-// K x K stages of the carry scan still fit in shared memory.
+// own range (FP32 up to 155, FP64 up to 108; wider bands take the block path).
+// The shared-memory kernels of precond_kernels.cuh take the bands that leave no
+// room for packed factors, and wider ones that SAPB_WIDE_MIN_K keeps on the
+// narrow path.  At these widths two K x K stages of the carry scan still fit in
+// shared memory.
 template <typename T>
 constexpr int kWinMaxK = sizeof(T) == 8 ? 112 : 160;
 // Lanes that hold a chunk's window: the warp, or half of it (two chunks per
@@ -54,8 +55,8 @@ constexpr size_t win_smem(int R1, int LW = 32) { return (size_t)(32 / LW) * (kRi
 // resolved redundantly in every lane, and each lane subtracts the four
 // products from its rows.  Each row receives its updates in source order with
 // one fused multiply-add each, as in a row-at-a-time solve.  The coefficients
-// come through shared memory, staged by cp.async one group ahead; all warps
-// of the CTA share them (each has its own right-hand sides).
+// come through shared memory, staged by cp.async kStages - 1 stages ahead; all
+// warps of the CTA share them (each has its own right-hand sides).
 //
 // rhs(c, v) is called once per row, by the lane that holds it, at least 32
 // rows ahead of out(c, v, x), which is called once per row.  The staging area
@@ -375,11 +376,10 @@ __host__ __device__ inline size_t scan_pad(size_t values) {  // to a multiple of
   constexpr size_t per = 16 / sizeof(T);
   return (values + per - 1) / per * per;
 }
-// values of one batch: NB matrices, NB tails (these with room for the offset
-// of an unaligned source)
+// values of one batch: NB matrices, NB tails
 template <typename T>
 inline size_t scan_batch(int K, int NB) {
-  return (size_t)scan_rows(K) * scan_stride(K) * NB + scan_pad<T>((size_t)K * NB + 4);
+  return (size_t)scan_rows(K) * scan_stride(K) * NB + scan_pad<T>((size_t)K * NB);
 }
 // maxK: the widest partition's (its strides hold for all); TSC: scan_stride(maxK)
 // when it is a compile-time class, else 0
@@ -395,7 +395,7 @@ k_win_scan(const PartDev* __restrict__ parts, const int* __restrict__ pchunk0, c
   extern __shared__ __align__(16) unsigned char win_raw[];
   constexpr bool WARP = TSC > 0 && TSC <= 32;
   const int TS = TSC ? TSC : ts, KR = scan_rows(K), KT = KR * TS;
-  const size_t TO = (size_t)KT * NB, SB = TO + scan_pad<T>((size_t)K * NB + 4);
+  const size_t TO = (size_t)KT * NB, SB = TO + scan_pad<T>((size_t)K * NB);
   T* st = reinterpret_cast<T*>(win_raw);
   T* sig = st + 2 * SB;                            // the carry, zeros up to KZ
   const int G = (K + KG - 1) / KG, KZ = WARP ? 32 : G * KG;

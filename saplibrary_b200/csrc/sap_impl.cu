@@ -244,8 +244,8 @@ class PrecondT : public PrecBase {
   // Partitions are factored and applied as block tridiagonal (wide_host.cuh)
   // when the narrow factor's window (K+1+8 band columns of 2K+1 values) does
   // not fit in 200 KB of shared memory, where the narrow kernels fall back to
-  // a global-memory window and the block path is faster (FP64 from K ~ 108,
-  // FP32 from K ~ 155 on B200), and always above K = 1024.  The environment
+  // a global-memory window and the block path is faster (FP64 from K = 109,
+  // FP32 from K = 156 on), and always above K = 1024.  The environment
   // variable SAPB_WIDE_MIN_K sets an explicit threshold instead.
   static bool use_wide(int kmax) {
     if (kmax > 1024) return true;

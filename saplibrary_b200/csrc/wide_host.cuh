@@ -340,9 +340,13 @@ class WideBand {
   // Block size bs >= the largest half-bandwidth, a multiple of the leaf size.
   // Larger blocks mean fewer block rows, hence fewer dependent launches per
   // partition, for more factor flops and sweep bytes; with the tensor-core
-  // TF32 products the flops are cheap and bs is at least 448 (2M-row K = 200
-  // workload, TF32 + FGMRES: 0.154 s at bs 448 against 0.221 / 0.179 / 0.182 s
-  // at 224 / 672 / 896; FP32 and FP64 are fastest at the smallest bs).
+  // TF32 products the flops are cheap and bs is at least 448, the widest that
+  // k_sweep_cluster takes.  Setup + FGMRES solve, TF32, at bs 224 / 256 / 320 /
+  // 448 / 672 / 896: 83 / 81 / 86 / 77 / 118 / 108 ms for 2,000,000 rows, K = 200,
+  // 32 partitions; 128 partitions 51 / - / 51 / 47 ms; 1,000,000 rows, K = 300:
+  // 320 / 448 / 672 53 / 46 / 66 ms.  A short band alone prefers the smallest
+  // (200,000 rows, K = 160: 224 / 448 15.4 / 17.2 ms).  FP32 and FP64, whose
+  // products are not cheap, take the smallest bs.
   // SAPB_BLOCK_SIZE raises it further.
   static int block_size(int kmax, bool tf32_products = false) {
     int bs = std::max(kLeaf, ((kmax + kLeaf - 1) / kLeaf) * kLeaf);

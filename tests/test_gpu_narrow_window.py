@@ -2,7 +2,9 @@
 the oracle's apply at the widths where they can go wrong: half-bandwidths at
 the edges of a lane's 32-row slots and of the packed rows' 16-byte padding,
 the narrowest and widest of the path, partitions shorter than a window group,
-ragged chunk lengths, LU_UL and LU_only tips, decoupled partitions.
+ragged chunk lengths, LU_UL and LU_only tips, decoupled partitions (two chunks
+per warp up to K = 16, an odd number of them included); two live solvers on the
+same kernels; the kernels that read the factors in place.
 Tolerances as in the other apply tests: 1e-10 (FP64), 2e-4 (FP32)."""
 import numpy as np
 import pytest
@@ -17,6 +19,7 @@ TOL = {"double": 1e-10, "float": 2e-4}
 SHAPES = [  # n, K, P
     (41, 1, 3), (1003, 2, 5), (2000, 8, 4), (6007, 31, 6), (6011, 32, 5), (9001, 33, 7), (12011, 64, 5),
     (12013, 65, 6), (15013, 96, 4), (16001, 97, 5), (18001, 107, 3), (150, 30, 2), (700, 5, 60),
+    (18007, 108, 3),
 ]
 
 
@@ -24,7 +27,7 @@ SHAPES = [  # n, K, P
 @pytest.mark.parametrize("fact", [sap.LU_UL, sap.LU_only])
 @pytest.mark.parametrize("n,K,P", SHAPES + [(20011, 121, 4), (20021, 155, 3)])
 def test_window_apply_matches_oracle(n, K, P, fact, dtype):
-    if dtype == "double" and K > 107:
+    if dtype == "double" and K > 108:
         pytest.skip("FP64 bands this wide take the block path")
     band = sap.generate_band_host(n, K, 1.0, 1, seed=n + K)
     opts = sap.Options(performReorder=False, variableBandwidth=False, applyScaling=False, factMethod=fact)
@@ -37,6 +40,22 @@ def test_window_apply_matches_oracle(n, K, P, fact, dtype):
     z = torch.empty(n, dtype=torch.float64, device="cuda")
     s.precond(torch.tensor(v, device="cuda"), z)
     z, zo = z.cpu().numpy(), o.apply(v)
+    assert np.linalg.norm(z - zo) / np.linalg.norm(zo) <= TOL[dtype]
+
+
+@pytest.mark.parametrize("dtype", ["double", "float"])
+@pytest.mark.parametrize("n,K,P", [(130, 1, 1), (97, 3, 1), (1009, 7, 3), (850, 16, 1), (5003, 16, 7), (5009, 17, 7), (9001, 33, 7),
+                                   (16001, 97, 5), (18007, 108, 3)])
+def test_decoupled_partitions_match_oracle(n, K, P, dtype):
+    band = sap.generate_band_host(n, K, 1.0, 1, seed=n + K)
+    s = sap.Solver(P, sap.Options(performReorder=False, variableBandwidth=False, applyScaling=False,
+                                  precondType=sap.Block), prec=dtype)
+    s.setup(sap.BandedMatrix.from_array(band, n, K))
+    assert s.blockLayout()[0] == 0
+    o = oracle.Precond(P, ptype=sap.Block, dtype=dtype)
+    assert o.setup_banded(band, n, K) == 0
+    v = np.random.default_rng(K).standard_normal(n)
+    z, zo = band_apply(s, v), o.apply(v)
     assert np.linalg.norm(z - zo) / np.linalg.norm(zo) <= TOL[dtype]
 
 
