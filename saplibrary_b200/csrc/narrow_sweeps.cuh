@@ -222,7 +222,8 @@ __global__ void k_pack(const PartDev* __restrict__ parts, const T* __restrict__ 
 // The three passes of a chunked partition sweep (see precond_kernels.cuh), one
 // warp (up to K = 16 half a warp) per chunk.  About 50 ns per row: 1,000,000
 // rows, K = 10, FP64, passes 1 / 2 / 3 65 / 140 / 66 us with a CTA per chunk and
-// a barrier per row, 51 / 105 / 51 us with a warp per chunk.
+// a barrier per row, 51 / 105 / 51 us with a warp per chunk, 39 / 66 / 35 us with
+// half a warp.
 // The chunk of this lane's window (past the last one: a sweep of no rows).
 template <int LW>
 __device__ __forceinline__ int win_chunk() {
