@@ -966,9 +966,13 @@ class WideBand {
   // persistent).  SAPB_SWEEP_PERSISTENT = 1 (or 0) and SAPB_SWEEP_LANES =
   // 1 / 2 / 4 fix the schedule instead.
   DBuf<T> tune_x;
-  static std::map<std::tuple<int, int, int, int>, int>& tuned() {
-    static std::map<std::tuple<int, int, int, int>, int> m;
-    return m;
+  struct Tuned {  // shared by the solvers of all threads
+    std::mutex mu;
+    std::map<std::tuple<int, int, int, int>, int> mode;
+  };
+  static Tuned& tuned() {
+    static Tuned t;
+    return t;
   }
   static int fixed_mode() {
     const char* pe = std::getenv("SAPB_SWEEP_PERSISTENT");
@@ -1016,9 +1020,17 @@ class WideBand {
     if (mode < 0 && bs <= kClusterMaxBs) return sweep_cluster(x);
     if (mode < 0) {
       const auto key = std::make_tuple(P, bs, nb, h16 ? 2 : (int)sizeof(T));
-      auto it = tuned().find(key);
-      if (it == tuned().end()) it = tuned().emplace(key, tune_sweep(x)).first;
-      mode = it->second;
+      Tuned& t = tuned();
+      {
+        std::lock_guard<std::mutex> lk(t.mu);
+        const auto it = t.mode.find(key);
+        if (it != t.mode.end()) mode = it->second;
+      }
+      if (mode < 0) {  // (timed outside of the lock; the first result stays)
+        const int m = tune_sweep(x);
+        std::lock_guard<std::mutex> lk(t.mu);
+        mode = t.mode.emplace(key, m).first->second;
+      }
     }
     if (!run_sweep(x, mode)) run_sweep(x, 2);
   }

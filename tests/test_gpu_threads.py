@@ -97,6 +97,37 @@ def test_captured_setups_beside_other_solvers(prec):
     assert not errors, errors
 
 
+def test_threads_choose_their_sweep_schedules_side_by_side():
+    # blocks above 448 rows, a layout of its own for each solver: every first
+    # application times the schedules and enters the choice
+    jobs = [(6011 + 97 * i, 449 + 32 * (i % 3), 2 + i % 4) for i in range(8)]
+    bands = [sap.generate_band_host(n, K, 1.0, 1, seed=n) for n, K, _ in jobs]
+    As = [sap.BandedMatrix.from_array(b, n, K) for b, (n, K, _) in zip(bands, jobs)]
+
+    def apply(i, rounds, out):
+        n, K, P = jobs[i]
+        s = sap.Solver(P, options(), prec="tf32")
+        s.setup(As[i])
+        v = torch.ones(n, dtype=torch.float64, device="cuda")
+        torch.cuda.synchronize()
+        for _ in range(rounds):
+            z = torch.zeros_like(v)
+            torch.cuda.synchronize()
+            s.precond(v, z)
+            out.append(z)
+
+    outs = [[] for _ in jobs]
+    ts = [in_thread(lambda i=i: apply(i, 3, outs[i])) for i in range(len(jobs))]
+    for t, errors in ts:
+        t.join()
+        assert not errors, errors
+    for i, (n, K, P) in enumerate(jobs):
+        alone = []
+        apply(i, 1, alone)
+        for z in outs[i]:
+            assert float((z - alone[0]).norm() / alone[0].norm()) <= 1e-5
+
+
 def test_kept_memory_is_returned_on_request():
     n, K = 400003, 50
     A = sap.BandedMatrix.from_array(sap.generate_band_host(n, K, 1.0, 1, seed=3), n, K)
