@@ -23,7 +23,9 @@ falls back to it where the network is unsure.  Two families:
 
 Labels are the settings with the lowest measured time-to-solution (setup +
 flexible GMRES with an FP32 preconditioner to relres 1e-10, best of a few
-repetitions); a setting that fails or does not converge costs infinity.
+repetitions); of settings within the measurement's noise of each other, the one
+that is never far off on the other matrices.  A setting that fails or does not
+converge costs infinity.
 """
 from __future__ import annotations
 
@@ -206,7 +208,8 @@ def sweep(family, count: int | None = None, seed: int = 0, **kw) -> tuple[np.nda
             b = np.random.default_rng(n).standard_normal(n)
             X.append(csr_features(rp, ci, v))
             A = CsrMatrix(rp, ci, v)
-            T.append([measure_sparse(A, s, b) for s in range(len(family.settings))])
+            # two rounds over the settings: a host stall can cover all of a setting's repetitions
+            T.append(np.min([[measure_sparse(A, s, b) for s in range(len(family.settings))] for _ in range(2)], axis=0))
     return np.asarray(X, np.float32), np.asarray(T, np.float64)
 
 
@@ -283,9 +286,20 @@ class SettingsNet:
         return picks
 
 
+# times closer than this are not told apart: partition counts that a matrix clamps
+# to the same number give the same solve under several settings
+TIE = 0.1
+
+
 def labels_from_times(T: np.ndarray) -> np.ndarray:
-    """The fastest setting per matrix."""
-    return np.argmin(T, axis=1).astype(np.int32)
+    """The fastest setting per matrix; of those within TIE of it, the one whose
+    largest time over all matrices, relative to each matrix's best, is lowest (so
+    that a tie does not teach a setting that costs many times more elsewhere)."""
+    T = np.asarray(T, np.float64)
+    best = T.min(axis=1, keepdims=True)
+    solved = np.isfinite(best[:, 0])  # (a matrix that every setting fails tells nothing)
+    worst = np.minimum(T[solved] / best[solved], 10.0).max(axis=0, initial=1.0)
+    return np.where(T <= (1.0 + TIE) * best, worst, np.inf).argmin(axis=1).astype(np.int32)
 
 
 def gain(*args) -> dict:

@@ -23,6 +23,15 @@ def test_gain_and_labels_from_a_time_table():
     assert g["total_chosen_s"] == 6.0 and g["total_default_s"] == 10.0 and g["picked_best"] == 1.0
 
 
+def test_labels_of_tied_settings():
+    inf = np.inf
+    # settings 1 and 2 tie on the first two matrices; 2 costs five times the best on the third
+    T = np.array([[3.0, 1.02, 1.0], [3.0, 1.0, 1.05], [1.0, 1.5, 5.0], [inf, 2.0, 4.0], [inf, inf, inf]])
+    assert list(learned.labels_from_times(T)) == [1, 1, 0, 1, 1]
+    assert learned.labels_from_times(T).dtype == np.int32
+    assert list(learned.labels_from_times(np.array([[2.0, 1.0], [inf, 3.0]]))) == [1, 1]
+
+
 def test_ensemble_generator_shapes_and_seeds():
     bands, ks, bs = ensemble.make_ensemble(12, seed=4, n_min=2000, n_max=8000, ks=(8, 16))
     assert len(bands) == len(ks) == len(bs) == 12
