@@ -596,5 +596,5 @@ class Solver:
 
 
 __all__ = ["Options", "Stats", "Solver", "BandedMatrix", "CsrMatrix", "MVBanded", "SpmvCusp", "SystemError",
-           "LibraryError", "generate_band_host", "kernel_launch_count", "BiCGStab1", "BiCGStab2", "FGMRES", "LU_UL",
-           "LU_only", "Spike", "Block", "NoPrecond", "EXPORTED_SYMBOLS"]
+           "LibraryError", "generate_band_host", "kernel_launch_count", "trim_memory", "BiCGStab1", "BiCGStab2", "FGMRES",
+           "LU_UL", "LU_only", "Spike", "Block", "NoPrecond", "EXPORTED_SYMBOLS"]

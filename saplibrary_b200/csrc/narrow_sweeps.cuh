@@ -774,9 +774,11 @@ k_win_reduced_apply(const PartDev* __restrict__ parts, const T* __restrict__ V, 
   }
   __syncthreads();
   rows_dot(Vi, z, [&](int r, T a) { x1[r] = xb[r] - a; });
-  rows_dot(Bm, z, [&](int r, T b) { F[pos_b(r)] -= b; });
+  // (a partition of fewer than 2 K rows has rows that belong to both of its
+  // interfaces, whose CTAs run side by side)
+  rows_dot(Bm, z, [&](int r, T b) { atomicAdd(&F[pos_b(r)], -b); });
   __syncthreads();
-  rows_dot(Cm, x1, [&](int r, T a) { F[pos_t(r)] -= a; });
+  rows_dot(Cm, x1, [&](int r, T a) { atomicAdd(&F[pos_t(r)], -a); });
 }
 
 }  // namespace sapb

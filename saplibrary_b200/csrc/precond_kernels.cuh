@@ -981,8 +981,10 @@ k_reduced_apply(const PartDev* __restrict__ parts, const T* __restrict__ V, cons
       t1 += Bm[r * K + c] * z[c];
       t2 += Cm[r * K + c] * x1[c];
     }
-    F[pos_b(r)] -= t1;
-    F[pos_t(r)] -= t2;
+    // (a partition of fewer than 2 K rows has rows that belong to both of its
+    // interfaces, whose CTAs run side by side)
+    atomicAdd(&F[pos_b(r)], -t1);
+    atomicAdd(&F[pos_t(r)], -t2);
   }
 }
 

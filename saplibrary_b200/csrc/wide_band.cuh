@@ -1097,6 +1097,17 @@ __global__ void k_gather_idx(const T* __restrict__ src, const long long* __restr
     dst[e] = idx[e] >= 0 ? src[idx[e]] : T(0);
 }
 
+// dst[idx[e]] = vals[e] for the K rows from `first` on of every interface's 2 K
+// (first: 0 bottom of the partition before, K top of the one after)
+template <typename T>
+__global__ void k_iface_rows(const long long* __restrict__ idx, int K, long long rows, int first,
+                             const T* __restrict__ vals, T* __restrict__ dst) {
+  for (long long r = blockIdx.x * (long long)blockDim.x + threadIdx.x; r < rows; r += (long long)gridDim.x * blockDim.x) {
+    const long long e = r / K * 2 * K + first + r % K;
+    dst[idx[e]] = vals[e];
+  }
+}
+
 // leftTrans into the band-order right-hand side: F[row] = T(v[gin[row]]) * sin[row]
 template <typename T>
 __global__ void k_wb_in(const double* __restrict__ v, const int* __restrict__ gin, const T* __restrict__ sin,

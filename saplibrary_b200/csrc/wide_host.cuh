@@ -271,6 +271,7 @@ class WideBand {
   int ldK = 0;                               // leading dimension of the K x K blocks (16-byte multiple)
   long long sK = 0;                          // their batch stride, ldK * K
   bool spike = false;
+  bool overlap = false;  // a partition has rows that belong to both of its interfaces
   long long plen = 0, BB = 0;
   std::vector<int> pstart_h, psize_h;
   DBuf<int> pstart_d, psize_d, rowpart_d;
@@ -1119,6 +1120,7 @@ class WideBand {
     ldK = (K + V - 1) / V * V;
     sK = (long long)ldK * K;
     spike = true;
+    overlap = *std::min_element(psize_h.begin(), psize_h.end()) < 2 * K;
     const int nI = P - 1;
     Vc.alloc((size_t)nI * sK);
     Wc.alloc((size_t)nI * sK);
@@ -1292,8 +1294,15 @@ class WideBand {
     gemv(Vc.get(), ldK, sK, t1.get(), K, xb, s2, t2.get(), K, K, nI, 1, 0);       // z1 = xb - V z2
     // the coupling blocks' entries lie within the half-bandwidth: B lower, C upper triangular
     gemv(Bc.get(), ldK, sK, t1.get(), K, fb, s2, fb, s2, K, nI, 1, 1);            // f_b -= B z2
+    if (overlap) {  // rows of both interfaces of a partition: f_t from what f_b left
+      k_iface_rows<T><<<grid1d(m / 2), 256, 0, st>>>(irow.get(), K, m / 2, 0, fbt.get(), F);
+      SAPB_LAUNCHED();
+      k_gather_idx<T><<<grid1d(m), 256, 0, st>>>(F, irow.get(), m, fbt.get());
+      SAPB_LAUNCHED();
+    }
     gemv(Cc.get(), ldK, sK, t2.get(), K, ft, s2, ft, s2, K, nI, 1, 2);            // f_t -= C z1
-    k_scatter_idx<T><<<grid1d(m), 256, 0, st>>>(irow.get(), fbt.get(), m, F);
+    if (overlap) k_iface_rows<T><<<grid1d(m / 2), 256, 0, st>>>(irow.get(), K, m / 2, K, fbt.get(), F);
+    else k_scatter_idx<T><<<grid1d(m), 256, 0, st>>>(irow.get(), fbt.get(), m, F);
     SAPB_LAUNCHED();
   }
 

@@ -216,3 +216,46 @@ def test_wide_setup_drops_the_packed_factors_of_a_narrow_one():
     z = band_apply(s, np.ones(n))
     s2.setup(narrow)
     assert np.array_equal(band_apply(s2, np.ones(n)), z)
+
+
+@pytest.mark.parametrize("wide", [False, True])
+@pytest.mark.parametrize("variable", [False, True])
+@pytest.mark.parametrize("dtype", ["double", "float"])
+def test_partitions_shorter_than_two_couplings(dtype, variable, wide, monkeypatch):
+    # a reordered matrix may be cut into partitions of K + 1 rows on, whose rows
+    # then belong to both interfaces: both corrections arrive
+    n, P = 700, 16
+    rp, ci, v = uneven_band(n, (30,), 5)
+    if wide:
+        monkeypatch.setenv("SAPB_WIDE_MIN_K", "1")
+    s = sap.Solver(P, sap.Options(performDB=False, applyScaling=False, variableBandwidth=variable), prec=dtype)
+    s.setup(sap.CsrMatrix(rp, ci, v))
+    assert (s.blockLayout()[0] > 0) == wide
+    K = s.getStats().bandwidth
+    q, r = divmod(n, P)
+    assert s.getStats().numPartitions == P and K < q < 2 * K
+    x = np.random.default_rng(1).standard_normal(n)
+    z = [band_apply(s, x) for _ in range(20)]
+    assert max(np.linalg.norm(a - z[0]) for a in z) <= 1e-2 * TOL[dtype] * np.linalg.norm(z[0])
+    if variable:  # (the same matrix in another order inside the partitions)
+        monkeypatch.delenv("SAPB_WIDE_MIN_K", raising=False)
+        s = sap.Solver(P, sap.Options(performDB=False, applyScaling=False, variableBandwidth=False), prec=dtype)
+        s.setup(sap.CsrMatrix(rp, ci, v))
+    row, col = s.getReorder("finalPerm"), np.argsort(s.getReorder("finalReordering"))
+    A = np.zeros((n, n))
+    A[row[np.repeat(np.arange(n), np.diff(rp))], col[ci]] = v
+    ends = np.concatenate([[0], np.cumsum([q + (i < r) for i in range(P)])])
+    D = [A[a:e, a:e] for a, e in zip(ends[:-1], ends[1:])]
+    f = np.empty(n)
+    f[row] = x
+    solve = lambda f: np.concatenate([np.linalg.solve(d, f[a:a + len(d)]) for d, a in zip(D, ends)])
+    g, f2 = solve(f), f.copy()
+    for i, e in enumerate(ends[1:-1]):
+        b, t = slice(e - K, e), slice(e, e + K)
+        V = np.linalg.solve(D[i], np.concatenate([np.zeros((len(D[i]) - K, K)), A[b, t]]))[-K:]
+        W = np.linalg.solve(D[i + 1], np.concatenate([A[t, b], np.zeros((len(D[i + 1]) - K, K))]))[:K]
+        z2 = np.linalg.solve(np.eye(K) - W @ V, g[t] - W @ g[b])
+        f2[b] -= A[b, t] @ z2
+        f2[t] -= A[t, b] @ (g[b] - V @ z2)
+    ref = solve(f2)[col]
+    assert np.linalg.norm(z[0] - ref) / np.linalg.norm(ref) <= TOL[dtype]
